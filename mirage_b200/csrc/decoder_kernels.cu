@@ -25,13 +25,13 @@ extern "C" int mpk_family_prepare(int smem_bytes, int) {
 
 extern "C" int mpk_family_launch(const mpk::KernelParams *params, int smem_bytes, void *stream) {
   if (params->general_kernel && params->world_size > 1)
-    mpk::mpk_megakernel<true, true><<<params->num_workers, mpk::kBlockThreads, smem_bytes, (cudaStream_t)stream>>>(*params);
+    mpk::mpk_megakernel<true, true><<<params->num_workers, mpk::block_threads(true), smem_bytes, (cudaStream_t)stream>>>(*params);
   else if (params->general_kernel)
-    mpk::mpk_megakernel<true><<<params->num_workers, mpk::kBlockThreads, smem_bytes, (cudaStream_t)stream>>>(*params);
+    mpk::mpk_megakernel<true><<<params->num_workers, mpk::block_threads(true), smem_bytes, (cudaStream_t)stream>>>(*params);
   else if (params->world_size > 1 && params->tp_extensions)
-    mpk::mpk_megakernel<false, true><<<params->num_workers, mpk::kBlockThreads, smem_bytes, (cudaStream_t)stream>>>(*params);
+    mpk::mpk_megakernel<false, true><<<params->num_workers, mpk::block_threads(false), smem_bytes, (cudaStream_t)stream>>>(*params);
   else
-    mpk::mpk_megakernel<false><<<params->num_workers, mpk::kBlockThreads, smem_bytes, (cudaStream_t)stream>>>(*params);
+    mpk::mpk_megakernel<false><<<params->num_workers, mpk::block_threads(false), smem_bytes, (cudaStream_t)stream>>>(*params);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : (int)e;
 }

@@ -23,7 +23,7 @@ extern "C" int mpk_family_prepare(int smem_bytes, int) {
 }
 
 extern "C" int mpk_family_launch(const mpk::KernelParams *params, int smem_bytes, void *stream) {
-  pick(params->hybrid, params->general_kernel)<<<params->num_workers, mpk::kBlockThreads, smem_bytes, (cudaStream_t)stream>>>(*params);
+  pick(params->hybrid, params->general_kernel)<<<params->num_workers, mpk::block_threads(params->hybrid == mpk::HYB_BF16 && params->general_kernel), smem_bytes, (cudaStream_t)stream>>>(*params);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : (int)e;
 }

@@ -5,7 +5,7 @@
 // include/mirage/persistent_kernel/persistent_kernel.cuh:513-1082) and the task bodies
 // it dispatches to (include/mirage/persistent_kernel/tasks/**) for the decode path.
 //
-// Structure of a worker CTA (one per SM, 288 threads):
+// Structure of a worker CTA (one per SM, 288 threads; 384 in the general instantiations):
 //   * warp 8 is the weight streamer.  It walks the worker's task list ahead of the
 //     compute warps and issues cp.async.bulk copies of the weight rows every linear
 //     task will need into a ring of 32 KB shared-memory stages guarded by mbarriers.
@@ -2238,6 +2238,13 @@ __device__ __noinline__ LinearState run_moe_gemm_hybrid(const Ctx c, const TaskD
   return ls;
 }
 
+// Out of line: inlined beside the other bodies its loop comes out worse with 224 registers than with the 168 a function call gets
+// (32 tokens, 103 experts: 2038 us inlined, 1926 us like this, 1870 to 1910 us before the register split).
+static __device__ __noinline__ LinearState run_moe_gemm_decoder(const Ctx c, const TaskDesc &d, LinearState ls, int task, bool ok) {
+  run_moe_gemm<false>(c, d, ls, task, ok);
+  return ls;
+}
+
 static __device__ void run_moe_silu_mul(const Ctx &c, const TaskDesc &d) {
   const int I = d.a[2], ldi = d.a[3], ldo = d.a[4];
   const int r1 = min(d.a[1], active_tokens(c.P) * d.a[5]);
@@ -4239,7 +4246,7 @@ __device__ void consumer_loop(const Ctx &c, int t_begin, int t_end) {
       ls = run_moe_gemm_hybrid<GENERAL>(c, d, ls, t, ok);
     } else if (GENERAL && !HYB && type == TASK_MOE_GEMM) {
       ok = wait_dependencies(c, d, t, ok, tt);
-      run_moe_gemm<false>(c, d, ls, t, ok);
+      ls = run_moe_gemm_decoder(c, d, ls, t, ok);
     } else if (!HYB && type == TASK_ATTENTION) ok = task_attention<GENERAL>(c, d, t, ok, tt);
     else ok = task_other<GENERAL, TPX, HYB>(c, d, t, ok, tt);
     if (fetch) reinterpret_cast<uint4 *>(&c.s.desc[(t + 1 - t_begin) & 1])[tid - 224] = nxt;
@@ -4281,7 +4288,7 @@ __device__ void consumer_loop(const Ctx &c, int t_begin, int t_end) {
 // linear bodies and the hybrid tasks only.  HYB_BF16 serves in bf16; HYB_F32 computes everything in 32-bit floats and has
 // no tensor-core code at all.
 template <bool GENERAL, bool TPX = false, int HYB = 0>
-__global__ void __launch_bounds__(kBlockThreads, 1) mpk_megakernel(const __grid_constant__ KernelParams P) {
+__global__ void __launch_bounds__(block_threads(GENERAL), 1) mpk_megakernel(const __grid_constant__ KernelParams P) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   Smem s = carve(smem_raw, P);
   const int tid = threadIdx.x;
@@ -4311,8 +4318,10 @@ __global__ void __launch_bounds__(kBlockThreads, 1) mpk_megakernel(const __grid_
         use_tmem ? *reinterpret_cast<volatile uint32_t *>(s.tmem_holder) : 0u};
   const int t_begin = P.worker_begin[blockIdx.x], t_end = P.worker_begin[blockIdx.x + 1];
   if (tid >= kConsumerThreads) {
-    streamer_loop<GENERAL, HYB>(c, t_begin, t_end);
+    if (GENERAL) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kStreamerRegs));
+    if (tid < kConsumerThreads + 32) streamer_loop<GENERAL, HYB>(c, t_begin, t_end);
   } else {
+    if (GENERAL) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kConsumerRegs));
     consumer_loop<GENERAL, TPX, HYB>(c, t_begin, t_end);
   }
   if (use_tmem) tc_fence_before_sync();

@@ -12,7 +12,15 @@ namespace mpk {
 
 constexpr int kMaxDeps = 3;
 constexpr int kConsumerThreads = 256;          // 8 compute warps
-constexpr int kBlockThreads = kConsumerThreads + 32;  // + 1 weight-streaming warp
+// + 1 weight-streaming warp.  That ninth warp costs the compute warps a third of the register file (three warps on a scheduler instead
+// of two: 168 registers a thread), and what is spilled comes back from L2: beside 220 KB of shared memory there is next to no L1.  So in
+// the general instantiations the streaming warp is the first of a warpgroup (the other three idle) that hands its registers over.
+// 36 layers of width 4096: 16 requests 7842 -> 7539 us, 64 requests 12.58 -> 12.05 ms, 64 prompt tokens 16.90 -> 14.58 ms (88 or 104 registers
+// for the streaming warp: 1 % slower).  Not in the narrow instantiations: their streaming warp copies row by row and loses more to
+// spills than their bodies gain (one request 3.34 -> 3.53 ms).
+constexpr int block_threads(bool general) { return kConsumerThreads + (general ? 128 : 32); }
+constexpr int kConsumerRegs = 224, kStreamerRegs = 56;  // registers a thread after the split of the launch's 168 x 384
+static_assert(kConsumerRegs * kConsumerThreads + kStreamerRegs * 128 <= 168 * block_threads(true), "a larger sum would wait for registers that never come");
 constexpr int kChunkRows = 16;                 // weight rows per streamed chunk, at most (one mma m-tile)
 constexpr int kChunkColsMax = 2048;            // k extent of a chunk, at most (the graph compiler may settle for 1024)
 constexpr int kRowPadBytes = 16;               // shared-memory row padding: conflict-free ldmatrix
