@@ -32,6 +32,8 @@
 
 namespace mpk {
 
+constexpr int kFlagsOffset = 960;   // of the flags in the area of small things
+
 struct Smem {
   uint8_t *stages;      // num_stages * stage_bytes
   uint8_t *xtile;       // x_tile_bytes (activation tile / attention scratch)
@@ -45,8 +47,6 @@ struct Smem {
   uint32_t *tmem_holder;   // tensor-memory base address written by tcgen05.alloc
 };
 
-constexpr int kStashRing = 16;     // attention stash records of the general instantiation (32 bytes each, after the flags)
-
 __device__ __forceinline__ Smem carve(uint8_t *base, const KernelParams &P) {
   Smem s;
   s.stages = base;
@@ -57,7 +57,7 @@ __device__ __forceinline__ Smem carve(uint8_t *base, const KernelParams &P) {
   s.empty = s.full + 16;                                    // 16 * 8
   s.desc = reinterpret_cast<TaskDesc *>(misc + 256);        // 2 * 224 = 448
   s.red = reinterpret_cast<float *>(misc + 704);            // 64 * 4 = 256
-  s.flags = reinterpret_cast<int *>(misc + 960);            // 16 ints
+  s.flags = reinterpret_cast<int *>(misc + kFlagsOffset);   // 16 ints
   s.acc_bar = s.empty + 8;                                  // entries 8.. of the empty-barrier array are unused (<= 8 stages)
   s.tmem_holder = reinterpret_cast<uint32_t *>(s.empty + 9);
   return s;
@@ -105,6 +105,25 @@ __device__ __forceinline__ bool wait_mbar(const Ctx &c, uint64_t *bar, uint32_t 
   return true;
 }
 
+// The same for bodies that take no Ctx, on a shared-memory address.
+static __device__ __noinline__ bool wait_bar_slow(const KernelParams &P, uint32_t bar, uint32_t parity, uint64_t deadline, int task) {
+  uint32_t polls = 0;
+  while (!bar_try_wait(bar, parity)) {
+    if ((++polls & 0x3ff) == 0) {
+      if (ld_volatile_i32(&P.status->error) != 0) return false;
+      if (globaltimer_ns() > deadline) {
+        report_timeout(P.status, (int)blockIdx.x, 2, task);
+        return false;
+      }
+    }
+  }
+  return true;
+}
+__device__ __forceinline__ bool wait_bar(const KernelParams &P, uint32_t bar, uint32_t parity, uint64_t deadline, int task) {
+  if (bar_try_wait(bar, parity)) return true;
+  return wait_bar_slow(P, bar, parity, deadline, task);
+}
+
 __device__ __forceinline__ bool wait_counter(const Ctx &c, const unsigned long long *ctr,
                                              unsigned long long need, bool sys_scope, int where, int task) {
   uint32_t polls = 0;
@@ -122,8 +141,7 @@ __device__ __forceinline__ bool wait_counter(const Ctx &c, const unsigned long l
   }
 }
 
-template <bool GENERAL>
-__device__ void prefetch_attention_kv_l2(const Ctx &c, const TaskDesc *d, int lane, int task);
+static __device__ void prefetch_attention_kv_l2(const Ctx &c, const TaskDesc *d, int lane, int task);
 
 // ---------------------------------------------------------------------------
 // weight streamer (warp 8)
@@ -148,7 +166,7 @@ __device__ void streamer_loop(const Ctx &c, int t_begin, int t_end) {
   // The whole warp walks the task list; lane 0 owns the barrier traffic, lane r copies row r of a chunk.
   for (int t = t_begin; t < t_end && ok; ++t) {
     const TaskDesc *d = &P.tasks[t];
-    if (!HYB && d->type == TASK_ATTENTION && P.kv_l2_prefetch) prefetch_attention_kv_l2<GENERAL>(c, d, lane, t);
+    if (!GENERAL && !HYB && d->type == TASK_ATTENTION && P.kv_l2_prefetch) prefetch_attention_kv_l2(c, d, lane, t);
     if (d->type != TASK_LINEAR && !(kMoe && d->type == TASK_MOE_GEMM)) continue;
     if (d->flags & TF_STREAM_AFTER_DEP) {
       if (lane == 0)
@@ -2615,17 +2633,11 @@ __device__ __forceinline__ size_t kv_offset(const KernelParams &P, const TaskDes
 // batching event of this iteration had already fired (acquire), i.e. when what was read is final; it carries the task
 // index, is written index-last and read index-first-and-last, so a reader either gets a consistent record of its own
 // task or falls back to its own loads.
-// Where the stash record of a task lives: the narrow instantiation has one record in the unused tail of the
-// full-barrier array; the general one, whose workers see runs of many attention tasks that the streaming warp walks
-// past at once, has a ring of kStashRing records after the flags.
-template <bool GENERAL>
-__device__ __forceinline__ volatile int *attention_stash(const Ctx &c, int task) {
-  if (GENERAL) return reinterpret_cast<volatile int *>(c.s.flags + 16) + (task & (kStashRing - 1)) * 8;
+__device__ __forceinline__ volatile int *attention_stash(const Ctx &c) {
   return reinterpret_cast<volatile int *>(&c.s.full[8]);
 }
 
-template <bool GENERAL>
-__device__ void prefetch_attention_kv_l2(const Ctx &c, const TaskDesc *d, int lane, int task) {
+static __device__ void prefetch_attention_kv_l2(const Ctx &c, const TaskDesc *d, int lane, int task) {
   const KernelParams &P = c.P;
   if ((d->a[A_FLAGS] & 4) || P.meta.qo_indptr == nullptr) return;
   const bool final_meta = P.meta_static || ld_acquire_gpu(&P.counters[0]) >= c.iteration;
@@ -2649,7 +2661,7 @@ __device__ void prefetch_attention_kv_l2(const Ctx &c, const TaskDesc *d, int la
     const int p0 = __ldcg(&P.meta.paged_kv_indices[kv0 + pb]);
     const int p1 = (pb + 1 < npages) ? __ldcg(&P.meta.paged_kv_indices[kv0 + pb + 1]) : p0;
     if (lane == 0) {
-      volatile int *st = attention_stash<GENERAL>(c, task);
+      volatile int *st = attention_stash(c);
       st[0] = -1;
       __threadfence_block();
       st[1] = q0; st[2] = nq; st[3] = kv0; st[4] = (npages - 1) * page + __ldcg(&P.meta.paged_kv_last_page_len[slot]);
@@ -2658,10 +2670,7 @@ __device__ void prefetch_attention_kv_l2(const Ctx &c, const TaskDesc *d, int la
       st[0] = task;
     }
   }
-  // The general instantiation streams the chunk through shared memory with many copies in flight: an L2 prefetch
-  // ahead of it only fetches every row twice whenever the rows do not survive in L2 until they are used (measured:
-  // DRAM reads 1.87 x the K/V bytes on a 268 MB attention-only launch).
-  for (int pos = start + lane; !GENERAL && pos < old_end; pos += 32) {
+  for (int pos = start + lane; pos < old_end; pos += 32) {
     const int pidx = pos / page;
     const int pid = min(max(__ldcg(&P.meta.paged_kv_indices[kv0 + pidx]), 0), P.max_num_pages - 1);
     const size_t off = ((((size_t)pid * page + (pos - pidx * page)) * hkv + d->a[A_HEAD]) * 128) * 2;
@@ -2676,12 +2685,11 @@ __device__ __forceinline__ void load_rope(const __nv_bfloat16 *cosT, const __nv_
                                           int lane, uint2 &cs, uint2 &sn);
 
 // Runs before the dependency wait (the batch description is already final).
-template <bool GENERAL>
 __device__ __forceinline__ void attention_prefetch(const Ctx &c, const TaskDesc &d, AttnPre &pre, int task) {
   const KernelParams &P = c.P;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   // the streaming warp may have left this task's request description and first page ids in shared memory
-  const volatile int *st = attention_stash<GENERAL>(c, task);
+  const volatile int *st = attention_stash(c);
   bool hit = st[0] == task;
   int pb = 0, p0 = 0, p1 = 0;
   if (hit) {
@@ -3078,395 +3086,612 @@ __device__ __forceinline__ void run_attention(const Ctx &c, const TaskDesc &d, c
 }
 
 // ---------------------------------------------------------------------------
-// TASK_ATTENTION, general instantiation (many requests): per-warp K/V streams through shared memory, tensor-core math
+// TASK_ATTENTION, general instantiation (many tokens): every warp takes an equal share of all key steps
 // ---------------------------------------------------------------------------
-// With many requests a worker gets whole (request, kv head) pairs or large chunks of them, and what matters is
-// bytes in flight and instructions per byte.  The cached positions of the chunk are split evenly over the eight
-// compute warps; every warp runs its OWN cp.async pipeline over its share -- steps of 8 positions (K and V rows,
-// 4 KB) through a private ring of shared-memory stages, no block-wide barrier inside the loop -- and starts it
-// before the task waits for this layer's qkv projection, because rows already in the cache do not depend on it.
-// Per step: S = Q K^T on mma.sync m16n8k16 (the query heads of the kv head are the M rows, at most 8 of 16), online
-// softmax on the score fragment (fp32, base 2), P rounded to bf16 as the reference does
-// (tasks/blackwell/attention_sm100.cuh:558), O += P V on m16n8k8 with V read through ldmatrix.trans.  The rows this
-// step appends form one more tile in the same layout, taken by the last warp.  Page ids of the chunk are fetched
-// once into shared memory; a step never straddles a page (page sizes are multiples of 8).
-constexpr int kAsStepRows = 8;
-constexpr int kAsPitch = 272;                              // bytes between rows of a K or V tile (256 + 16: conflict-free ldmatrix)
-constexpr int kAsStepBytes = 2 * kAsStepRows * kAsPitch;   // K rows, then V rows
-constexpr int kAsPageCap = 256;                            // page ids of a chunk kept in shared memory
+// The unit of work is a step: 8 positions of one (request, kv head) for one tile of 16 query rows (16 / G tokens x the G heads of the
+// group; a decoding request has one tile).  Eight kv heads go together, one per warp of a worker (with fewer, the warps share out
+// ranges), so that a cached position is read whole, 2 KB at a time: with a range per (head, warp) the same bytes came at 1.3 TB/s.  The
+// steps of the whole layer, in the order request, head group, tile, position, are cut into equal ranges by arithmetic on the batch
+// description alone: 16 requests of 512 to 4000 positions keep all workers busy to the end, where a task per (request, head, chunk)
+// left the last ones 38 us behind.  A warp walks its range without any block barrier: its
+// own ring of stages, filled by two tensor-map copies a step, runs on across the borders of heads and requests, and starts before the task waits for this layer's
+// qkv projection, because rows already in the cache do not depend on it.  Rows that this launch appends are normed and rotated by
+// the warp that meets them (the first tile's warp writes them to the cache), so no warp waits for another's append.
+// A tile that lies in one range is written out at once; otherwise every range leaves its part in a scratch record and the last of them
+// to arrive (a ticket per tile) merges.  Per step: S = Q K^T on mma.sync m16n8k16, online softmax (fp32, base 2), P rounded to bf16 as the
+// reference does (tasks/blackwell/attention_sm100.cuh:558), O += P V on m16n8k8 with V through ldmatrix.trans.
+// Where that leaves a range fewer than kAfMinSteps steps, the latency of a few steps in a row and of merging many parts through L2 is what
+// counts.  Then a worker takes a tile of one kv head (or one of NC parts of it, where there are fewer tiles than workers), its eight warps
+// share the positions and combine in shared memory.
+// Measured, us per layer, before (one task per request, head and chunk) and now: 16 requests of 512 to 4000 positions 76 -> 56,
+// 64 of 512 to 1536 109 -> 75 (3.6 TB/s), 32 + 32 prompt tokens behind 1000 and 343 positions 235 -> 39, 24 requests of 60 positions 14.8 -> 11.8, 41 of
+// 94 to 214 positions with 4 kv heads 14.4 -> 12.4.  The two ways are instantiations of their own and rows are prepared two at a time:
+// what one body of both spilled cost a tenth.  What bounds it now is the latency of the steps of a warp (two in flight) and, for short contexts, the fixed part.
+constexpr int kAfRows = 8;                       // positions of a step
+constexpr int kAfTile = kAfRows * 256;           // K or V rows of a step: two blocks of 64 columns in the 128-byte swizzle of the tensor map
+constexpr int kAfStage = 2 * kAfTile;            // K rows, then V rows; also the 16 query rows of a tile
+constexpr int kAfMinSteps = 16;                  // ranges of fewer steps: the warps of a worker share a tile instead (see below)
+constexpr int kAfRecord = 16 * 132;              // floats of a record: 16 rows x {max, sum, -, -, 128 outputs}
 
-struct AttnStream {
-  ReqView rv;
-  int start, end, new_start, old_end, n_active, nstg, pg0, new_rows_cap;
-  int w_begin, w_end;   // cached positions this warp streams
-  int issued;           // steps of this warp requested so far
-  uint2 cs0, sn0;
-  int *pg;              // shared: page ids of pages pg0 .. of the request
-  uint8_t *stages;      // shared: [8 warps][nstg] steps
-  uint8_t *q_tile;      // shared: 8 rows x kAsPitch, bf16 query heads (rows >= G are zero)
-  float *w_ml;          // shared: per warp and head {max, sum}
-  uint8_t *new_tile;    // shared: rows appended by this task, K rows then V rows, kAsPitch apart
-  // descriptor fields the copy loop needs, read once
-  const uint8_t *kbase, *vbase;
-  int page, hkv, head, flags, slot, cseq;
-};
+__device__ __forceinline__ uint32_t af_piece(int row, int piece) { return (uint32_t)((piece >> 3) * 1024 + row * 128 + (((piece & 7) ^ row) << 4)); }
+__device__ __forceinline__ uint32_t af_qpiece(int row, int piece) { return (uint32_t)((piece >> 3) * 2048 + row * 128 + (((piece & 7) ^ (row & 7)) << 4)); }
 
 __device__ __forceinline__ void mma_bf16_1688(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t b0) {
   asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
                : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
                : "r"(a0), "r"(a1), "r"(b0));
 }
+
 __device__ __forceinline__ void ldmatrix_x2(uint32_t (&r)[2], uint32_t smem_addr) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(smem_addr));
 }
 
-// This warp requests step `step` of its share (8 positions): a row is 16 pieces of 16 bytes, lane -> piece lane % 16
-// of rows lane / 16 + 2 i.  One commit per call, empty or not: the waits count groups.
-__device__ __forceinline__ void attn_stream_issue(const Ctx &c, const AttnStream &a, int step, int warp, int lane) {
-  const int pos0 = a.w_begin + step * kAsStepRows;
-  if (pos0 < a.w_end) {
-    size_t off;
-    if (a.flags & 4) {
-      off = (((size_t)a.slot * a.cseq + pos0) * a.hkv + a.head) * 256;
-    } else {
-      const int pidx = pos0 / a.page, rel = pidx - a.pg0;
-      const int pid = rel < kAsPageCap ? a.pg[rel] : __ldcg(&c.P.meta.paged_kv_indices[a.rv.kv0 + pidx]);
-      off = (((size_t)pid * a.page + (pos0 - pidx * a.page)) * a.hkv + a.head) * 256;
-    }
-    const size_t row_stride = (size_t)a.hkv * 256;
-    const int piece = lane & 15, r0 = lane >> 4;
-    uint8_t *stage = a.stages + (size_t)(warp * a.nstg + step % a.nstg) * kAsStepBytes;
-    const int n = a.w_end - pos0;   // valid rows of this step (>= 1)
-#pragma unroll
-    for (int i = 0; i < kAsStepRows / 2; ++i) {
-      const int r = r0 + 2 * i;
-      uint8_t *dst = stage + r * kAsPitch + piece * 16;
-      if (r < n) {
-        const size_t o = off + (size_t)r * row_stride + piece * 16;
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(a.kbase + o) : "memory");
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst + kAsStepRows * kAsPitch)), "l"(a.vbase + o)
-                     : "memory");
+// Table of the requests that have tokens, behind the other small areas of shared memory: {q0, tokens, kv0 (contiguous caches: slot), length}, then
+// the first step of each (and the total), then the first tile.  The order is that of the batch slots, the same in every worker.  Warp 0
+// builds it in the first attention task of a launch (three round trips to L2); it holds for every layer with the same geometry.
+struct AfTable {
+  int4 *req;
+  int *step0, *tile0;
+};
+struct AfHead {              // in front of the table: what it was built for (slots, kv heads, query heads, page | contiguous), then the
+  int4 key;                  // number of its entries
+  int n, pad[3];
+};
+__device__ __forceinline__ AfTable af_table(uint8_t *base, int cap) {
+  AfTable t;
+  t.req = reinterpret_cast<int4 *>(base);
+  t.step0 = reinterpret_cast<int *>(base + cap * 16);
+  t.tile0 = t.step0 + cap + 1;
+  return t;
+}
+// kv heads that go together: the largest power of two, eight at most, that divides their number.
+__device__ __forceinline__ int af_heads(int hkv) { return min(hkv & -hkv, 8); }
+__device__ __forceinline__ void af_build_table(const KernelParams &P, const TaskDesc &d, const AfTable &t, AfHead *head) {
+  const int lane = threadIdx.x & 31, slots = d.a[A_SLOT], G = d.a[A_HQ] / d.a[A_HKV], hkv = d.a[A_HKV], page = d.a[A_PAGE], hh = af_heads(hkv);
+  int n = 0, steps = 0, tiles = 0;
+  for (int s0 = 0; s0 < slots; s0 += 32) {
+    const int slot = s0 + lane;
+    int4 r = make_int4(0, 0, 0, 0);
+    if (slot < slots) {
+      if (d.a[A_FLAGS] & 4) {   // contiguous cache: one token per slot, length = step + 1
+        r = make_int4(slot, slot < active_tokens(P) ? 1 : 0, slot, P.meta.step ? __ldcg(&P.meta.step[slot]) + 1 : 1);
       } else {
-        // positions past the end: defined zeros (a masked position has weight 0, and 0 x NaN from stale bytes would
-        // still be NaN in the P V product)
-        *reinterpret_cast<uint4 *>(dst) = make_uint4(0, 0, 0, 0);
-        *reinterpret_cast<uint4 *>(dst + kAsStepRows * kAsPitch) = make_uint4(0, 0, 0, 0);
+        r.x = __ldcg(&P.meta.qo_indptr[slot]);
+        r.y = __ldcg(&P.meta.qo_indptr[slot + 1]) - r.x;
+        r.z = __ldcg(&P.meta.paged_kv_indptr[slot]);
+        const int pages = __ldcg(&P.meta.paged_kv_indptr[slot + 1]) - r.z;
+        r.w = (pages - 1) * page + __ldcg(&P.meta.paged_kv_last_page_len[slot]);
       }
     }
-  }
-  asm volatile("cp.async.commit_group;" ::: "memory");
-}
-
-__device__ __forceinline__ void attn_stream_wait(int nstg) {   // all but the (nstg - 2) newest groups have landed
-  if (nstg >= 4) asm volatile("cp.async.wait_group 2;" ::: "memory");
-  else if (nstg == 3) asm volatile("cp.async.wait_group 1;" ::: "memory");
-  else asm volatile("cp.async.wait_group 0;" ::: "memory");
-}
-
-// Runs before the dependency wait (the batch description is already final): request view, chunk bounds, page ids,
-// shared-memory plan, and the first copies of every warp.
-template <bool GENERAL>
-__device__ __forceinline__ void attention_stream_begin(const Ctx &c, const TaskDesc &d, AttnStream &a, int task) {
-  const KernelParams &P = c.P;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const volatile int *st = attention_stash<GENERAL>(c, task);
-  bool hit = st[0] == task;
-  if (hit) {
-    a.rv.q0 = st[1]; a.rv.nq = st[2]; a.rv.kv0 = st[3]; a.rv.seq_len = st[4];
-    __threadfence_block();
-    hit = st[0] == task;
-  }
-  if (!hit) a.rv = request_view(P, d);
-  const int NC = d.a[A_NCHUNK], G = d.a[A_HQ] / d.a[A_HKV];
-  a.kbase = reinterpret_cast<const uint8_t *>(d.p[1]);
-  a.vbase = reinterpret_cast<const uint8_t *>(d.p[2]);
-  a.page = max(d.a[A_PAGE], 1); a.hkv = d.a[A_HKV]; a.head = d.a[A_HEAD]; a.flags = d.a[A_FLAGS];
-  a.slot = d.a[A_SLOT]; a.cseq = d.a[A_CSEQ];
-  int L = (a.rv.seq_len + NC - 1) / NC;
-  L = max((L + 15) & ~15, 16);
-  a.n_active = a.rv.nq > 0 ? (a.rv.seq_len + L - 1) / L : 0;
-  a.start = d.a[A_CHUNK] * L;
-  a.end = min(a.rv.seq_len, a.start + L);
-  a.new_start = a.rv.seq_len - a.rv.nq;
-  a.old_end = min(a.end, a.new_start);
-  const int n_old = (a.rv.nq > 0 && a.old_end > a.start) ? a.old_end - a.start : 0;
-  const int per_warp = ((n_old + 7) / 8 + kAsStepRows - 1) / kAsStepRows * kAsStepRows;   // multiple of 8 positions
-  a.w_begin = a.start + warp * per_warp;
-  a.w_end = min(a.w_begin + per_warp, a.start + n_old);
-  a.issued = 0;
-  a.cs0 = a.sn0 = make_uint2(0, 0);
-  // shared-memory plan: [q tile | warp maxima and sums | page ids | tile of the new rows | stages of the 8 warps]; the
-  // per-warp partial outputs of the final combine reuse the stage area once every warp's stream has drained
-  uint8_t *base = c.s.xtile;
-  a.q_tile = base;
-  a.w_ml = reinterpret_cast<float *>(base + 8 * kAsPitch);
-  a.pg = reinterpret_cast<int *>(a.w_ml + 8 * G * 2);
-  a.new_tile = reinterpret_cast<uint8_t *>(a.pg + kAsPageCap);
-  a.new_rows_cap = (min(P.max_num_batched_tokens, 64) + 7) & ~7;
-  a.stages = a.new_tile + (size_t)2 * a.new_rows_cap * kAsPitch;
-  const int avail = P.x_tile_bytes + kPartialBytes - (int)(a.stages - base);
-  a.nstg = max(1, min(4, avail / (8 * kAsStepBytes)));   // (the graph compiler sizes the region for at least two)
-  a.pg0 = a.start / a.page;
-  if (a.rv.nq <= 0) return;
-  load_rope((a.flags & 2) ? reinterpret_cast<const __nv_bfloat16 *>(d.p[5]) : nullptr,
-            reinterpret_cast<const __nv_bfloat16 *>(d.p[6]), a.new_start, d.a[A_ROPE_ROWS], lane, a.cs0, a.sn0);
-  if (!(a.flags & 4) && n_old > 0) {
-    const int n_pg = min((a.old_end - 1) / a.page - a.pg0 + 1, kAsPageCap);
-    for (int i = tid; i < n_pg; i += kConsumerThreads) a.pg[i] = __ldcg(&P.meta.paged_kv_indices[a.rv.kv0 + a.pg0 + i]);
-  }
-  // query rows the kv head does not have stay zero for the whole task; so do the rows of the new-row tile that this
-  // step does not fill (masked, but read by the P V product)
-  for (int i = tid; i < 8 * kAsPitch / 16; i += kConsumerThreads) reinterpret_cast<uint4 *>(a.q_tile)[i] = make_uint4(0, 0, 0, 0);
-  for (int i = tid; i < 2 * a.new_rows_cap * kAsPitch / 16; i += kConsumerThreads)
-    reinterpret_cast<uint4 *>(a.new_tile)[i] = make_uint4(0, 0, 0, 0);
-  consumer_sync();
-  for (int j = 0; j < a.nstg - 1; ++j) attn_stream_issue(c, a, j, warp, lane);
-  a.issued = a.nstg - 1;
-}
-
-// Eight positions against the query fragments: scores, online softmax, P V.  `n_valid` (1..8): positions below this
-// index take part.  The M rows are the query heads (rows 8-15 of the fragments are zero and never read back).
-__device__ __forceinline__ void attn_step_mma(const uint8_t *ktile, const uint8_t *vtile, int n_valid, const uint32_t (&qa)[8][2],
-                                              float &m_run, float &l_run, float (&o)[16][4], int lane) {
-  const int q = lane & 3;
-  float sc[4] = {0.f, 0.f, 0.f, 0.f};
-  const uint32_t k_addr = smem_u32(ktile) + (uint32_t)((lane & 7) * kAsPitch + (lane >> 3) * 16);
+    const bool on = r.y > 0 && r.w >= r.y;
+    const unsigned bal = __ballot_sync(0xffffffffu, on);
+    const int at = n + __popc(bal & ((1u << lane) - 1u));
+    const int nt = on ? hkv * ((r.y * G + 15) / 16) : 0, ns = nt / hh * ((r.w + kAfRows - 1) / kAfRows);
+    int it = nt, is = ns;
 #pragma unroll
-  for (int kk = 0; kk < 4; ++kk) {
-    uint32_t b[4];
-    ldmatrix_x4(b, k_addr + kk * 64u);
-    const uint32_t a0[4] = {qa[2 * kk][0], 0u, qa[2 * kk][1], 0u}, a1[4] = {qa[2 * kk + 1][0], 0u, qa[2 * kk + 1][1], 0u};
-    mma_bf16_16816(sc, a0, b[0], b[1]);
-    mma_bf16_16816(sc, a1, b[2], b[3]);
+    for (int o = 1; o < 32; o <<= 1) {
+      const int a = __shfl_up_sync(0xffffffffu, it, o), b = __shfl_up_sync(0xffffffffu, is, o);
+      if (lane >= o) { it += a; is += b; }
+    }
+    if (on && at < d.a[A_CAP]) {
+      t.req[at] = r;
+      t.step0[at] = steps + is - ns;
+      t.tile0[at] = tiles + it - nt;
+    }
+    steps += __shfl_sync(0xffffffffu, is, 31);
+    tiles += __shfl_sync(0xffffffffu, it, 31);
+    n += __popc(bal);
   }
-  const float qscale = 0.08838834764831845f * 1.4426950408889634f;   // 1/sqrt(128) * log2(e)
-  const int col = 2 * q;
-  const float s0 = (col < n_valid) ? sc[0] * qscale : -INFINITY;
-  const float s1 = (col + 1 < n_valid) ? sc[1] * qscale : -INFINITY;
-  float mx = fmaxf(s0, s1);
-  mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-  mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-  const float mn = fmaxf(m_run, mx);                    // finite: position 0 of the step is valid
-  const float corr = exp2f(m_run - mn);                 // 0 on the first step (m_run = -inf)
-  const float p0 = exp2f(s0 - mn), p1 = exp2f(s1 - mn);
-  float ps = p0 + p1;
-  ps += __shfl_xor_sync(0xffffffffu, ps, 1);
-  ps += __shfl_xor_sync(0xffffffffu, ps, 2);
-  l_run = l_run * corr + ps;
-  m_run = mn;
-#pragma unroll
-  for (int nt = 0; nt < 16; ++nt) { o[nt][0] *= corr; o[nt][1] *= corr; }
-  const uint32_t pa = pack_bf16(p0, p1);
-  const uint32_t v_addr = smem_u32(vtile) + (uint32_t)((lane & 7) * kAsPitch + (lane >> 3) * 16);
-#pragma unroll
-  for (int vq = 0; vq < 4; ++vq) {
-    uint32_t b[4];
-    ldmatrix_x4_trans(b, v_addr + vq * 64u);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) mma_bf16_1688(o[4 * vq + i], pa, 0u, b[i]);
+  n = min(n, d.a[A_CAP]);
+  if (lane == 0) {
+    t.step0[n] = steps;
+    t.tile0[n] = tiles;
+    head->key = make_int4(slots, hkv, G, (d.a[A_FLAGS] & 4) ? -page : page);
+    head->n = n;
   }
 }
 
-static __device__ void attention_stream_body(const Ctx &c, const TaskDesc &d, AttnStream &a, int task) {
-  const KernelParams &P = c.P;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const ReqView rv = a.rv;
-  if (rv.nq <= 0) return;
-  const int G = d.a[A_HQ] / d.a[A_HKV];
-  const int NC = d.a[A_NCHUNK], chunk = d.a[A_CHUNK], head = d.a[A_HEAD];
-  const int hq = d.a[A_HQ];
-  const int flags = d.a[A_FLAGS];
-  const float eps = __int_as_float(d.a[A_EPS]);
-  const __nv_bfloat16 *qkv = reinterpret_cast<const __nv_bfloat16 *>(d.p[0]);
-  __nv_bfloat16 *kc = reinterpret_cast<__nv_bfloat16 *>(d.p[1]);
-  __nv_bfloat16 *vc = reinterpret_cast<__nv_bfloat16 *>(d.p[2]);
-  const __nv_bfloat16 *qn = (flags & 1) ? reinterpret_cast<const __nv_bfloat16 *>(d.p[3]) : nullptr;
-  const __nv_bfloat16 *kn = (flags & 1) ? reinterpret_cast<const __nv_bfloat16 *>(d.p[4]) : nullptr;
-  const __nv_bfloat16 *cosT = (flags & 2) ? reinterpret_cast<const __nv_bfloat16 *>(d.p[5]) : nullptr;
-  const __nv_bfloat16 *sinT = (flags & 2) ? reinterpret_cast<const __nv_bfloat16 *>(d.p[6]) : nullptr;
-  __nv_bfloat16 *out = reinterpret_cast<__nv_bfloat16 *>(d.p[7]);
-  const int ldq = d.a[A_LDQKV], ldo = d.a[A_LDO];
-  const int rope_rows = d.a[A_ROPE_ROWS];
-  const int start = a.start, end = a.end, new_start = a.new_start, n_active = a.n_active;
-  const size_t head_base = (size_t)head * (G + 2) * 128;
-  float *w_ml = a.w_ml;
-  float *w_o = reinterpret_cast<float *>(a.stages);   // [8 warps][G][128], valid once every warp's stream has drained
-  uint8_t *new_k = a.new_tile, *new_v = a.new_tile + (size_t)a.new_rows_cap * kAsPitch;
-  const int new_lo = max(start, new_start);            // first position this task appends (if any: new_lo < end)
-  const bool aprof = P.profiler != nullptr && (uint64_t)(task + 1) * 8 <= P.profiler_entries && tid == 0;
-
-  // ---- append the new keys / values that fall into this chunk (cache + a tile in shared memory) ----
-  for (int pos = new_lo + warp; pos < end; pos += 8) {
-    const int tok = rv.q0 + (pos - new_start);
-    const __nv_bfloat16 *kp = qkv + (size_t)tok * ldq + head_base + (size_t)G * 128 + lane * 4;
-    const uint2 kr = __ldcg(reinterpret_cast<const uint2 *>(kp));
-    const uint2 vr = __ldcg(reinterpret_cast<const uint2 *>(kp + 128));
-    float x[4] = {bf16_lo(kr.x), bf16_hi(kr.x), bf16_lo(kr.y), bf16_hi(kr.y)};
-    uint2 cs = a.cs0, sn = a.sn0;
-    if (pos != new_start) load_rope(cosT, sinT, pos, rope_rows, lane, cs, sn);
-    norm_rope_head(x, kn, eps, cosT != nullptr, cs, sn, lane);
-    const uint2 kw = make_uint2(pack_bf16(x[0], x[1]), pack_bf16(x[2], x[3]));
-    const size_t off = kv_offset(P, d, rv, pos) + lane * 4;
-    *reinterpret_cast<uint2 *>(kc + off) = kw;
-    *reinterpret_cast<uint2 *>(vc + off) = vr;
-    const int r = pos - new_lo;
-    if (r < a.new_rows_cap) {
-      *reinterpret_cast<uint2 *>(new_k + (size_t)r * kAsPitch + lane * 8) = kw;
-      *reinterpret_cast<uint2 *>(new_v + (size_t)r * kAsPitch + lane * 8) = vr;
-    }
-  }
-  const int g = lane >> 2, q = lane & 3;
-  const int my_steps = a.w_end > a.w_begin ? (a.w_end - a.w_begin + kAsStepRows - 1) / kAsStepRows : 0;
-  bool first_pass = true;                    // the copies of the first pass were started before the dependency wait
-
-  for (int t = 0; t < rv.nq; ++t) {
-    const int pq = new_start + t;
-    const int tok = rv.q0 + t;
-    const int lim = min(end, pq + 1);
-    if (t > 0) consumer_sync();              // the combine of the previous token has read the stage area
-    if (warp < G) {
-      const __nv_bfloat16 *qp = qkv + (size_t)tok * ldq + head_base + (size_t)warp * 128 + lane * 4;
-      const uint2 qr = __ldcg(reinterpret_cast<const uint2 *>(qp));
-      float x[4] = {bf16_lo(qr.x), bf16_hi(qr.x), bf16_lo(qr.y), bf16_hi(qr.y)};
-      uint2 cs = a.cs0, sn = a.sn0;
-      if (t != 0) load_rope(cosT, sinT, pq, rope_rows, lane, cs, sn);
-      norm_rope_head(x, qn, eps, cosT != nullptr, cs, sn, lane);   // (results are bf16-rounded values)
-      *reinterpret_cast<uint2 *>(a.q_tile + (size_t)warp * kAsPitch + lane * 8) =
-          make_uint2(pack_bf16(x[0], x[1]), pack_bf16(x[2], x[3]));
-    }
-    consumer_sync();   // the q tile and the tile of new rows are ready
-    if (aprof && t == 0) P.profiler[(size_t)task * 8 + 4] = globaltimer_ns();
-    uint32_t qa[8][2];   // rows 0-7 of the A fragments of the eight k steps (rows 8-15 are zero)
-    {
-      const uint32_t q_addr = smem_u32(a.q_tile) + (uint32_t)((lane & 7) * kAsPitch + ((lane >> 3) & 1) * 16);
-#pragma unroll
-      for (int ks = 0; ks < 8; ++ks) ldmatrix_x2(qa[ks], q_addr + ks * 32u);
-    }
-    float m_run = -INFINITY, l_run = 0.f;
-    float o[16][4];
-#pragma unroll
-    for (int nt = 0; nt < 16; ++nt) o[nt][0] = o[nt][1] = o[nt][2] = o[nt][3] = 0.f;
-    // ---- this warp's share of the cached rows, step by step through its own stage ring ----
-    if (!first_pass) {
-      for (int j = 0; j < a.nstg - 1; ++j) attn_stream_issue(c, a, j, warp, lane);
-      a.issued = a.nstg - 1;
-    }
-    first_pass = false;
-    for (int j = 0; j < my_steps; ++j) {
-      attn_stream_wait(a.nstg);
-      __syncwarp();                                      // step j has landed for the whole warp; stage (j - 1) % nstg is free
-      attn_stream_issue(c, a, j + a.nstg - 1, warp, lane);
-      if (a.nstg == 1) {   // a single stage cannot run ahead: the step just requested is the one consumed now
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
-        __syncwarp();
-      }
-      const uint8_t *stg = a.stages + (size_t)(warp * a.nstg + j % a.nstg) * kAsStepBytes;
-      attn_step_mma(stg, stg + kAsStepRows * kAsPitch, min(kAsStepRows, a.w_end - (a.w_begin + j * kAsStepRows)), qa, m_run, l_run, o,
-                    lane);
-      __syncwarp();                                      // every lane is done reading the stage before it is refilled
-    }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    if (aprof && t == 0) P.profiler[(size_t)task * 8 + 5] = globaltimer_ns();
-    // ---- rows appended by this task (causal: query token t sees the new rows up to its own position): last warp ----
-    if (warp == 7 && new_lo < lim) {
-      const int n_new = min(lim - new_lo, a.new_rows_cap);
-      for (int r0 = 0; r0 < n_new; r0 += kAsStepRows)
-        attn_step_mma(new_k + (size_t)r0 * kAsPitch, new_v + (size_t)r0 * kAsPitch, min(kAsStepRows, n_new - r0), qa, m_run, l_run, o,
-                      lane);
-    }
-    consumer_sync();   // every warp's stream has drained: the stage area becomes the partial-output area
-    if (g < G) {
-      float *wo = &w_o[((size_t)warp * G + g) * 128 + 2 * q];
-#pragma unroll
-      for (int nt = 0; nt < 16; ++nt) *reinterpret_cast<float2 *>(wo + nt * 8) = make_float2(o[nt][0], o[nt][1]);
-      if (q == 0) {
-        w_ml[(warp * G + g) * 2 + 0] = m_run;
-        w_ml[(warp * G + g) * 2 + 1] = l_run;
-      }
-    }
-    consumer_sync();
-    if (aprof && t == 0) P.profiler[(size_t)task * 8 + 6] = globaltimer_ns();
-    // combine the 8 warps; thread -> (g, dim) pairs
-    for (int idx = tid; idx < G * 128; idx += kConsumerThreads) {
-      const int gg = idx >> 7, dd = idx & 127;
-      float M = -INFINITY;
-#pragma unroll
-      for (int w = 0; w < 8; ++w) M = fmaxf(M, w_ml[(w * G + gg) * 2]);
-      float Ls = 0.f, O = 0.f;
-#pragma unroll
-      for (int w = 0; w < 8; ++w) {
-        const float mw = w_ml[(w * G + gg) * 2];
-        const float scw = (mw == -INFINITY) ? 0.f : exp2f(mw - M);
-        Ls += w_ml[(w * G + gg) * 2 + 1] * scw;
-        O += w_o[((size_t)w * G + gg) * 128 + dd] * scw;
-      }
-      const int hq_idx = head * G + gg;
-      if (NC == 1) {
-        out[(size_t)tok * ldo + (size_t)hq_idx * 128 + dd] = __float2bfloat16_rn(Ls > 0.f ? O / Ls : 0.f);
-      } else {
-        const size_t base = ((size_t)tok * hq + hq_idx) * NC + chunk;
-        __stcg(&P.attn_scratch[base * 130 + 2 + dd], O);
-        if (dd == 0) {
-          __stcg(&P.attn_scratch[base * 130 + 0], M);
-          __stcg(&P.attn_scratch[base * 130 + 1], Ls);
+// Thread 0 acquires the task's events, then the compute warps meet (wait_dependencies, for bodies that take no Ctx).
+static __device__ __noinline__ bool af_wait(const KernelParams &P, const TaskDesc &d, unsigned long long iteration, uint64_t deadline, int *flags, int task) {
+  if (threadIdx.x == 0) {
+    bool good = flags[0] == 0;
+    for (int i = 0; i < kMaxDeps && good; ++i) {
+      const int ev = d.dep_event[i];
+      if (ev < 0) continue;
+      const unsigned long long need = (unsigned long long)d.dep_need[i] * iteration;
+      const bool remote = (d.flags & (TF_DEP0_REMOTE << i)) != 0;
+      uint32_t polls = 0;
+      while ((remote ? ld_acquire_sys(&P.counters[ev]) : ld_acquire_gpu(&P.counters[ev])) < need) {
+        if ((++polls & 0xff) != 0) continue;
+        if (ld_volatile_i32(&P.status->error) != 0) { good = false; break; }
+        if (globaltimer_ns() > deadline) {
+          report_timeout(P.status, (int)blockIdx.x, 1, task);
+          good = false;
+          break;
         }
       }
     }
-  }
-  if (NC == 1) return;
-  // ---- split-KV merge by the last chunk task to arrive ---------------------------
-  consumer_sync();
-  if (tid == 0) {
-    unsigned int old;
-    asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;"
-                 : "=r"(old)
-                 : "l"(&P.attn_tickets[d.a[A_TICKET] + d.a[A_SLOT] * d.a[A_HKV] + head])
-                 : "memory");
-    c.s.flags[1] = ((old + 1u) % (unsigned)NC == 0u) ? 1 : 0;
+    if (!good) flags[0] = 1;
+    *reinterpret_cast<volatile uint64_t *>(flags + 6) = globaltimer_ns();   // (profiler: dependencies satisfied)
   }
   consumer_sync();
-  if (c.s.flags[1] == 0) return;
-  for (int item = warp; item < rv.nq * G * 4; item += 8) {
-    const int row = item >> 2, dd = ((item & 3) << 5) + lane;
-    const int t = row / G, gg = row - t * G;
-    const int tok = rv.q0 + t;
-    const int hq_idx = head * G + gg;
-    const size_t base = ((size_t)tok * hq + hq_idx) * NC;
-    const bool v = lane < n_active;
-    const float m = v ? __ldcg(&P.attn_scratch[(base + lane) * 130]) : -INFINITY;
-    const float l = v ? __ldcg(&P.attn_scratch[(base + lane) * 130 + 1]) : 0.f;
-    float ow[16], ow2[16];
-#pragma unroll
-    for (int u = 0; u < 16; ++u)
-      ow[u] = (u < n_active) ? __ldcg(&P.attn_scratch[(base + u) * 130 + 2 + dd]) : 0.f;
-    if (n_active > 16) {
-#pragma unroll
-      for (int u = 0; u < 16; ++u)
-        ow2[u] = (16 + u < n_active) ? __ldcg(&P.attn_scratch[(base + 16 + u) * 130 + 2 + dd]) : 0.f;
-    }
-    float M = m;
-#pragma unroll
-    for (int o2 = 16; o2 > 0; o2 >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o2));
-    const float w = (m == -INFINITY) ? 0.f : exp2f(m - M);
-    const float Ls = warp_sum(l * w);
-    float O = 0.f;
-#pragma unroll
-    for (int u = 0; u < 16; ++u) O = fmaf(ow[u], __shfl_sync(0xffffffffu, w, u), O);
-    if (n_active > 16) {
-#pragma unroll
-      for (int u = 0; u < 16; ++u) O = fmaf(ow2[u], __shfl_sync(0xffffffffu, w, 16 + u), O);
-    }
-    out[(size_t)tok * ldo + (size_t)hq_idx * 128 + dd] = __float2bfloat16_rn(Ls > 0.f ? O / Ls : 0.f);
+  return *reinterpret_cast<volatile int *>(flags) == 0;
+}
+
+// Where a warp stands: tile (entry of the table, head group, query tile) and step, and what it needs of the request.
+struct AfCursor {
+  int e, h, i, s;            // table entry, head group, query tile, step
+  int kv0, nq, q0, len, S, I;
+  int pg, off;               // page of the step's first position, and the position within it
+};
+__device__ __forceinline__ void af_load(AfCursor &c, const AfTable &t, int G) {
+  const int4 r = t.req[c.e];
+  c.q0 = r.x; c.nq = r.y; c.kv0 = r.z; c.len = r.w;
+  c.S = (c.len + kAfRows - 1) / kAfRows;
+  c.I = (c.nq * G + 15) / 16;
+}
+__device__ __forceinline__ void af_next_tile(AfCursor &c, const AfTable &t, int G, int groups, int n) {
+  c.s = c.pg = c.off = 0;
+  if (++c.i < c.I) return;
+  c.i = 0;
+  if (++c.h < groups) return;
+  c.h = 0;
+  if (++c.e < n) af_load(c, t, G);
+}
+template <bool shared>
+__device__ __forceinline__ bool run_attention_steps(const KernelParams &P, const TaskDesc &d, uint8_t *xtile, int *sflags, const AfTable &tab, int n, int total,
+                                                    unsigned long long iteration, uint64_t deadline, int task) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+  const int hkv = d.a[A_HKV], G = d.a[A_HQ] / hkv, flags = d.a[A_FLAGS], page = (flags & 4) ? 1 << 30 : d.a[A_PAGE];
+  const int nstg = d.a[A_NSTAGE];
+  const uint32_t tile = (smem_u32(xtile) + 1023u) & ~1023u;
+  const int hh = af_heads(hkv), hw = warp & (hh - 1), groups = hkv / hh;   // this warp's head of every head group
+  const int ranges = P.num_workers * (8 / hh);
+  const int per = max((total + ranges - 1) / ranges, kAfMinSteps);
+  const int range = warp / hh * P.num_workers + d.a[A_CHUNK];
+  const int tiles = n > 0 ? tab.tile0[n] : 0, NC = shared && tiles > 0 ? max(1, P.num_workers / tiles) : 1;
+  int item = d.a[A_CHUNK];                                      // (tile, part) of this worker, then the one num_workers on
+  const int u0 = min(range * per, total);
+  int left = shared ? 0 : min(per, total - u0);                 // steps to consume
+  int flying = 0;                                               // requested steps that have not been consumed
+  const uint32_t qbuf = tile + (uint32_t)(warp * (nstg + 1) * kAfStage), ring = qbuf + kAfStage;
+  const uint32_t bars = smem_u32(sflags + 16) + (uint32_t)(warp * kAttnStages * 8);
+  const uint8_t *maps = reinterpret_cast<const uint8_t *>(P.tmaps) + (size_t)d.a[A_TMAP] * 128;
+  int *place = sflags + 16 + 16 * kAttnStages + warp;           // where this warp's ring stood after its last task: parities of the stages
+  uint32_t parity = *reinterpret_cast<volatile int *>(place);
+
+  AfCursor cur;
+  cur.e = cur.h = cur.i = cur.s = cur.pg = cur.off = 0;
+  cur.kv0 = cur.nq = cur.q0 = cur.len = 0;
+  cur.S = cur.I = 1;
+  int head = 0;                                                 // kv head
+  // this warp's steps of the worker's item
+  const auto take_item = [&]() {
+    const int k = item / NC, part = item - k * NC;
+    cur.e = -1;
+    for (int b = 0; b < n; b += 32) cur.e += __popc(__ballot_sync(0xffffffffu, b + lane < n && tab.tile0[b + lane] <= k));
+    af_load(cur, tab, G);
+    const int rest = k - tab.tile0[cur.e];
+    head = rest / cur.I;
+    cur.i = rest - head * cur.I;
+    const int a = cur.S * part / NC, b = cur.S * (part + 1) / NC, first = a + (b - a) * warp / 8;
+    left = a + (b - a) * (warp + 1) / 8 - first;
+    cur.s = first;
+    cur.pg = first * kAfRows / page;
+    cur.off = first * kAfRows - cur.pg * page;
+  };
+  if (shared) {
+    if (item < tiles * NC) take_item();
+  } else if (left > 0) {
+    // entry whose steps contain u0: the last one that begins at or before it
+    for (int k = 0; k < n; k += 32) cur.e += __popc(__ballot_sync(0xffffffffu, k + lane < n && tab.step0[k + lane] <= u0));
+    --cur.e;
+    af_load(cur, tab, G);
+    int u = u0 - tab.step0[cur.e];
+    cur.s = u % cur.S;
+    u /= cur.S;
+    cur.i = u % cur.I;
+    cur.h = u / cur.I;
+    cur.pg = cur.s * kAfRows / page;
+    cur.off = cur.s * kAfRows - cur.pg * page;
+    head = cur.h * hh + hw;
   }
+  AfCursor req = cur;                                           // the requesting cursor runs ahead
+  int togo = left;                                              // steps to request
+  int pg0 = 0, pages = 0;                                       // lane l holds the id of page pg0 + l of the requesting cursor's request
+  bool have = false;
+  int in_slot = 0;                                              // ring stage of the next request
+  bool ok = true;
+  const auto request = [&]() {
+    if (togo > 0 && ok) {
+      --togo;
+      ++flying;
+      const uint32_t bar = bars + (uint32_t)(in_slot * 8);
+      if (req.s * kAfRows < req.len - req.nq) {                 // some of its positions lie in the cache
+        int row;
+        if (flags & 4) {
+          row = req.kv0 * d.a[A_CSEQ] + req.off;
+        } else {
+          if (!have || req.pg < pg0 || req.pg >= pg0 + 32) {
+            pg0 = req.pg;
+            pages = req.pg + lane < (req.len + page - 1) / page ? __ldcg(&P.meta.paged_kv_indices[req.kv0 + req.pg + lane]) : 0;
+            have = true;
+          }
+          row = __shfl_sync(0xffffffffu, pages, req.pg - pg0) * page + req.off;
+        }
+        if (lane == 0) {
+          const uint32_t dst = ring + (uint32_t)(in_slot * kAfStage);
+          const int at = shared ? head : req.h * hh + hw;
+          bar_arrive_expect_tx(bar, kAfStage);
+          tma_load_3d_shared(dst, maps, 0, row, 2 * at, bar);
+          tma_load_3d_shared(dst + kAfTile, maps + 128, 0, row, 2 * at, bar);
+        }
+      } else if (lane == 0) {
+        bar_arrive(bar);
+      }
+      if (++in_slot == nstg) in_slot = 0;
+      req.off += kAfRows;
+      if (req.off >= page) { req.off = 0; ++req.pg; }
+      if (++req.s == req.S && !shared) {
+        const int e = req.e;
+        af_next_tile(req, tab, G, groups, n);
+        if (req.e != e) have = false;
+      }
+    }
+  };
+  for (int j = 0; j < nstg - 1; ++j) request();
+  ok = af_wait(P, d, iteration, deadline, sflags, task);
+  const bool run = ok;                                          // (the same in all warps)
+
+  // (pointers are read from the descriptor where they are used: registers)
+  const auto ptr = [&](int k, bool on) { return on ? reinterpret_cast<const __nv_bfloat16 *>(d.p[k]) : nullptr; };
+  const int ldq = d.a[A_LDQKV], ldo = d.a[A_LDO], rope_rows = d.a[A_ROPE_ROWS];
+  const float eps = __int_as_float(d.a[A_EPS]);
+  const int TP = 16 / G;                                        // tokens of a query tile
+  int out_slot = 0, unit = u0;
+  // (a warp whose wait was abandoned still takes part in the barriers of shared tiles)
+  while (run && (shared ? item < tiles * NC : ok && left > 0)) {
+    // ---- query tile of this segment: rows (token, head), normed and rotated ----
+    const int t0 = cur.i * TP, rows = min(16, (cur.nq - t0) * G), new_start = cur.len - cur.nq;
+    if (!shared) head = cur.h * hh + hw;
+    const size_t head0 = (size_t)head * (G + 2) * 128 + lane * 4;
+    // (warps that share a tile share it out, two rows each)
+    const uint32_t qtile = shared ? tile : qbuf;
+    const int rend = shared ? 2 : 16;
+    for (int r = 0; r < rend; r += 2) {
+      const __nv_bfloat16 *qkv = ptr(0, true), *qn = ptr(3, flags & 1), *cosT = ptr(5, flags & 2), *sinT = ptr(6, flags & 2);
+      uint2 x2[2], cs[2], sn[2];
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        const int row = shared ? warp + 8 * k : r + k;
+        x2[k] = make_uint2(0, 0);
+        if (r + k < rend && row < rows) {
+          load_rope(cosT, sinT, new_start + t0 + row / G, rope_rows, lane, cs[k], sn[k]);
+          x2[k] = __ldcg(reinterpret_cast<const uint2 *>(qkv + (size_t)(cur.q0 + t0 + row / G) * ldq + head0 + (size_t)(row % G) * 128));
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        const int row = shared ? warp + 8 * k : r + k;
+        if (r + k >= rend) continue;
+        if (row < rows) {
+          float x[4] = {bf16_lo(x2[k].x), bf16_hi(x2[k].x), bf16_lo(x2[k].y), bf16_hi(x2[k].y)};
+          norm_rope_head(x, qn, eps, cosT != nullptr, cs[k], sn[k], lane);
+          x2[k] = make_uint2(pack_bf16(x[0], x[1]), pack_bf16(x[2], x[3]));
+        }
+        asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(qtile + af_qpiece(row, lane >> 1) + (lane & 1) * 8), "r"(x2[k].x), "r"(x2[k].y) : "memory");
+      }
+    }
+    if (shared) consumer_sync();
+    __syncwarp();
+    const int lim0 = new_start + t0 + g / G, lim1 = new_start + t0 + (g + 8) / G;   // last position that row g / row g + 8 sees
+    float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f, o[16][4];
+#pragma unroll
+    for (int nt = 0; nt < 16; ++nt) o[nt][0] = o[nt][1] = o[nt][2] = o[nt][3] = 0.f;
+
+    const int seg = shared ? left : min(left, cur.S - cur.s), first_s = cur.s;
+    for (int j = 0; j < seg && ok; ++j) {
+      ok = wait_bar(P, bars + (uint32_t)(out_slot * 8), (parity >> out_slot) & 1u, deadline, task);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+      --flying;
+      request();                                                // (into the stage before this one, which the whole warp has left)
+      const uint32_t kt = ring + (uint32_t)(out_slot * kAfStage), vt = kt + kAfTile;
+      parity ^= 1u << out_slot;
+      if (++out_slot == nstg) out_slot = 0;
+      const int pos0 = (first_s + j) * kAfRows;
+      if (pos0 + kAfRows > new_start) {
+        // rows that this launch appends; behind them zeros (a masked position has weight 0, and 0 x NaN would still be NaN)
+        const int end = min(pos0 + kAfRows, cur.len);
+        for (int r = end - pos0; r < kAfRows; ++r) {
+          const uint32_t to = af_piece(r, lane >> 1) + (lane & 1) * 8;
+          asm volatile("st.shared.v2.b32 [%0], {%1, %1};" ::"r"(kt + to), "r"(0u) : "memory");
+          asm volatile("st.shared.v2.b32 [%0], {%1, %1};" ::"r"(vt + to), "r"(0u) : "memory");
+        }
+        for (int p0 = max(pos0, new_start); p0 < end; p0 += 2) {   // two rows' loads in flight
+          const __nv_bfloat16 *qkv = ptr(0, true), *kn = ptr(4, flags & 1), *cosT = ptr(5, flags & 2), *sinT = ptr(6, flags & 2);
+          uint2 kr[2], vr[2], cs[2], sn[2];
+#pragma unroll
+          for (int k = 0; k < 2; ++k) {
+            const int pos = min(p0 + k, end - 1);
+            const __nv_bfloat16 *kp = qkv + (size_t)(cur.q0 + pos - new_start) * ldq + head0 + (size_t)G * 128;
+            kr[k] = __ldcg(reinterpret_cast<const uint2 *>(kp));
+            vr[k] = __ldcg(reinterpret_cast<const uint2 *>(kp + 128));
+            load_rope(cosT, sinT, pos, rope_rows, lane, cs[k], sn[k]);
+          }
+#pragma unroll
+          for (int k = 0; k < 2; ++k) {
+            const int pos = p0 + k;
+            if (pos >= end) continue;
+            float x[4] = {bf16_lo(kr[k].x), bf16_hi(kr[k].x), bf16_lo(kr[k].y), bf16_hi(kr[k].y)};
+            norm_rope_head(x, kn, eps, cosT != nullptr, cs[k], sn[k], lane);
+            const uint2 kw = make_uint2(pack_bf16(x[0], x[1]), pack_bf16(x[2], x[3]));
+            const uint32_t to = af_piece(pos - pos0, lane >> 1) + (lane & 1) * 8;
+            asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(kt + to), "r"(kw.x), "r"(kw.y) : "memory");
+            asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(vt + to), "r"(vr[k].x), "r"(vr[k].y) : "memory");
+            if (cur.i == 0) {   // the first tile's warp writes the cache
+              size_t row;
+              if (flags & 4) row = (size_t)cur.kv0 * d.a[A_CSEQ] + pos;
+              else row = (size_t)__ldcg(&P.meta.paged_kv_indices[cur.kv0 + pos / page]) * page + pos % page;
+              const size_t off = (row * hkv + head) * 128 + lane * 4;
+              *reinterpret_cast<uint2 *>(reinterpret_cast<__nv_bfloat16 *>(d.p[1]) + off) = kw;
+              *reinterpret_cast<uint2 *>(reinterpret_cast<__nv_bfloat16 *>(d.p[2]) + off) = vr[k];
+            }
+          }
+        }
+        fence_proxy_async_smem();                               // these stores come before the copy that refills the stage
+        __syncwarp();
+      }
+      // ---- scores, online softmax, P V ----
+      float sc[4] = {0.f, 0.f, 0.f, 0.f}, sd[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int kk = 0; kk < 4; ++kk) {
+        uint32_t a[4], b[4];                                    // (the query fragments are read again each step: registers)
+        ldmatrix_x4(b, kt + af_piece(lane & 7, 4 * kk + (lane >> 3)));
+        ldmatrix_x4(a, qtile + af_qpiece(lane & 15, 4 * kk + (lane >> 4)));
+        mma_bf16_16816(sc, a, b[0], b[1]);
+        ldmatrix_x4(a, qtile + af_qpiece(lane & 15, 4 * kk + 2 + (lane >> 4)));
+        mma_bf16_16816(sd, a, b[2], b[3]);
+      }
+      const float qscale = 0.08838834764831845f * 1.4426950408889634f;   // 1/sqrt(128) * log2(e)
+      const int p = pos0 + 2 * q;
+      const float s0 = p <= lim0 ? (sc[0] + sd[0]) * qscale : -INFINITY, s1 = p + 1 <= lim0 ? (sc[1] + sd[1]) * qscale : -INFINITY;
+      const float s2 = p <= lim1 ? (sc[2] + sd[2]) * qscale : -INFINITY, s3 = p + 1 <= lim1 ? (sc[3] + sd[3]) * qscale : -INFINITY;
+      float x0 = fmaxf(s0, s1), x1 = fmaxf(s2, s3);
+      x0 = fmaxf(x0, __shfl_xor_sync(0xffffffffu, x0, 1));
+      x1 = fmaxf(x1, __shfl_xor_sync(0xffffffffu, x1, 1));
+      x0 = fmaxf(x0, __shfl_xor_sync(0xffffffffu, x0, 2));
+      x1 = fmaxf(x1, __shfl_xor_sync(0xffffffffu, x1, 2));
+      const float n0 = fmaxf(m0, x0), n1 = fmaxf(m1, x1);
+      const float z0 = n0 == -INFINITY ? 0.f : n0, z1 = n1 == -INFINITY ? 0.f : n1;   // (a row that sees nothing yet)
+      const float c0 = exp2f(m0 - z0), c1 = exp2f(m1 - z1);                            // 0 on the first step (m = -inf)
+      const float p0 = exp2f(s0 - z0), p1 = exp2f(s1 - z0), p2 = exp2f(s2 - z1), p3 = exp2f(s3 - z1);
+      l0 = l0 * c0 + p0 + p1;                                                           // (this lane's columns; summed over the quad at the end)
+      l1 = l1 * c1 + p2 + p3;
+      m0 = n0;
+      m1 = n1;
+      if (__any_sync(0xffffffffu, c0 != 1.f || c1 != 1.f)) {
+#pragma unroll
+        for (int nt = 0; nt < 16; ++nt) { o[nt][0] *= c0; o[nt][1] *= c0; o[nt][2] *= c1; o[nt][3] *= c1; }
+      }
+      const uint32_t pa = pack_bf16(p0, p1), pb = pack_bf16(p2, p3);
+#pragma unroll
+      for (int vq = 0; vq < 4; ++vq) {
+        uint32_t b[4];
+        ldmatrix_x4_trans(b, vt + af_piece(lane & 7, 4 * vq + (lane >> 3)));
+#pragma unroll
+        for (int k = 0; k < 4; ++k) mma_bf16_1688(o[4 * vq + k], pa, pb, b[k]);
+      }
+      __syncwarp();                                             // every lane is done with the stage before it is refilled
+    }
+    if (!ok && !shared) break;
+    l0 += __shfl_xor_sync(0xffffffffu, l0, 1);
+    l1 += __shfl_xor_sync(0xffffffffu, l1, 1);
+    l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
+    l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
+
+    // ---- results of the segment ----
+    __nv_bfloat16 *out = reinterpret_cast<__nv_bfloat16 *>(d.p[7]);
+    const size_t row_out = (size_t)(cur.q0 + t0) * ldo + (size_t)head * G * 128;
+    if (shared) {
+      // the eight warps' parts meet in shared memory: sums and maxima where the query tiles were, outputs in the rings (idle now)
+      consumer_sync();                                          // (the query tile has been read by all)
+      float *mine = reinterpret_cast<float *>(xtile + (ring - smem_u32(xtile))), *ml = reinterpret_cast<float *>(xtile + (qbuf - smem_u32(xtile)));
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        const int row = g + 8 * half;
+        if (row < rows) {
+          if (q == 0) { ml[2 * row] = half ? m1 : m0; ml[2 * row + 1] = half ? l1 : l0; }
+#pragma unroll
+          for (int nt = 0; nt < 16; ++nt) *reinterpret_cast<float2 *>(mine + row * 128 + nt * 8 + 2 * q) = make_float2(o[nt][2 * half], o[nt][2 * half + 1]);
+        }
+      }
+      consumer_sync();
+      const int k = item / NC, pitch = (nstg + 1) * kAfStage / 4;   // floats between two warps' areas
+      const float *ml0 = reinterpret_cast<const float *>(xtile + (tile - smem_u32(xtile)));
+      for (int idx = threadIdx.x; idx < rows * 128; idx += kConsumerThreads) {
+        const int row = idx >> 7, dim = idx & 127;
+        float M = -INFINITY, L = 0.f, O = 0.f;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) M = fmaxf(M, ml0[w * pitch + 2 * row]);
+        const float z = M == -INFINITY ? 0.f : M;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) {
+          const float e = exp2f(ml0[w * pitch + 2 * row] - z);
+          L += ml0[w * pitch + 2 * row + 1] * e;
+          O += ml0[w * pitch + kAfStage / 4 + row * 128 + dim] * e;
+        }
+        if (NC == 1) {
+          out[row_out + (size_t)(row / G) * ldo + (size_t)(row % G) * 128 + dim] = __float2bfloat16_rn(L > 0.f ? O / L : 0.f);
+        } else {
+          float *rec = P.attn_scratch + (size_t)item * kAfRecord + row * 132;
+          if (dim == 0) __stcg(reinterpret_cast<float2 *>(rec), make_float2(M, L));
+          __stcg(rec + 4 + dim, O);
+        }
+      }
+      if (NC > 1) {
+        consumer_sync();
+        if (threadIdx.x == 0) {
+          unsigned int old;
+          asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(old) : "l"(&P.attn_tickets[d.a[A_TICKET] + k]) : "memory");
+          const bool last = old + 1u == (unsigned)NC;
+          if (last) P.attn_tickets[d.a[A_TICKET] + k] = 0u;       // for the next launch
+          sflags[4] = last ? 1 : 0;
+        }
+        consumer_sync();
+        for (int idx = threadIdx.x; sflags[4] && idx < rows * 128; idx += kConsumerThreads) {
+          const int row = idx >> 7, dim = idx & 127;
+          const float *rec = P.attn_scratch + (size_t)(k * NC) * kAfRecord + row * 132;
+          float M = -INFINITY, L = 0.f, O = 0.f;
+          for (int c0 = 0; c0 < NC; c0 += 4) {
+            float2 pm[4];
+            float po[4];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+              const bool on = c0 + c < NC;
+              pm[c] = on ? __ldcg(reinterpret_cast<const float2 *>(rec + (size_t)(c0 + c) * kAfRecord)) : make_float2(-INFINITY, 0.f);
+              po[c] = on ? __ldcg(rec + (size_t)(c0 + c) * kAfRecord + 4 + dim) : 0.f;
+            }
+            float N = M;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) N = fmaxf(N, pm[c].x);
+            const float z = N == -INFINITY ? 0.f : N, w = exp2f(M - z);
+            L *= w;
+            O *= w;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+              const float e = exp2f(pm[c].x - z);
+              L += pm[c].y * e;
+              O += po[c] * e;
+            }
+            M = N;
+          }
+          out[row_out + (size_t)(row / G) * ldo + (size_t)(row % G) * 128 + dim] = __float2bfloat16_rn(L > 0.f ? O / L : 0.f);
+        }
+      }
+      item += P.num_workers;
+      left = 0;
+      if (item < tiles * NC) {
+        fence_proxy_async_smem();                               // the rings were written and read through the generic proxy
+        consumer_sync();
+        take_item();
+        req = cur;
+        togo = left;
+        have = false;
+        for (int j = 0; j < nstg - 1; ++j) request();
+      }
+      continue;
+    }
+    if (seg == cur.S) {
+      const float i0 = l0 > 0.f ? 1.f / l0 : 0.f, i1 = l1 > 0.f ? 1.f / l1 : 0.f;
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        const int row = g + 8 * half;
+        if (row < rows) {
+          __nv_bfloat16 *dst = out + row_out + (size_t)(row / G) * ldo + (size_t)(row % G) * 128 + 2 * q;
+#pragma unroll
+          for (int nt = 0; nt < 16; ++nt)
+            *reinterpret_cast<uint32_t *>(dst + nt * 8) = pack_bf16(o[nt][2 * half] * (half ? i1 : i0), o[nt][2 * half + 1] * (half ? i1 : i0));
+        }
+      }
+    } else {
+      // a range has at most two records: of the tile it begins in (0) and of the one it ends in (1)
+      float *rec = P.attn_scratch + (size_t)((2 * range + (unit == u0 ? 0 : 1)) * hh + hw) * kAfRecord;
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        const int row = g + 8 * half;
+        if (row < rows) {
+          float *dst = rec + row * 132;
+          if (q == 0) __stcg(reinterpret_cast<float2 *>(dst), half ? make_float2(m1, l1) : make_float2(m0, l0));
+#pragma unroll
+          for (int nt = 0; nt < 16; ++nt) __stcg(reinterpret_cast<float2 *>(dst + 4 + nt * 8 + 2 * q), make_float2(o[nt][2 * half], o[nt][2 * half + 1]));
+        }
+      }
+      __threadfence();
+      __syncwarp();
+      const int begin = unit - first_s, end = begin + cur.S;     // the tile's steps
+      const int r0 = begin / per, parts = (end - 1) / per - r0 + 1;
+      unsigned int *ticket = &P.attn_tickets[d.a[A_TICKET] + tab.tile0[cur.e] + head * cur.I + cur.i];
+      unsigned int old = 0;
+      if (lane == 0) asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(old) : "l"(ticket) : "memory");
+      old = __shfl_sync(0xffffffffu, old, 0);
+      if (old + 1u == (unsigned)parts) {
+        if (lane == 0) *ticket = 0u;                            // for the next launch
+        for (int row = 0; row < rows; ++row) {
+          float M = -INFINITY, L = 0.f;
+          float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+          for (int k0 = 0; k0 < parts; k0 += 8) {
+            float2 ml[8];
+            float4 ov[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+              ml[k] = make_float2(-INFINITY, 0.f);
+              ov[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+              if (k0 + k < parts) {
+                const int r = r0 + k0 + k;
+                const float *src = P.attn_scratch + (size_t)((2 * r + (begin <= r * per ? 0 : 1)) * hh + hw) * kAfRecord + row * 132;
+                ml[k] = __ldcg(reinterpret_cast<const float2 *>(src));
+                ov[k] = __ldcg(reinterpret_cast<const float4 *>(src + 4) + lane);
+              }
+            }
+            float N = M;
+#pragma unroll
+            for (int k = 0; k < 8; ++k) N = fmaxf(N, ml[k].x);
+            const float z = N == -INFINITY ? 0.f : N, w = exp2f(M - z);
+            L *= w; acc.x *= w; acc.y *= w; acc.z *= w; acc.w *= w;
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+              const float e = exp2f(ml[k].x - z);
+              L += ml[k].y * e;
+              acc.x += ov[k].x * e; acc.y += ov[k].y * e; acc.z += ov[k].z * e; acc.w += ov[k].w * e;
+            }
+            M = N;
+          }
+          const float inv = L > 0.f ? 1.f / L : 0.f;
+          *reinterpret_cast<uint2 *>(out + row_out + (size_t)(row / G) * ldo + (size_t)(row % G) * 128 + lane * 4) =
+              make_uint2(pack_bf16(acc.x * inv, acc.y * inv), pack_bf16(acc.z * inv, acc.w * inv));
+        }
+      }
+    }
+    left -= seg;
+    unit += seg;
+    cur.s += seg;
+    if (cur.s == cur.S) af_next_tile(cur, tab, G, groups, n);
+  }
+  if (!ok) {
+    // abandoned: what is in flight always arrives; wait for it, a bounded number of polls each
+    for (; flying > 0; --flying) {
+      uint32_t polls = 0;
+      while (!bar_try_wait(bars + (uint32_t)(out_slot * 8), (parity >> out_slot) & 1u) && ++polls < (1u << 22)) {}
+      parity ^= 1u << out_slot;
+      if (++out_slot == nstg) out_slot = 0;
+    }
+    sflags[0] = 1;
+    return false;
+  }
+  if (lane == 0) *place = (int)parity;
+  __syncwarp();
+  return true;
 }
 
-__device__ __forceinline__ void run_attention_stream(const Ctx &c, const TaskDesc &d, AttnStream &a, int task) {
-  attention_stream_body(c, d, a, task);
+static __device__ __forceinline__ bool run_attention_flat(const KernelParams &P, const TaskDesc &d, uint8_t *xtile, int *sflags, unsigned long long iteration,
+                                                          uint64_t deadline, int task) {
+  const int warp = threadIdx.x >> 5;
+  const int hkv = d.a[A_HKV], G = d.a[A_HQ] / hkv, flags = d.a[A_FLAGS];
+  AfHead *th = reinterpret_cast<AfHead *>(reinterpret_cast<uint8_t *>(sflags) - kFlagsOffset + kMiscBytes);
+  const AfTable tab = af_table(reinterpret_cast<uint8_t *>(th + 1), d.a[A_CAP]);
+  fence_proxy_async_smem();                                     // earlier generic accesses to the area come before its copies
+  if (warp == 0) {
+    const int4 k = th->key;
+    if (k.x != d.a[A_SLOT] || k.y != hkv || k.z != G || k.w != ((flags & 4) ? -d.a[A_PAGE] : d.a[A_PAGE])) af_build_table(P, d, tab, th);
+  }
+  consumer_sync();
+  const int n = th->n, total = n > 0 ? tab.step0[n] : 0;
+  // few steps to a range: the warps share tiles
+  if (total < P.num_workers * (8 / af_heads(hkv)) * kAfMinSteps) return run_attention_steps<true>(P, d, xtile, sflags, tab, n, total, iteration, deadline, task);
+  return run_attention_steps<false>(P, d, xtile, sflags, tab, n, total, iteration, deadline, task);
 }
 
-// ---------------------------------------------------------------------------
-// small tasks
-// ---------------------------------------------------------------------------
 static __device__ void run_embed(const Ctx &c, const TaskDesc &d) {
   const int B = active_tokens(c.P);
   const int t0 = d.a[E_T0], t1 = min(d.a[E_T1], B), width = d.a[E_WIDTH];
@@ -4163,18 +4388,15 @@ __device__ __forceinline__ bool task_attention(const Ctx &c, const TaskDesc &d, 
     ok = ok && (c.s.flags[0] == 0);
   }
   if (GENERAL) {
-    AttnStream as;
-    as.rv.nq = 0;
-    if (tt.on && threadIdx.x == 0) P.profiler[(size_t)t * 8 + 7] = globaltimer_ns();
-    if (ok) attention_stream_begin<GENERAL>(c, d, as, t);
-    ok = wait_dependencies(c, d, t, ok, tt);
-    if (ok) run_attention_stream(c, d, as, t);
-    asm volatile("cp.async.wait_group 0;" ::: "memory");   // (also on the abandoned path: nothing may stay in flight)
+    if (tt.on && threadIdx.x == 0) tt.begin_ns = globaltimer_ns();
+    if (!ok) return false;
+    ok = run_attention_flat(P, d, c.s.xtile, c.s.flags, c.iteration, c.deadline_ns, t);
+    if (tt.on && threadIdx.x == 0) tt.ready_ns = *reinterpret_cast<volatile uint64_t *>(c.s.flags + 6);
     return ok;
   }
   AttnPre pre;
   pre.rv.nq = 0;
-  if (ok) attention_prefetch<GENERAL>(c, d, pre, t);
+  if (ok) attention_prefetch(c, d, pre, t);
   if (threadIdx.x == 0) *reinterpret_cast<volatile int *>(&c.s.flags[2]) = 1;   // quiet the weight stream
   ok = wait_dependencies(c, d, t, ok, tt);
   if (ok) run_attention(c, d, pre, t);
@@ -4302,10 +4524,13 @@ __global__ void __launch_bounds__(block_threads(GENERAL), 1) mpk_megakernel(cons
     s.flags[0] = 0;
     s.flags[1] = 0;
     s.flags[2] = 0;
-    *reinterpret_cast<volatile int *>(&s.full[8]) = -1;   // attention stash: empty
-    if (GENERAL)
-      for (int i = 0; i < kStashRing; ++i) reinterpret_cast<volatile int *>(s.flags + 16)[i * 8] = -1;
-    if (GENERAL) mbar_init(s.acc_bar, 8);   // one tcgen05.commit per compute warp
+    if (!GENERAL) *reinterpret_cast<volatile int *>(&s.full[8]) = -1;   // attention stash: empty
+    if (GENERAL) {
+      mbar_init(s.acc_bar, 8);   // one tcgen05.commit per compute warp
+      for (int i = 0; i < 8 * kAttnStages; ++i) mbar_init(reinterpret_cast<uint64_t *>(s.flags + 16) + i, 1);
+      for (int i = 0; i < 8; ++i) s.flags[16 + 16 * kAttnStages + i] = 0;
+      if (P.attn_table_bytes) *reinterpret_cast<int *>(reinterpret_cast<uint8_t *>(s.flags) - kFlagsOffset + kMiscBytes) = -1;   // the request table: not built
+    }
     mbar_fence_init();
   }
   // graphs with tcgen05 tasks: warp 0 takes all 512 tensor-memory columns (one CTA per SM, so nothing else asks)

@@ -396,7 +396,7 @@ int mpk_compile(mpk_handle *h) {
   CompiledGraph &g = h->graph;
   if (g.num_stages > 8)   // entries 8.. of the 16-entry barrier arrays are scratch (attention stash, accumulator barrier)
     return set_err(h, MPK_ERR_UNSUPPORTED, "internal: more than 8 weight stages planned");
-  h->smem_bytes = g.num_stages * g.stage_bytes + g.x_tile_bytes + kPartialBytes + kMiscBytes;
+  h->smem_bytes = g.num_stages * g.stage_bytes + g.x_tile_bytes + kPartialBytes + kMiscBytes + g.attn_table_bytes;
   // 5. runtime buffers
   h->counters_bytes = ((uint64_t)g.num_events * 8 + 255) / 256 * 256;
   h->comm_bytes = h->counters_bytes + (uint64_t)2 * g.inbox_floats_per_buffer * 4 + 256;
@@ -457,6 +457,7 @@ int mpk_compile(mpk_handle *h) {
   P.num_stages = g.num_stages;
   P.stage_bytes = g.stage_bytes;
   P.x_tile_bytes = g.x_tile_bytes;
+  P.attn_table_bytes = g.attn_table_bytes;
   P.max_inflight = g.num_stages;
   P.general_kernel = g.general_kernel ? 1 : 0;
   P.hybrid = g.hybrid;

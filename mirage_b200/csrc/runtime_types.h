@@ -26,7 +26,7 @@ constexpr int kChunkColsMax = 2048;            // k extent of a chunk, at most (
 constexpr int kRowPadBytes = 16;               // shared-memory row padding: conflict-free ldmatrix
 constexpr int stage_bytes_for(int chunk_cols) { return kChunkRows * (chunk_cols * 2 + kRowPadBytes); }
 constexpr int kPartialBytes = 8 * 1024;        // per-task partial-sum slots
-constexpr int kMiscBytes = 1536;               // barriers, descriptors, flags (1 KB) + the attention stash ring
+constexpr int kMiscBytes = 1536;               // barriers, descriptors, flags (1 KB), then the barriers of the attention rings
 constexpr int kMaxLinearTokens = 64;           // eight mma n-tiles of 8 tokens, one per compute warp
 constexpr int kFp8TaskRows = 64;               // weight rows of one FP8 linear task (their scales are staged in shared memory)
 constexpr int kTcSlotBytes = 16 * 1024;        // weight ring slot of graphs whose linears run on tcgen05 (1 KB multiples: swizzle atoms)
@@ -34,6 +34,7 @@ constexpr int kTmemCols = 512;                 // tensor-memory columns a worker
 constexpr int kTcKBlock = 64;                  // bf16 columns of one 128-byte swizzle row (an e4m3 row holds 128)
 constexpr int kTcSfCols = 64;                  // tensor-memory columns kept for scale factors: 8 warps x (4 for A + 4 for B)
 constexpr int kTcAccCols = kTmemCols - kTcSfCols;   // columns available to the accumulators of a task
+constexpr int kAttnStages = 3;                 // copy stages of a warp's attention ring (general instantiation), at most
 constexpr int kTcFp8MaxTiles = 4;              // row tiles of one FP8 tcgen05 task (their scale words are staged in shared memory)
 
 enum TaskType : uint32_t {
@@ -205,8 +206,10 @@ enum { LR_POST = 13, LR_ADD = 14, LR_ROW = 16, L_CAP = 23, LR_BIAS = 24, LR_LDAD
 //  a[6] head_dim  a[7] page_size  a[8] flags(1 qk_norm, 2 rope, 4 contiguous cache)  a[9] ld_qkv
 //  a[10] ld_out  a[11] eps bits  a[12] rope table rows  a[13] cache seq (contiguous mode)
 //  a[14] ticket bank offset  a[15] event of the batching task (-1: none)  a[16] its arrivals per iteration
+//  general instantiation: one task per worker (run_attention_flat): a[0] batch slots  a[2] the task's number  a[17] copy stages of a warp  a[18] requests the table holds
+//  a[19] tensor map of the keys (the next one: the values)
 enum { A_SLOT = 0, A_HEAD, A_CHUNK, A_NCHUNK, A_HQ, A_HKV, A_HD, A_PAGE, A_FLAGS, A_LDQKV, A_LDO, A_EPS, A_ROPE_ROWS, A_CSEQ,
-       A_TICKET, A_EARLY_EV, A_EARLY_NEED };
+       A_TICKET, A_EARLY_EV, A_EARLY_NEED, A_NSTAGE, A_CAP, A_TMAP };
 // ---- TASK_EMBED / RMSNORM / SILU / ADD / INIT ---------------------------------
 //  rows [a[0],a[1]) of the token dimension, width a[2]; p[0] in  p[1] weight/second input  p[2] out
 //  a[3] ld_in  a[4] ld_out  a[5] eps bits | silu groups | vocab  a[6] ld_in2
@@ -377,6 +380,7 @@ struct KernelParams {
   const void *tmaps;                    // array of 128-byte tensor maps (one per tcgen05 linear task), 64-byte aligned
   int32_t use_tmem;                     // the graph has tcgen05 tasks: every worker CTA allocates tensor memory
   int32_t tc_tokens;                    // token rows of the activation operand tile (batched tokens rounded up to 16)
+  int32_t attn_table_bytes;             // area of the attention tasks' request table, behind the small things (general instantiation)
   int32_t meta_static;                  // the batch description is the caller's and final at launch (test mode, online_notoken):
                                         // the graph has no batching task
 };

@@ -82,6 +82,13 @@ struct Builder {
   // (these tasks keep no partial sums there), and the buffer may grow until five 16 KB ring slots remain (what the
   // 129 KB bf16 tile leaves as well): at 64 tokens that admits k tiles of 2048 instead of 1024, i.e. half as many
   // stage / drain pauses per task.
+  // Copy stages of a warp's attention ring (general instantiation): 64 KB in flight per worker with three; graphs of few tokens keep the
+  // room for their weight ring.
+  int attention_stages() const { return nb_max > 8 ? kAttnStages : 2; }
+  // Requests that can have tokens in one launch.
+  int attention_requests(const LayerInfo &l) const {
+    return std::min(l.op == MPK_OP_PAGED_ATTENTION ? cfg.max_num_batched_requests : std::max(l.grid[0], 1), std::max(cfg.max_num_batched_tokens, 1));
+  }
   static int64_t fp8_tc_tile_cap() { return (kSmemBudget - kMiscBytes - kPartialBytes - 5 * kTcSlotBytes) / 256 * 256; }
   int64_t linear_tile_bytes(int64_t K) const {
     return tc_linear(K) ? (int64_t)tc_np() * K * 2 : (int64_t)nb_max * (K * 2 + kRowPadBytes);
@@ -539,11 +546,10 @@ struct Builder {
       } else if (l.op == MPK_OP_ATTENTION || l.op == MPK_OP_PAGED_ATTENTION) {
         const int G = (int)(l.params[0] / l.params[1]);
         int64_t attn = (int64_t)G * (128 + 16 + 8 * 128) * 4 + (int64_t)cfg.max_num_batched_tokens * 512;
-        // the general instantiation streams cached K/V rows through 32 KB stages (two at least) beside the query
-        // heads, the per-warp maxima / sums, 256 page ids and the rows of the new tokens
+        // the general instantiation: a query tile and a ring of copy stages per warp, and the table of the requests
         if (general_graph()) {
-          const int64_t new_rows = (std::min(cfg.max_num_batched_tokens, 64) + 7) / 8 * 8;
-          attn = 8 * 272 + (int64_t)G * 64 + 1024 + 2 * new_rows * 272 + 2 * (8 * 2 * 8 * 272);   // two stages per warp
+          attn = 1024 + 8 * (attention_stages() + 1) * 4096;   // (1024: alignment)
+          g->attn_table_bytes = std::max(g->attn_table_bytes, (32 + 24 * attention_requests(l) + 8 + 255) / 256 * 256);
         }
         need = std::max(need, attn - kPartialBytes);
       }
@@ -551,7 +557,7 @@ struct Builder {
     if (!no_batch_task()) need = std::max<int64_t>(need, (int64_t)(16 * cfg.max_num_batched_requests + 20 + (cfg.mode == MPK_MODE_ONLINE ? cfg.total_num_requests : 0)) * 4 - kPartialBytes);
     need = (need + 255) / 256 * 256;
     // 64 KB stages (4 KB row segments) when at least three of them fit, else 32 KB stages
-    const int64_t room = kSmemBudget - kMiscBytes - kPartialBytes - need;
+    const int64_t room = kSmemBudget - kMiscBytes - g->attn_table_bytes - kPartialBytes - need;
     g->x_tile_bytes = (int)need;
     g->tc_tokens = tc_np();
     if (g->use_tmem) {
@@ -1108,26 +1114,40 @@ struct Builder {
     // task stays near 128 rows at full length (the rows a task prefetches before its dependency wait are its
     // cheapest ones; long serial chunks are latency-bound)
     int NC = std::max(1, W / std::max(slots * hkv, 1));
-    if (general_graph()) {
-      // streamed K/V: long chunks are cheap (a task's fixed part is paid once), so a (request, kv head) pair is cut
-      // only as far as it takes to occupy the workers, and into chunks of at most ~2048 positions so that requests
-      // of very different lengths still spread evenly
-      NC = std::max(NC, (max_seq + 2047) / 2048);
-    } else {
-      NC = std::max(NC, std::min((max_seq + 127) / 128, 16));
-    }
+    NC = std::max(NC, std::min((max_seq + 127) / 128, 16));
     NC = std::min(NC, std::max(1, max_seq / 32));
     NC = std::min(NC, 32);
     const int rope_rows = rope ? (int)T[l.t[5]].dim(0) : 1;
-    for (int s = 0; s < slots; ++s)
-      for (int h = 0; h < hkv; ++h)
+    // (general instantiation: one task per worker, each of its warps takes a range of all requests' steps)
+    const bool flat = general_graph();
+    int map = 0;
+    if (flat) {
+      NC = W;
+      // boxes of 8 positions x 128 columns over the rows of a cache, in the 128-byte-swizzled layout
+      map = (int)g->tmaps.size();
+      for (int t : {l.t[1], l.t[2]}) {
+        TmapSpec m;
+        m.base = (uint64_t)T[t].ptr;
+        m.rows = T[t].dim(0) * T[t].dim(1);
+        m.ld_bytes = (int64_t)hkv * 256;
+        m.kblocks = (int64_t)hkv * 2;
+        m.box_rows = 8;
+        m.box_kblocks = 2;
+        g->tmaps.push_back(m);
+      }
+    }
+    for (int s = 0; s < (flat ? 1 : slots); ++s)
+      for (int h = 0; h < (flat ? 1 : hkv); ++h)
         for (int c = 0; c < NC; ++c) {
           TaskDesc d = blank(TASK_ATTENTION, li);
           for (int i = 0; i < 8; ++i) d.p[i] = l.t[i] >= 0 ? (uint64_t)T[l.t[i]].ptr : 0;
-          d.a[A_SLOT] = s;
+          d.a[A_SLOT] = flat ? slots : s;
           d.a[A_HEAD] = h;
           d.a[A_CHUNK] = c;
           d.a[A_NCHUNK] = NC;
+          d.a[A_NSTAGE] = attention_stages();
+          d.a[A_CAP] = attention_requests(l);
+          d.a[A_TMAP] = map;
           d.a[A_HQ] = hq;
           d.a[A_HKV] = hkv;
           d.a[A_HD] = 128;
@@ -1143,9 +1163,14 @@ struct Builder {
           d.a[A_EARLY_NEED] = 1;
           put(((s * hkv + h) * NC + c + rot) % W, d, ex);
         }
-    g->attn_scratch_floats =
-        std::max<int64_t>(g->attn_scratch_floats, (int64_t)cfg.max_num_batched_tokens * hq * NC * 130);
-    g->attn_tickets = std::max<int64_t>(g->attn_tickets, (int64_t)slots * hkv);
+    if (flat) {
+      // two records per warp; a ticket per (kv head, 16-row query tile) of every request
+      g->attn_scratch_floats = std::max<int64_t>(g->attn_scratch_floats, (int64_t)W * 8 * 2 * 16 * 132);
+      g->attn_tickets = std::max<int64_t>(g->attn_tickets, (int64_t)hkv * (attention_requests(l) + cfg.max_num_batched_tokens * G / 16 + 1));
+    } else {
+      g->attn_scratch_floats = std::max<int64_t>(g->attn_scratch_floats, (int64_t)cfg.max_num_batched_tokens * hq * NC * 130);
+      g->attn_tickets = std::max<int64_t>(g->attn_tickets, (int64_t)slots * hkv);
+    }
     return MPK_OK;
   }
 

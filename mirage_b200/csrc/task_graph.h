@@ -94,6 +94,7 @@ struct CompiledGraph {
   int stage_bytes = 0;
   int chunk_cols = 0;                     // k extent of a streamed chunk, at most
   int x_tile_bytes = 0;
+  int attn_table_bytes = 0;               // request table of the attention tasks (general instantiation)
   int num_allreduce = 0;
   bool general_kernel = false;            // FP8 tasks or more than 8 batched tokens: needs the general instantiation
   int hybrid = 0;                         // HYB_* family: recurrent / extended-attention layers present

@@ -275,3 +275,55 @@ def test_paged_attention_long_context(mi, lens, new, hkv, max_seq, token_budget)
     # a second launch appends the same rows again and must reproduce the output bit for bit
     pk.run_test_mode()
     assert torch.equal(first, out)
+
+
+# kv heads that go together are powers of two; pages smaller and larger than a step of 8 positions; query tiles of 16 rows with one, some
+# and all of them in use; requests shorter than a step, idle slots, and many more tiles than workers share
+@pytest.mark.parametrize("hkv,G,page,lens,new", [
+    (1, 8, 8, [8, 1, 129, 17], [1, 1, 9, 3]),
+    (3, 2, 24, [65, 200, 7], [16, 30, 7]),
+    (16, 1, 64, [300, 40, 64], [17, 1, 1]),
+    (2, 4, 16, [(i * 97) % 611 + 1 for i in range(40)], [0 if i % 7 == 3 else 1 for i in range(40)]),
+    (8, 4, 64, [1500, 64], [60, 4]),
+    (4, 1, 32, [2100, 31, 33], [12, 31, 2]),
+])
+def test_paged_attention_ranges(mi, hkv, G, page, lens, new):
+    D, R, T = 128, len(lens), sum(new)
+    g = torch.Generator().manual_seed(sum(lens))
+    need = [(n + page - 1) // page for n in lens]
+    total = sum(need) + 2
+    perm = torch.randperm(total, generator=g).tolist()
+    indptr, qo = [0], [0]
+    for n, k in zip(new, need):
+        indptr.append(indptr[-1] + k)
+        qo.append(qo[-1] + n)
+    qkv = torch.randn(T, hkv * (G + 2) * D, generator=g).to(torch.bfloat16)
+    kc, vc = (torch.randn(total, page, hkv, D, generator=g).to(torch.bfloat16) for _ in range(2))
+    kc_ref, vc_ref = kc.clone(), vc.clone()
+    for r, n in enumerate(lens):      # what lies behind a request's cached rows is never used
+        for pos in range(n - new[r], need[r] * page):
+            kc[perm[indptr[r] + pos // page], pos % page] = vc[perm[indptr[r] + pos // page], pos % page] = float("nan")
+    cos, sin = ops.rope_tables(D, max(lens) + 1, 1e6)
+    qn, kn = _bf16(D, seed=14, scale=0.1, shift=1.0), _bf16(D, seed=15, scale=0.1, shift=1.0)
+    ref = torch.cat([ops.paged_attention_request(qkv[qo[r]:qo[r + 1]], kc_ref, vc_ref, perm[indptr[r]:indptr[r + 1]], lens[r], hkv * G, hkv,
+                                                 qn, kn, cos, sin, 1e-6) for r in range(R) if new[r]])
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    meta = {"qo_indptr_buffer": i32(qo), "paged_kv_indptr_buffer": i32(indptr), "paged_kv_indices_buffer": i32(perm),
+            "paged_kv_last_page_len_buffer": i32([(n - 1) % page + 1 for n in lens])}
+    pk = make_test_kernel(mi, max(T, 16), max_num_batched_requests=R, max_num_pages=total, page_size=page,
+                          max_seq_length=max(need) * page, meta_tensors=meta)
+    kc_d, vc_d, out = kc.cuda(), vc.cuda(), torch.zeros(T, hkv * G * D, dtype=torch.bfloat16, device="cuda")
+    pk.paged_attention_layer(
+        input=pk.attach_input(qkv.cuda(), "qkv"), k_cache=pk.attach_input(kc_d, "kc"), v_cache=pk.attach_input(vc_d, "vc"),
+        q_norm=pk.attach_input(qn.cuda(), "qn"), k_norm=pk.attach_input(kn.cuda(), "kn"), cos_pos_embed=pk.attach_input(cos.cuda(), "cos"),
+        sin_pos_embed=pk.attach_input(sin.cuda(), "sin"), output=pk.attach_input(out, "out"), grid_dim=(R, hkv, 1), block_dim=(128, 1, 1))
+    pk.compile()
+    pk.run_test_mode()
+    first = out.clone()
+    assert rel_err(out.cpu(), ref) <= TOL
+    for r, n in enumerate(lens):
+        for pos in range(n):
+            at = (perm[indptr[r] + pos // page], pos % page)
+            assert rel_err(kc_d[at].cpu(), kc_ref[at]) <= 1e-2 and torch.equal(vc_d[at].cpu(), vc_ref[at])
+    pk.run_test_mode()
+    assert torch.equal(first, out)
