@@ -327,3 +327,20 @@ def test_paged_attention_ranges(mi, hkv, G, page, lens, new):
             assert rel_err(kc_d[at].cpu(), kc_ref[at]) <= 1e-2 and torch.equal(vc_d[at].cpu(), vc_ref[at])
     pk.run_test_mode()
     assert torch.equal(first, out)
+
+
+# columns that start on no 16-byte boundary, fewer columns than a vector, fewer tokens than warps; equal maxima: the lowest column wins
+@pytest.mark.parametrize("T,V,parts", [(1, 37, 5), (3, 1000, 7), (9, 4099, 148), (64, 777, 3)])
+def test_argmax_partial_edges(mi, T, V, parts):
+    g = torch.Generator().manual_seed(V)
+    x = (torch.randint(-3, 4, (T, V), generator=g)).to(torch.bfloat16)
+    x[0] = float("-inf")
+    pk = make_test_kernel(mi, T)
+    pv, pi = pk.new_tensor((T, parts), name="pv"), pk.new_tensor((T, parts), dtype=mi.int64, name="pi")
+    out = torch.full((T, 1), -1, dtype=torch.int64, device="cuda")
+    pk.argmax_partial_layer(input=pk.attach_input(x.cuda(), "x"), output=(pv, pi), grid_dim=(parts, 1, 1), block_dim=(128, 1, 1))
+    pk.argmax_reduce_layer(input=(pv, pi), output=pk.attach_input(out, "out"), grid_dim=(1, 1, 1), block_dim=(128, 1, 1))
+    pk.compile()
+    pk.run_test_mode()
+    want = torch.stack([(row == row.max()).nonzero()[0, 0] for row in x.float()])
+    assert torch.equal(out[:, 0].cpu(), want)
