@@ -2285,6 +2285,43 @@ static __device__ void run_moe_mul_sum_add(const Ctx &c, const TaskDesc &d) {
   const float *w = reinterpret_cast<const float *>(d.p[1]);
   const __nv_bfloat16 *res = reinterpret_cast<const __nv_bfloat16 *>(d.p[3]);
   __nv_bfloat16 *out = reinterpret_cast<__nv_bfloat16 *>(d.p[2]);
+  if (((c0 | c1 | H | ldo | ldres) & 7) == 0 && ((d.p[0] | d.p[2] | d.p[3]) & 15) == 0 && topk <= 16) {
+    // Eight columns of a token a thread, the slots' rows in flight together: a task holds 64 columns of every token, and walked
+    // token by token, slot by slot it took 50 us for 32 tokens x 8 slots.  The sum runs in slot order as below.
+    const int nv = (c1 - c0) >> 3;
+    for (int i = threadIdx.x; i < nv * B; i += kConsumerThreads) {
+      const int b = i / nv, h = c0 + ((i - b * nv) << 3);
+      float acc[8];
+      uint4 r = make_uint4(0, 0, 0, 0);
+      if (res) r = __ldcg(reinterpret_cast<const uint4 *>(res + (size_t)b * ldres + h));
+      const uint32_t rw[4] = {r.x, r.y, r.z, r.w};
+#pragma unroll
+      for (int q = 0; q < 4; ++q) { acc[2 * q] = bf16_lo(rw[q]); acc[2 * q + 1] = bf16_hi(rw[q]); }
+      for (int k0 = 0; k0 < topk; k0 += 4) {
+        float wk[4];
+        uint4 x[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          wk[k] = k0 + k < topk ? __ldcg(&w[(size_t)b * ldw + k0 + k]) : 0.f;   // 0: the row may never have been written
+          x[k] = make_uint4(0, 0, 0, 0);
+          if (wk[k] != 0.f) x[k] = __ldcg(reinterpret_cast<const uint4 *>(in + ((size_t)b * topk + k0 + k) * H + h));
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          if (wk[k] == 0.f) continue;
+          const uint32_t xw[4] = {x[k].x, x[k].y, x[k].z, x[k].w};
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            acc[2 * q] += bf16_lo(xw[q]) * wk[k];
+            acc[2 * q + 1] += bf16_hi(xw[q]) * wk[k];
+          }
+        }
+      }
+      *reinterpret_cast<uint4 *>(out + (size_t)b * ldo + h) =
+          make_uint4(pack_bf16(acc[0], acc[1]), pack_bf16(acc[2], acc[3]), pack_bf16(acc[4], acc[5]), pack_bf16(acc[6], acc[7]));
+    }
+    return;
+  }
   for (int b = 0; b < B; ++b)
     for (int h = c0 + threadIdx.x; h < c1; h += kConsumerThreads) {
       float acc = res ? bf16_to_f(__ldcg(&res[(size_t)b * ldres + h])) : 0.f;

@@ -2016,7 +2016,8 @@ struct Builder {
           TaskDesc d = blank(TASK_MOE_MUL_SUM_ADD, li);
           d.p[0] = (uint64_t)x.ptr; d.p[1] = (uint64_t)w.ptr; d.p[2] = (uint64_t)y.ptr;
           d.p[3] = has_res ? (uint64_t)T[l.t[2]].ptr : 0;
-          d.a[0] = (int)((int64_t)H * i / nt); d.a[1] = (int)((int64_t)H * (i + 1) / nt); d.a[2] = H; d.a[3] = (int)x.dim(1);
+          const int unit = H % 8 == 0 ? 8 : 1;               // (16-byte vectors)
+          d.a[0] = (int)((int64_t)(H / unit) * i / nt) * unit; d.a[1] = (int)((int64_t)(H / unit) * (i + 1) / nt) * unit; d.a[2] = H; d.a[3] = (int)x.dim(1);
           d.a[4] = (int)y.ld(); d.a[5] = has_res ? (int)T[l.t[2]].ld() : 0; d.a[6] = (int)w.ld(); d.a[7] = (int)x.dim(0);
           put((i + rot) % W, d, ex);
         }
