@@ -3147,6 +3147,7 @@ __device__ __forceinline__ void run_attention(const Ctx &c, const TaskDesc &d, c
 constexpr int kAfRows = 8;                       // positions of a step
 constexpr int kAfTile = kAfRows * 256;           // K or V rows of a step: two blocks of 64 columns in the 128-byte swizzle of the tensor map
 constexpr int kAfStage = 2 * kAfTile;            // K rows, then V rows; also the 16 query rows of a tile
+constexpr uint32_t kAfWild = 1u << 31;           // bit of a warp's stage parities: values that are not finite have been set aside
 constexpr int kAfMinSteps = 16;                  // ranges of fewer steps: the warps of a worker share a tile instead (see below)
 constexpr int kAfRecord = 16 * 132;              // floats of a record: 16 rows x {max, sum, -, -, 128 outputs}
 
@@ -3465,7 +3466,10 @@ __device__ __forceinline__ bool run_attention_steps(const KernelParams &P, const
             const uint2 kw = make_uint2(pack_bf16(x[0], x[1]), pack_bf16(x[2], x[3]));
             const uint32_t to = af_piece(pos - pos0, lane >> 1) + (lane & 1) * 8;
             asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(kt + to), "r"(kw.x), "r"(kw.y) : "memory");
-            asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(vt + to), "r"(vr[k].x), "r"(vr[k].y) : "memory");
+            // (0 x infinity is NaN, for every query row of the tile: such values are zero here, and added to the rows that see them below)
+            const uint2 vs = make_uint2(finite_or_zero_bf16x2(vr[k].x), finite_or_zero_bf16x2(vr[k].y));
+            if (__any_sync(0xffffffffu, vs.x != vr[k].x || vs.y != vr[k].y)) parity |= kAfWild;
+            asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(vt + to), "r"(vs.x), "r"(vs.y) : "memory");
             if (cur.i == 0) {   // the first tile's warp writes the cache
               size_t row;
               if (flags & 4) row = (size_t)cur.kv0 * d.a[A_CSEQ] + pos;
@@ -3526,6 +3530,27 @@ __device__ __forceinline__ bool run_attention_steps(const KernelParams &P, const
     l1 += __shfl_xor_sync(0xffffffffu, l1, 1);
     l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
     l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
+
+    if (parity & kAfWild) {
+      // infinities and NaNs of the value rows that this segment appended
+      parity &= ~kAfWild;
+      const int end = min((first_s + seg) * kAfRows, cur.len);
+      for (int pos = max(first_s * kAfRows, new_start); pos < end; ++pos) {
+        const __nv_bfloat16 *vp = ptr(0, true) + (size_t)(cur.q0 + pos - new_start) * ldq + (size_t)(head * (G + 2) + G + 1) * 128 + 2 * q;
+#pragma unroll
+        for (int nt = 0; nt < 16; ++nt) {
+          const uint32_t v = __ldcg(reinterpret_cast<const uint32_t *>(vp + 8 * nt)), w = finite_or_zero_bf16x2(v) ^ v;
+          if (w & 0xffffu) {
+            if (pos <= lim0) o[nt][0] += bf16_lo(v);
+            if (pos <= lim1) o[nt][2] += bf16_lo(v);
+          }
+          if (w >> 16) {
+            if (pos <= lim0) o[nt][1] += bf16_hi(v);
+            if (pos <= lim1) o[nt][3] += bf16_hi(v);
+          }
+        }
+      }
+    }
 
     // ---- results of the segment ----
     __nv_bfloat16 *out = reinterpret_cast<__nv_bfloat16 *>(d.p[7]);

@@ -277,6 +277,64 @@ def test_paged_attention_long_context(mi, lens, new, hkv, max_seq, token_budget)
     assert torch.equal(first, out)
 
 
+class _Ranges:
+    """One paged attention layer over requests of `lens` positions, the last new[r] of them appended by the launch."""
+
+    def __init__(self, mi, hkv, G, page, lens, new, **kw):
+        self.hkv, self.G, self.page, self.lens, self.new = hkv, G, page, lens, new
+        D, R, T = 128, len(lens), sum(new)
+        g = torch.Generator().manual_seed(sum(lens))
+        need = [(n + page - 1) // page for n in lens]
+        total = sum(need) + 2
+        self.perm = perm = torch.randperm(total, generator=g).tolist()
+        self.indptr, self.qo = [0], [0]
+        for n, k in zip(new, need):
+            self.indptr.append(self.indptr[-1] + k)
+            self.qo.append(self.qo[-1] + n)
+        self.qkv = torch.randn(T, hkv * (G + 2) * D, generator=g).to(torch.bfloat16)
+        kc, vc = (torch.randn(total, page, hkv, D, generator=g).to(torch.bfloat16) for _ in range(2))
+        self.kc_ref, self.vc_ref = kc.clone(), vc.clone()
+        for r, n in enumerate(lens):      # what lies behind a request's cached rows is never used
+            for pos in range(n - new[r], need[r] * page):
+                kc[self.row(r, pos)] = vc[self.row(r, pos)] = float("nan")
+        self.tables = ops.rope_tables(D, max(lens) + 1, 1e6)
+        self.qn, self.kn = _bf16(D, seed=14, scale=0.1, shift=1.0), _bf16(D, seed=15, scale=0.1, shift=1.0)
+        i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+        meta = {"qo_indptr_buffer": i32(self.qo), "paged_kv_indptr_buffer": i32(self.indptr), "paged_kv_indices_buffer": i32(perm),
+                "paged_kv_last_page_len_buffer": i32([(n - 1) % page + 1 for n in lens])}
+        self.pk = pk = make_test_kernel(mi, max(T, 16), max_num_batched_requests=R, max_num_pages=total, page_size=page,
+                                        max_seq_length=max(need) * page, meta_tensors=meta, **kw)
+        self.qkv_d, self.kc, self.vc = self.qkv.cuda(), kc.cuda(), vc.cuda()
+        self.out = torch.zeros(T, hkv * G * D, dtype=torch.bfloat16, device="cuda")
+        att = lambda t, name: pk.attach_input(t, name)
+        pk.paged_attention_layer(
+            input=att(self.qkv_d, "qkv"), k_cache=att(self.kc, "kc"), v_cache=att(self.vc, "vc"), q_norm=att(self.qn.cuda(), "qn"),
+            k_norm=att(self.kn.cuda(), "kn"), cos_pos_embed=att(self.tables[0].cuda(), "cos"), sin_pos_embed=att(self.tables[1].cuda(), "sin"),
+            output=att(self.out, "out"), grid_dim=(R, hkv, 1), block_dim=(128, 1, 1))
+        pk.compile()
+
+    def row(self, r, pos):
+        return self.perm[self.indptr[r] + pos // self.page], pos % self.page
+
+    def launch(self):
+        self.pk.run_test_mode()
+        return self.out.clone()
+
+    def reference(self):
+        return torch.cat([ops.paged_attention_request(self.qkv[self.qo[r]:self.qo[r + 1]], self.kc_ref, self.vc_ref, self.perm[self.indptr[r]:self.indptr[r + 1]],
+                                                      n, self.hkv * self.G, self.hkv, self.qn, self.kn, *self.tables, 1e-6)
+                          for r, n in enumerate(self.lens) if self.new[r]])
+
+    def check(self):
+        ref, first = self.reference(), self.launch()
+        assert rel_err(first.cpu(), ref) <= TOL
+        for r, n in enumerate(self.lens):
+            for pos in range(n):
+                at = self.row(r, pos)
+                assert rel_err(self.kc[at].cpu(), self.kc_ref[at]) <= 1e-2 and torch.equal(self.vc[at].cpu(), self.vc_ref[at])
+        assert torch.equal(first, self.launch())
+
+
 # kv heads that go together are powers of two; pages smaller and larger than a step of 8 positions; query tiles of 16 rows with one, some
 # and all of them in use; requests shorter than a step, idle slots, and many more tiles than workers share
 @pytest.mark.parametrize("hkv,G,page,lens,new", [
@@ -288,45 +346,25 @@ def test_paged_attention_long_context(mi, lens, new, hkv, max_seq, token_budget)
     (4, 1, 32, [2100, 31, 33], [12, 31, 2]),
 ])
 def test_paged_attention_ranges(mi, hkv, G, page, lens, new):
-    D, R, T = 128, len(lens), sum(new)
-    g = torch.Generator().manual_seed(sum(lens))
-    need = [(n + page - 1) // page for n in lens]
-    total = sum(need) + 2
-    perm = torch.randperm(total, generator=g).tolist()
-    indptr, qo = [0], [0]
-    for n, k in zip(new, need):
-        indptr.append(indptr[-1] + k)
-        qo.append(qo[-1] + n)
-    qkv = torch.randn(T, hkv * (G + 2) * D, generator=g).to(torch.bfloat16)
-    kc, vc = (torch.randn(total, page, hkv, D, generator=g).to(torch.bfloat16) for _ in range(2))
-    kc_ref, vc_ref = kc.clone(), vc.clone()
-    for r, n in enumerate(lens):      # what lies behind a request's cached rows is never used
-        for pos in range(n - new[r], need[r] * page):
-            kc[perm[indptr[r] + pos // page], pos % page] = vc[perm[indptr[r] + pos // page], pos % page] = float("nan")
-    cos, sin = ops.rope_tables(D, max(lens) + 1, 1e6)
-    qn, kn = _bf16(D, seed=14, scale=0.1, shift=1.0), _bf16(D, seed=15, scale=0.1, shift=1.0)
-    ref = torch.cat([ops.paged_attention_request(qkv[qo[r]:qo[r + 1]], kc_ref, vc_ref, perm[indptr[r]:indptr[r + 1]], lens[r], hkv * G, hkv,
-                                                 qn, kn, cos, sin, 1e-6) for r in range(R) if new[r]])
-    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
-    meta = {"qo_indptr_buffer": i32(qo), "paged_kv_indptr_buffer": i32(indptr), "paged_kv_indices_buffer": i32(perm),
-            "paged_kv_last_page_len_buffer": i32([(n - 1) % page + 1 for n in lens])}
-    pk = make_test_kernel(mi, max(T, 16), max_num_batched_requests=R, max_num_pages=total, page_size=page,
-                          max_seq_length=max(need) * page, meta_tensors=meta)
-    kc_d, vc_d, out = kc.cuda(), vc.cuda(), torch.zeros(T, hkv * G * D, dtype=torch.bfloat16, device="cuda")
-    pk.paged_attention_layer(
-        input=pk.attach_input(qkv.cuda(), "qkv"), k_cache=pk.attach_input(kc_d, "kc"), v_cache=pk.attach_input(vc_d, "vc"),
-        q_norm=pk.attach_input(qn.cuda(), "qn"), k_norm=pk.attach_input(kn.cuda(), "kn"), cos_pos_embed=pk.attach_input(cos.cuda(), "cos"),
-        sin_pos_embed=pk.attach_input(sin.cuda(), "sin"), output=pk.attach_input(out, "out"), grid_dim=(R, hkv, 1), block_dim=(128, 1, 1))
-    pk.compile()
-    pk.run_test_mode()
-    first = out.clone()
-    assert rel_err(out.cpu(), ref) <= TOL
-    for r, n in enumerate(lens):
-        for pos in range(n):
-            at = (perm[indptr[r] + pos // page], pos % page)
-            assert rel_err(kc_d[at].cpu(), kc_ref[at]) <= 1e-2 and torch.equal(vc_d[at].cpu(), vc_ref[at])
-    pk.run_test_mode()
-    assert torch.equal(first, out)
+    _Ranges(mi, hkv, G, page, lens, new).check()
+
+
+# one worker: ranges of steps; all of them: the warps of a worker share a tile
+@pytest.mark.parametrize("workers", [1, 0])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_paged_attention_value_rows_that_are_not_finite(mi, workers, bad):
+    """A value row reaches the tokens that see its position and no others, bit for bit."""
+    hkv, G, lens, new = 2, 1, [300, 40], [21, 5]
+    a = _Ranges(mi, hkv, G, 16, lens, new, num_workers=workers)
+    clean = a.launch()
+    values = a.qkv_d.view(-1, hkv, G + 2, 128)[:, :, G + 1]
+    for token, head, column in ((6, 0, 3), (13, 1, 127), (20, 0, 64), (22, 1, 0)):
+        values[token, head, column] = bad
+    out, sees = a.launch().view(-1, hkv, 128), clean.view(-1, hkv, 128).clone()
+    for first, last, head, column in ((6, 21, 0, 3), (13, 21, 1, 127), (20, 21, 0, 64), (22, 26, 1, 0)):
+        assert not out[first:last, head, column].isfinite().any()
+        sees[first:last, head, column] = out[first:last, head, column]
+    assert torch.equal(out.nan_to_num(7.0, 8.0), sees.nan_to_num(7.0, 8.0))
 
 
 # columns that start on no 16-byte boundary, fewer columns than a vector, fewer tokens than warps; equal maxima: the lowest column wins
