@@ -3645,6 +3645,14 @@ __device__ __forceinline__ bool run_attention_steps(const KernelParams &P, const
       continue;
     }
     if (seg == cur.S) {
+      // (a row whose sum is not positive, or NaN, is zero in every form)
+      if (!(l0 > 0.f && l1 > 0.f)) {
+#pragma unroll
+        for (int nt = 0; nt < 16; ++nt) {
+          if (!(l0 > 0.f)) o[nt][0] = o[nt][1] = 0.f;
+          if (!(l1 > 0.f)) o[nt][2] = o[nt][3] = 0.f;
+        }
+      }
       const float i0 = l0 > 0.f ? 1.f / l0 : 0.f, i1 = l1 > 0.f ? 1.f / l1 : 0.f;
 #pragma unroll
       for (int half = 0; half < 2; ++half) {
@@ -3709,6 +3717,7 @@ __device__ __forceinline__ bool run_attention_steps(const KernelParams &P, const
             }
             M = N;
           }
+          if (!(L > 0.f)) acc = make_float4(0.f, 0.f, 0.f, 0.f);
           const float inv = L > 0.f ? 1.f / L : 0.f;
           *reinterpret_cast<uint2 *>(out + row_out + (size_t)(row / G) * ldo + (size_t)(row % G) * 128 + lane * 4) =
               make_uint2(pack_bf16(acc.x * inv, acc.y * inv), pack_bf16(acc.z * inv, acc.w * inv));

@@ -367,6 +367,20 @@ def test_paged_attention_value_rows_that_are_not_finite(mi, workers, bad):
     assert torch.equal(out.nan_to_num(7.0, 8.0), sees.nan_to_num(7.0, 8.0))
 
 
+# (1 worker: tiles that lie in one range and tiles that are merged)
+@pytest.mark.parametrize("workers", [1, 0])
+def test_paged_attention_key_row_that_is_nan(mi, workers):
+    """Rows of tokens that see a NaN score are zero, whichever way the positions are shared out; the others keep their bits."""
+    a = _Ranges(mi, 2, 1, 16, [300, 40, 90], [21, 5, 2], num_workers=workers)
+    clean = a.launch().view(-1, 2, 128)
+    keys = a.qkv_d.view(-1, 2, 3, 128)[:, :, 1]
+    for token, head in ((6, 0), (22, 1), (26, 0)):
+        keys[token, head] = float("nan")
+    for first, last, head in ((6, 21, 0), (22, 26, 1), (26, 28, 0)):
+        clean[first:last, head] = 0
+    assert torch.equal(a.launch().view(-1, 2, 128), clean)
+
+
 # columns that start on no 16-byte boundary, fewer columns than a vector, fewer tokens than warps; equal maxima: the lowest column wins
 @pytest.mark.parametrize("T,V,parts", [(1, 37, 5), (3, 1000, 7), (9, 4099, 148), (64, 777, 3)])
 def test_argmax_partial_edges(mi, T, V, parts):
