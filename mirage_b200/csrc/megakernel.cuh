@@ -3686,6 +3686,7 @@ __device__ __forceinline__ bool run_attention_steps(const KernelParams &P, const
       if (lane == 0) asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(old) : "l"(ticket) : "memory");
       old = __shfl_sync(0xffffffffu, old, 0);
       if (old + 1u == (unsigned)parts) {
+        __syncwarp();                                           // lane 0's acquire holds for all of them: a shuffle orders no memory
         if (lane == 0) *ticket = 0u;                            // for the next launch
         for (int row = 0; row < rows; ++row) {
           float M = -INFINITY, L = 0.f;
