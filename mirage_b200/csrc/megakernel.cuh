@@ -3138,8 +3138,8 @@ __device__ __forceinline__ void run_attention(const Ctx &c, const TaskDesc &d, c
 // to arrive (a ticket per tile) merges.  Per step: S = Q K^T on mma.sync m16n8k16, online softmax (fp32, base 2), P rounded to bf16 as the
 // reference does (tasks/blackwell/attention_sm100.cuh:558), O += P V on m16n8k8 with V through ldmatrix.trans.
 // Where that leaves a range fewer than kAfMinSteps steps, the latency of a few steps in a row and of merging many parts through L2 is what
-// counts.  Then a worker takes a tile of one kv head (or one of NC parts of it, where there are fewer tiles than workers), its eight warps
-// share the positions and combine in shared memory.
+// counts.  Then a worker takes a tile of one kv head, or one of the parts of a tile whose steps exceed a worker's average (af_parts), its eight
+// warps share the positions and combine in shared memory.
 // Measured, us per layer, before (one task per request, head and chunk) and now: 16 requests of 512 to 4000 positions 76 -> 56,
 // 64 of 512 to 1536 109 -> 75 (3.6 TB/s), 32 + 32 prompt tokens behind 1000 and 343 positions 235 -> 39, 24 requests of 60 positions 14.8 -> 11.8, 41 of
 // 94 to 214 positions with 4 kv heads 14.4 -> 12.4.  The two ways are instantiations of their own and rows are prepared two at a time:
@@ -3165,25 +3165,33 @@ __device__ __forceinline__ void ldmatrix_x2(uint32_t (&r)[2], uint32_t smem_addr
 }
 
 // Table of the requests that have tokens, behind the other small areas of shared memory: {q0, tokens, kv0 (contiguous caches: slot), length}, then
-// the first step of each (and the total), then the first tile.  The order is that of the batch slots, the same in every worker.  Warp 0
+// the first step of each (and the total; shared tiles: the first item), then the first tile, then the first record of shared tiles.  The order is that of the batch slots, the same in every worker.  Warp 0
 // builds it in the first attention task of a launch (three round trips to L2); it holds for every layer with the same geometry.
 struct AfTable {
   int4 *req;
-  int *step0, *tile0;
+  int *step0, *tile0, *rec0;
 };
 struct AfHead {              // in front of the table: what it was built for (slots, kv heads, query heads, page | contiguous), then the
-  int4 key;                  // number of its entries
-  int n, pad[3];
+  int4 key;                  // number of its entries, the steps, the items of shared tiles (0: ranges)
+  int n, total, items, pad;
 };
 __device__ __forceinline__ AfTable af_table(uint8_t *base, int cap) {
   AfTable t;
   t.req = reinterpret_cast<int4 *>(base);
   t.step0 = reinterpret_cast<int *>(base + cap * 16);
   t.tile0 = t.step0 + cap + 1;
+  t.rec0 = t.tile0 + cap + 1;
   return t;
 }
 // kv heads that go together: the largest power of two, eight at most, that divides their number.
 __device__ __forceinline__ int af_heads(int hkv) { return min(hkv & -hkv, 8); }
+// Shared tiles: parts of a tile of S steps, of `tile_steps` in all.  As many whole shares of a worker as it holds, so that a long request
+// among short ones is cut however many tiles there are; every part leaves the last one to arrive a record, so no more than 16 and one for
+// each 96 steps, and 64 in all.  The parts of cut tiles, each with a record, are no more than the workers.
+// Measured, every tile cut into workers / tiles parts and now: 6 layers, 8 kv heads, one request of 16000 positions and 15 of 64 2163 -> 1022 us; one layer alone,
+// one request, 1 kv head, 1000 positions 80 -> 35 us, 16000 84 -> 50, 100000 94 -> 76.  Caps tried there: 16, 24 and 32 parts 35, 39 and 41 us at
+// 1000 positions, 53, 51 and 51 at 16000, 121, 98 and 88 at 100000 (64: 76); in a model of 4 kv heads, 16000 positions, 23, 31, 36 and 37 parts 19.2, 18.3, 17.3 and 15.0.
+__device__ __forceinline__ int af_parts(int S, int workers, int tile_steps) { return max(1, min(S * workers / tile_steps, min(16 + S / 96, 64))); }
 __device__ __forceinline__ void af_build_table(const KernelParams &P, const TaskDesc &d, const AfTable &t, AfHead *head) {
   const int lane = threadIdx.x & 31, slots = d.a[A_SLOT], G = d.a[A_HQ] / d.a[A_HKV], hkv = d.a[A_HKV], page = d.a[A_PAGE], hh = af_heads(hkv);
   int n = 0, steps = 0, tiles = 0;
@@ -3221,11 +3229,39 @@ __device__ __forceinline__ void af_build_table(const KernelParams &P, const Task
     n += __popc(bal);
   }
   n = min(n, d.a[A_CAP]);
+  int items = 0;
+  if (steps < P.num_workers * (8 / hh) * kAfMinSteps) {   // few steps to a range: the warps share tiles
+    int recs = 0;
+    __syncwarp();
+    for (int e0 = 0; e0 < n; e0 += 32) {
+      const int e = e0 + lane;
+      int parts = 0, nt = 0;
+      if (e < n) {
+        nt = hkv * ((t.req[e].y * G + 15) / 16);
+        parts = af_parts((t.req[e].w + kAfRows - 1) / kAfRows, P.num_workers, steps * hh);
+      }
+      int it = nt * parts, ir = parts > 1 ? it : 0;
+      const int own = it, rec = ir;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int a = __shfl_up_sync(0xffffffffu, it, o), b = __shfl_up_sync(0xffffffffu, ir, o);
+        if (lane >= o) { it += a; ir += b; }
+      }
+      if (e < n) {
+        t.step0[e] = items + it - own;
+        t.rec0[e] = recs + ir - rec;
+      }
+      items += __shfl_sync(0xffffffffu, it, 31);
+      recs += __shfl_sync(0xffffffffu, ir, 31);
+    }
+  }
   if (lane == 0) {
-    t.step0[n] = steps;
+    t.step0[n] = items ? items : steps;
     t.tile0[n] = tiles;
     head->key = make_int4(slots, hkv, G, (d.a[A_FLAGS] & 4) ? -page : page);
     head->n = n;
+    head->total = steps;
+    head->items = items;
   }
 }
 
@@ -3277,7 +3313,7 @@ __device__ __forceinline__ void af_next_tile(AfCursor &c, const AfTable &t, int 
   if (++c.e < n) af_load(c, t, G);
 }
 template <bool shared>
-__device__ __forceinline__ bool run_attention_steps(const KernelParams &P, const TaskDesc &d, uint8_t *xtile, int *sflags, const AfTable &tab, int n, int total,
+__device__ __forceinline__ bool run_attention_steps(const KernelParams &P, const TaskDesc &d, uint8_t *xtile, int *sflags, const AfTable &tab, int n, int total, int items,
                                                     unsigned long long iteration, uint64_t deadline, int task) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
   const int hkv = d.a[A_HKV], G = d.a[A_HQ] / hkv, flags = d.a[A_FLAGS], page = (flags & 4) ? 1 << 30 : d.a[A_PAGE];
@@ -3287,8 +3323,7 @@ __device__ __forceinline__ bool run_attention_steps(const KernelParams &P, const
   const int ranges = P.num_workers * (8 / hh);
   const int per = max((total + ranges - 1) / ranges, kAfMinSteps);
   const int range = warp / hh * P.num_workers + d.a[A_CHUNK];
-  const int tiles = n > 0 ? tab.tile0[n] : 0, NC = shared && tiles > 0 ? max(1, P.num_workers / tiles) : 1;
-  int item = d.a[A_CHUNK];                                      // (tile, part) of this worker, then the one num_workers on
+  int item = d.a[A_CHUNK], NC = 1;                              // (tile, part) of this worker, then the one num_workers on; parts of its tile
   const int u0 = min(range * per, total);
   int left = shared ? 0 : min(per, total - u0);                 // steps to consume
   int flying = 0;                                               // requested steps that have not been consumed
@@ -3305,13 +3340,13 @@ __device__ __forceinline__ bool run_attention_steps(const KernelParams &P, const
   int head = 0;                                                 // kv head
   // this warp's steps of the worker's item
   const auto take_item = [&]() {
-    const int k = item / NC, part = item - k * NC;
     cur.e = -1;
-    for (int b = 0; b < n; b += 32) cur.e += __popc(__ballot_sync(0xffffffffu, b + lane < n && tab.tile0[b + lane] <= k));
+    for (int b = 0; b < n; b += 32) cur.e += __popc(__ballot_sync(0xffffffffu, b + lane < n && tab.step0[b + lane] <= item));
     af_load(cur, tab, G);
-    const int rest = k - tab.tile0[cur.e];
-    head = rest / cur.I;
-    cur.i = rest - head * cur.I;
+    NC = af_parts(cur.S, P.num_workers, total * hh);
+    const int k = (item - tab.step0[cur.e]) / NC, part = item - tab.step0[cur.e] - k * NC;
+    head = k / cur.I;
+    cur.i = k - head * cur.I;
     const int a = cur.S * part / NC, b = cur.S * (part + 1) / NC, first = a + (b - a) * warp / 8;
     left = a + (b - a) * (warp + 1) / 8 - first;
     cur.s = first;
@@ -3319,7 +3354,7 @@ __device__ __forceinline__ bool run_attention_steps(const KernelParams &P, const
     cur.off = first * kAfRows - cur.pg * page;
   };
   if (shared) {
-    if (item < tiles * NC) take_item();
+    if (item < items) take_item();
   } else if (left > 0) {
     // entry whose steps contain u0: the last one that begins at or before it
     for (int k = 0; k < n; k += 32) cur.e += __popc(__ballot_sync(0xffffffffu, k + lane < n && tab.step0[k + lane] <= u0));
@@ -3388,7 +3423,7 @@ __device__ __forceinline__ bool run_attention_steps(const KernelParams &P, const
   const int TP = 16 / G;                                        // tokens of a query tile
   int out_slot = 0, unit = u0;
   // (a warp whose wait was abandoned still takes part in the barriers of shared tiles)
-  while (run && (shared ? item < tiles * NC : ok && left > 0)) {
+  while (run && (shared ? item < items : ok && left > 0)) {
     // ---- query tile of this segment: rows (token, head), normed and rotated ----
     const int t0 = cur.i * TP, rows = min(16, (cur.nq - t0) * G), new_start = cur.len - cur.nq;
     if (!shared) head = cur.h * hh + hw;
@@ -3569,7 +3604,7 @@ __device__ __forceinline__ bool run_attention_steps(const KernelParams &P, const
         }
       }
       consumer_sync();
-      const int k = item / NC, pitch = (nstg + 1) * kAfStage / 4;   // floats between two warps' areas
+      const int pitch = (nstg + 1) * kAfStage / 4;               // floats between two warps' areas
       const float *ml0 = reinterpret_cast<const float *>(xtile + (tile - smem_u32(xtile)));
       for (int idx = threadIdx.x; idx < rows * 128; idx += kConsumerThreads) {
         const int row = idx >> 7, dim = idx & 127;
@@ -3586,42 +3621,43 @@ __device__ __forceinline__ bool run_attention_steps(const KernelParams &P, const
         if (NC == 1) {
           out[row_out + (size_t)(row / G) * ldo + (size_t)(row % G) * 128 + dim] = __float2bfloat16_rn(L > 0.f ? O / L : 0.f);
         } else {
-          float *rec = P.attn_scratch + (size_t)item * kAfRecord + row * 132;
+          float *rec = P.attn_scratch + (size_t)(tab.rec0[cur.e] + item - tab.step0[cur.e]) * kAfRecord + row * 132;
           if (dim == 0) __stcg(reinterpret_cast<float2 *>(rec), make_float2(M, L));
           __stcg(rec + 4 + dim, O);
         }
       }
       if (NC > 1) {
         consumer_sync();
+        const int k = head * cur.I + cur.i;
         if (threadIdx.x == 0) {
-          unsigned int old;
-          asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(old) : "l"(&P.attn_tickets[d.a[A_TICKET] + k]) : "memory");
+          unsigned int old, *ticket = &P.attn_tickets[d.a[A_TICKET] + tab.tile0[cur.e] + k];
+          asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(old) : "l"(ticket) : "memory");
           const bool last = old + 1u == (unsigned)NC;
-          if (last) P.attn_tickets[d.a[A_TICKET] + k] = 0u;       // for the next launch
+          if (last) *ticket = 0u;                                // for the next launch
           sflags[4] = last ? 1 : 0;
         }
         consumer_sync();
         for (int idx = threadIdx.x; sflags[4] && idx < rows * 128; idx += kConsumerThreads) {
           const int row = idx >> 7, dim = idx & 127;
-          const float *rec = P.attn_scratch + (size_t)(k * NC) * kAfRecord + row * 132;
+          const float *rec = P.attn_scratch + (size_t)(tab.rec0[cur.e] + k * NC) * kAfRecord + row * 132;
           float M = -INFINITY, L = 0.f, O = 0.f;
-          for (int c0 = 0; c0 < NC; c0 += 4) {
-            float2 pm[4];
-            float po[4];
+          for (int c0 = 0; c0 < NC; c0 += 8) {
+            float2 pm[8];
+            float po[8];
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
+            for (int c = 0; c < 8; ++c) {
               const bool on = c0 + c < NC;
               pm[c] = on ? __ldcg(reinterpret_cast<const float2 *>(rec + (size_t)(c0 + c) * kAfRecord)) : make_float2(-INFINITY, 0.f);
               po[c] = on ? __ldcg(rec + (size_t)(c0 + c) * kAfRecord + 4 + dim) : 0.f;
             }
             float N = M;
 #pragma unroll
-            for (int c = 0; c < 4; ++c) N = fmaxf(N, pm[c].x);
+            for (int c = 0; c < 8; ++c) N = fmaxf(N, pm[c].x);
             const float z = N == -INFINITY ? 0.f : N, w = exp2f(M - z);
             L *= w;
             O *= w;
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
+            for (int c = 0; c < 8; ++c) {
               const float e = exp2f(pm[c].x - z);
               L += pm[c].y * e;
               O += po[c] * e;
@@ -3633,7 +3669,7 @@ __device__ __forceinline__ bool run_attention_steps(const KernelParams &P, const
       }
       item += P.num_workers;
       left = 0;
-      if (item < tiles * NC) {
+      if (item < items) {
         fence_proxy_async_smem();                               // the rings were written and read through the generic proxy
         consumer_sync();
         take_item();
@@ -3758,10 +3794,9 @@ static __device__ __forceinline__ bool run_attention_flat(const KernelParams &P,
     if (k.x != d.a[A_SLOT] || k.y != hkv || k.z != G || k.w != ((flags & 4) ? -d.a[A_PAGE] : d.a[A_PAGE])) af_build_table(P, d, tab, th);
   }
   consumer_sync();
-  const int n = th->n, total = n > 0 ? tab.step0[n] : 0;
-  // few steps to a range: the warps share tiles
-  if (total < P.num_workers * (8 / af_heads(hkv)) * kAfMinSteps) return run_attention_steps<true>(P, d, xtile, sflags, tab, n, total, iteration, deadline, task);
-  return run_attention_steps<false>(P, d, xtile, sflags, tab, n, total, iteration, deadline, task);
+  const int n = th->n, total = th->total, items = th->items;
+  if (total == 0 || items > 0) return run_attention_steps<true>(P, d, xtile, sflags, tab, n, total, items, iteration, deadline, task);
+  return run_attention_steps<false>(P, d, xtile, sflags, tab, n, total, items, iteration, deadline, task);
 }
 
 static __device__ void run_embed(const Ctx &c, const TaskDesc &d) {

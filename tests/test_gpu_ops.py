@@ -349,6 +349,31 @@ def test_paged_attention_ranges(mi, hkv, G, page, lens, new):
     _Ranges(mi, hkv, G, page, lens, new).check()
 
 
+def _form(hkv, G, lens, new, workers):
+    """How the layer's steps are shared out: steps of a range (0: the warps of a worker share tiles), parts per tile, tiles and parts in all."""
+    hh, workers = min(hkv & -hkv, 8), workers or torch.cuda.get_device_properties(0).multi_processor_count
+    live = [(hkv * -(-t * G // 16), -(-n // 8)) for n, t in zip(lens, new) if t]
+    steps, ranges = sum(nt // hh * S for nt, S in live), workers * (8 // hh)
+    if steps >= ranges * 16:
+        return -(-steps // ranges), [], 0
+    parts = [max(1, min(S * workers // (steps * hh), 16 + S // 96, 64)) for _, S in live]
+    return 0, parts, sum(nt * p for (nt, _), p in zip(live, parts))
+
+
+# one long request among short ones: tiles of several parts beside whole ones, and more of them than workers
+@pytest.mark.parametrize("workers,hkv,G,page,lens,new", [
+    (8, 2, 4, 16, [20] * 9 + [700] + [23] * 11, [1] * 4 + [0, 3] + [1] * 15),
+    (0, 8, 4, 64, [3000] + [40] * 18, [1] * 19),
+    (0, 4, 8, 8, [1200] + [9, 30] * 20, [3] + [1, 2] * 20),
+    (16, 3, 1, 24, [3, 500, 3, 1, 3, 17, 9], [3, 20, 1, 1, 2, 17, 0]),
+])
+def test_paged_attention_unequal_requests(mi, workers, hkv, G, page, lens, new):
+    a = _Ranges(mi, hkv, G, page, lens, new, num_workers=workers)
+    per, parts, items = _form(hkv, G, lens, new, workers)
+    assert per == 0 and max(parts) > 1 and min(parts) == 1 and items > (workers or 148)
+    a.check()
+
+
 # one worker: ranges of steps; all of them: the warps of a worker share a tile
 @pytest.mark.parametrize("workers", [1, 0])
 @pytest.mark.parametrize("bad", [float("nan"), float("inf")])
