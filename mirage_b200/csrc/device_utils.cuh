@@ -219,6 +219,7 @@ __device__ __forceinline__ void consumer_sync() { asm volatile("bar.sync 1, 256;
 
 __device__ __forceinline__ float bf16_lo(uint32_t v) { return __uint_as_float(v << 16); }
 __device__ __forceinline__ float bf16_hi(uint32_t v) { return __uint_as_float(v & 0xffff0000u); }
+__device__ __forceinline__ bool finite_bf16x2(uint32_t v) { return (v & 0x7f80u) != 0x7f80u && (v & 0x7f800000u) != 0x7f800000u; }
 __device__ __forceinline__ uint32_t finite_or_zero_bf16x2(uint32_t v) {
   return ((v & 0x7f80u) == 0x7f80u ? 0u : v & 0xffffu) | ((v & 0x7f800000u) == 0x7f800000u ? 0u : v & 0xffff0000u);
 }

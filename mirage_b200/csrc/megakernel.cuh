@@ -3147,7 +3147,7 @@ __device__ __forceinline__ void run_attention(const Ctx &c, const TaskDesc &d, c
 constexpr int kAfRows = 8;                       // positions of a step
 constexpr int kAfTile = kAfRows * 256;           // K or V rows of a step: two blocks of 64 columns in the 128-byte swizzle of the tensor map
 constexpr int kAfStage = 2 * kAfTile;            // K rows, then V rows; also the 16 query rows of a tile
-constexpr uint32_t kAfWild = 1u << 31;           // bit of a warp's stage parities: values that are not finite have been set aside
+constexpr uint32_t kAfWild = 1u << 31;           // bit of a warp's stage parities: values that are not finite have been set aside (af_put_back)
 constexpr int kAfMinSteps = 16;                  // ranges of fewer steps: the warps of a worker share a tile instead (see below)
 constexpr int kAfRecord = 16 * 132;              // floats of a record: 16 rows x {max, sum, -, -, 128 outputs}
 
@@ -3164,25 +3164,20 @@ __device__ __forceinline__ void ldmatrix_x2(uint32_t (&r)[2], uint32_t smem_addr
   asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(smem_addr));
 }
 
-// Table of the requests that have tokens, behind the other small areas of shared memory: {q0, tokens, kv0 (contiguous caches: slot), length}, then
-// the first step of each (and the total; shared tiles: the first item), then the first tile, then the first record of shared tiles.  The order is that of the batch slots, the same in every worker.  Warp 0
+// Table of the requests that have tokens, behind the other small areas of shared memory: two vectors in front, [0] what it was built for
+// (slots, kv heads, query heads of one, page | contiguous) and [1] the number of entries, the steps, the items of shared tiles (0: ranges); then two
+// vectors an entry, {first token, tokens, kv0 (contiguous caches: slot), length} and {first step (shared tiles: item), first tile,
+// first record, parts of a tile}.  The order is that of the batch slots, the same in every worker.  Warp 0
 // builds it in the first attention task of a launch (three round trips to L2); it holds for every layer with the same geometry.
+// One pointer and counts that are read where they are used: held in registers they were spilled in the loop over the steps.
 struct AfTable {
-  int4 *req;
-  int *step0, *tile0, *rec0;
+  int4 *at;
+  __device__ __forceinline__ int n() const { return at[1].x; }
+  __device__ __forceinline__ int total() const { return at[1].y; }
+  __device__ __forceinline__ int items() const { return at[1].z; }
+  __device__ __forceinline__ int4 &req(int e) const { return at[2 * e + 2]; }
+  __device__ __forceinline__ int4 &pos(int e) const { return at[2 * e + 3]; }
 };
-struct AfHead {              // in front of the table: what it was built for (slots, kv heads, query heads, page | contiguous), then the
-  int4 key;                  // number of its entries, the steps, the items of shared tiles (0: ranges)
-  int n, total, items, pad;
-};
-__device__ __forceinline__ AfTable af_table(uint8_t *base, int cap) {
-  AfTable t;
-  t.req = reinterpret_cast<int4 *>(base);
-  t.step0 = reinterpret_cast<int *>(base + cap * 16);
-  t.tile0 = t.step0 + cap + 1;
-  t.rec0 = t.tile0 + cap + 1;
-  return t;
-}
 // kv heads that go together: the largest power of two, eight at most, that divides their number.
 __device__ __forceinline__ int af_heads(int hkv) { return min(hkv & -hkv, 8); }
 // Shared tiles: parts of a tile of S steps, of `tile_steps` in all.  As many whole shares of a worker as it holds, so that a long request
@@ -3192,7 +3187,7 @@ __device__ __forceinline__ int af_heads(int hkv) { return min(hkv & -hkv, 8); }
 // one request, 1 kv head, 1000 positions 80 -> 35 us, 16000 84 -> 50, 100000 94 -> 76.  Caps tried there: 16, 24 and 32 parts 35, 39 and 41 us at
 // 1000 positions, 53, 51 and 51 at 16000, 121, 98 and 88 at 100000 (64: 76); in a model of 4 kv heads, 16000 positions, 23, 31, 36 and 37 parts 19.2, 18.3, 17.3 and 15.0.
 __device__ __forceinline__ int af_parts(int S, int workers, int tile_steps) { return max(1, min(S * workers / tile_steps, min(16 + S / 96, 64))); }
-__device__ __forceinline__ void af_build_table(const KernelParams &P, const TaskDesc &d, const AfTable &t, AfHead *head) {
+static __device__ __noinline__ void af_build_table(const KernelParams &P, const TaskDesc &d, const AfTable t) {
   const int lane = threadIdx.x & 31, slots = d.a[A_SLOT], G = d.a[A_HQ] / d.a[A_HKV], hkv = d.a[A_HKV], page = d.a[A_PAGE], hh = af_heads(hkv);
   int n = 0, steps = 0, tiles = 0;
   for (int s0 = 0; s0 < slots; s0 += 32) {
@@ -3220,9 +3215,8 @@ __device__ __forceinline__ void af_build_table(const KernelParams &P, const Task
       if (lane >= o) { it += a; is += b; }
     }
     if (on && at < d.a[A_CAP]) {
-      t.req[at] = r;
-      t.step0[at] = steps + is - ns;
-      t.tile0[at] = tiles + it - nt;
+      t.req(at) = r;
+      t.pos(at) = make_int4(steps + is - ns, tiles + it - nt, 0, 1);
     }
     steps += __shfl_sync(0xffffffffu, is, 31);
     tiles += __shfl_sync(0xffffffffu, it, 31);
@@ -3237,8 +3231,8 @@ __device__ __forceinline__ void af_build_table(const KernelParams &P, const Task
       const int e = e0 + lane;
       int parts = 0, nt = 0;
       if (e < n) {
-        nt = hkv * ((t.req[e].y * G + 15) / 16);
-        parts = af_parts((t.req[e].w + kAfRows - 1) / kAfRows, P.num_workers, steps * hh);
+        nt = hkv * ((t.req(e).y * G + 15) / 16);
+        parts = af_parts((t.req(e).w + kAfRows - 1) / kAfRows, P.num_workers, steps * hh);
       }
       int it = nt * parts, ir = parts > 1 ? it : 0;
       const int own = it, rec = ir;
@@ -3248,20 +3242,17 @@ __device__ __forceinline__ void af_build_table(const KernelParams &P, const Task
         if (lane >= o) { it += a; ir += b; }
       }
       if (e < n) {
-        t.step0[e] = items + it - own;
-        t.rec0[e] = recs + ir - rec;
+        t.pos(e).x = items + it - own;
+        t.pos(e).z = recs + ir - rec;
+        t.pos(e).w = parts;
       }
       items += __shfl_sync(0xffffffffu, it, 31);
       recs += __shfl_sync(0xffffffffu, ir, 31);
     }
   }
   if (lane == 0) {
-    t.step0[n] = items ? items : steps;
-    t.tile0[n] = tiles;
-    head->key = make_int4(slots, hkv, G, (d.a[A_FLAGS] & 4) ? -page : page);
-    head->n = n;
-    head->total = steps;
-    head->items = items;
+    t.at[0] = make_int4(slots, hkv, G, (d.a[A_FLAGS] & 4) ? -page : page);
+    t.at[1] = make_int4(n, steps, items, 0);
   }
 }
 
@@ -3299,21 +3290,38 @@ struct AfCursor {
   int pg, off;               // page of the step's first position, and the position within it
 };
 __device__ __forceinline__ void af_load(AfCursor &c, const AfTable &t, int G) {
-  const int4 r = t.req[c.e];
+  const int4 r = t.req(c.e);
   c.q0 = r.x; c.nq = r.y; c.kv0 = r.z; c.len = r.w;
   c.S = (c.len + kAfRows - 1) / kAfRows;
   c.I = (c.nq * G + 15) / 16;
 }
-__device__ __forceinline__ void af_next_tile(AfCursor &c, const AfTable &t, int G, int groups, int n) {
+__device__ __forceinline__ void af_next_tile(AfCursor &c, const AfTable &t, int G, int groups) {
   c.s = c.pg = c.off = 0;
   if (++c.i < c.I) return;
   c.i = 0;
   if (++c.h < groups) return;
   c.h = 0;
-  if (++c.e < n) af_load(c, t, G);
+  if (++c.e < t.n()) af_load(c, t, G);
 }
+// Infinities and NaNs of the value rows of positions pos .. end - 1, which the products took for zeros (0 x infinity is NaN, for every query
+// row of a tile): each goes to the rows of the tile that see its position (`first`: of the tile's first token).  Out of line, on parts in
+// memory: as code of the segment, on the accumulators, it cost 16 requests of 512 to 4000 positions 2 us a layer.
+static __device__ __noinline__ void af_put_back(const __nv_bfloat16 *v, int ldq, int pos, int end, int first, int G, int rows, float *acc, int pitch) {
+  __syncwarp();
+  for (; pos < end; ++pos, v += ldq)
+    for (int col = threadIdx.x & 31; col < 128; col += 32) {
+      const float x = bf16_to_f(__ldcg(v + col));
+      if (fabsf(x) < INFINITY) continue;
+      for (int row = max(pos - first, 0) * G; row < rows; ++row) {
+        volatile float *to = acc + row * pitch + col;
+        *to = *to + x;
+      }
+    }
+  __syncwarp();
+}
+
 template <bool shared>
-__device__ __forceinline__ bool run_attention_steps(const KernelParams &P, const TaskDesc &d, uint8_t *xtile, int *sflags, const AfTable &tab, int n, int total, int items,
+__device__ __forceinline__ bool run_attention_steps(const KernelParams &P, const TaskDesc &d, uint8_t *xtile, int *sflags, const AfTable &tab,
                                                     unsigned long long iteration, uint64_t deadline, int task) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
   const int hkv = d.a[A_HKV], G = d.a[A_HQ] / hkv, flags = d.a[A_FLAGS], page = (flags & 4) ? 1 << 30 : d.a[A_PAGE];
@@ -3321,9 +3329,9 @@ __device__ __forceinline__ bool run_attention_steps(const KernelParams &P, const
   const uint32_t tile = (smem_u32(xtile) + 1023u) & ~1023u;
   const int hh = af_heads(hkv), hw = warp & (hh - 1), groups = hkv / hh;   // this warp's head of every head group
   const int ranges = P.num_workers * (8 / hh);
-  const int per = max((total + ranges - 1) / ranges, kAfMinSteps);
+  const int total = tab.total(), per = max((total + ranges - 1) / ranges, kAfMinSteps);
   const int range = warp / hh * P.num_workers + d.a[A_CHUNK];
-  int item = d.a[A_CHUNK], NC = 1;                              // (tile, part) of this worker, then the one num_workers on; parts of its tile
+  int item = d.a[A_CHUNK];                                      // (tile, part) of this worker, then the one num_workers on
   const int u0 = min(range * per, total);
   int left = shared ? 0 : min(per, total - u0);                 // steps to consume
   int flying = 0;                                               // requested steps that have not been consumed
@@ -3341,10 +3349,10 @@ __device__ __forceinline__ bool run_attention_steps(const KernelParams &P, const
   // this warp's steps of the worker's item
   const auto take_item = [&]() {
     cur.e = -1;
-    for (int b = 0; b < n; b += 32) cur.e += __popc(__ballot_sync(0xffffffffu, b + lane < n && tab.step0[b + lane] <= item));
+    for (int b = 0, n = tab.n(); b < n; b += 32) cur.e += __popc(__ballot_sync(0xffffffffu, b + lane < n && tab.pos(b + lane).x <= item));
     af_load(cur, tab, G);
-    NC = af_parts(cur.S, P.num_workers, total * hh);
-    const int k = (item - tab.step0[cur.e]) / NC, part = item - tab.step0[cur.e] - k * NC;
+    const int4 at = tab.pos(cur.e);
+    const int NC = at.w, k = (item - at.x) / NC, part = item - at.x - k * NC;
     head = k / cur.I;
     cur.i = k - head * cur.I;
     const int a = cur.S * part / NC, b = cur.S * (part + 1) / NC, first = a + (b - a) * warp / 8;
@@ -3354,13 +3362,13 @@ __device__ __forceinline__ bool run_attention_steps(const KernelParams &P, const
     cur.off = first * kAfRows - cur.pg * page;
   };
   if (shared) {
-    if (item < items) take_item();
+    if (item < tab.items()) take_item();
   } else if (left > 0) {
     // entry whose steps contain u0: the last one that begins at or before it
-    for (int k = 0; k < n; k += 32) cur.e += __popc(__ballot_sync(0xffffffffu, k + lane < n && tab.step0[k + lane] <= u0));
+    for (int k = 0, n = tab.n(); k < n; k += 32) cur.e += __popc(__ballot_sync(0xffffffffu, k + lane < n && tab.pos(k + lane).x <= u0));
     --cur.e;
     af_load(cur, tab, G);
-    int u = u0 - tab.step0[cur.e];
+    int u = u0 - tab.pos(cur.e).x;
     cur.s = u % cur.S;
     u /= cur.S;
     cur.i = u % cur.I;
@@ -3407,7 +3415,7 @@ __device__ __forceinline__ bool run_attention_steps(const KernelParams &P, const
       if (req.off >= page) { req.off = 0; ++req.pg; }
       if (++req.s == req.S && !shared) {
         const int e = req.e;
-        af_next_tile(req, tab, G, groups, n);
+        af_next_tile(req, tab, G, groups);
         if (req.e != e) have = false;
       }
     }
@@ -3423,7 +3431,7 @@ __device__ __forceinline__ bool run_attention_steps(const KernelParams &P, const
   const int TP = 16 / G;                                        // tokens of a query tile
   int out_slot = 0, unit = u0;
   // (a warp whose wait was abandoned still takes part in the barriers of shared tiles)
-  while (run && (shared ? item < items : ok && left > 0)) {
+  while (run && (shared ? item < tab.items() : ok && left > 0)) {
     // ---- query tile of this segment: rows (token, head), normed and rotated ----
     const int t0 = cur.i * TP, rows = min(16, (cur.nq - t0) * G), new_start = cur.len - cur.nq;
     if (!shared) head = cur.h * hh + hw;
@@ -3501,9 +3509,12 @@ __device__ __forceinline__ bool run_attention_steps(const KernelParams &P, const
             const uint2 kw = make_uint2(pack_bf16(x[0], x[1]), pack_bf16(x[2], x[3]));
             const uint32_t to = af_piece(pos - pos0, lane >> 1) + (lane & 1) * 8;
             asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(kt + to), "r"(kw.x), "r"(kw.y) : "memory");
-            // (0 x infinity is NaN, for every query row of the tile: such values are zero here, and added to the rows that see them below)
-            const uint2 vs = make_uint2(finite_or_zero_bf16x2(vr[k].x), finite_or_zero_bf16x2(vr[k].y));
-            if (__any_sync(0xffffffffu, vs.x != vr[k].x || vs.y != vr[k].y)) parity |= kAfWild;
+            // (0 x infinity is NaN, for every query row of the tile: such values are zero here and are put back later)
+            uint2 vs = vr[k];
+            if (__builtin_expect(__any_sync(0xffffffffu, !finite_bf16x2(vs.x) || !finite_bf16x2(vs.y)), 0)) {
+              parity |= kAfWild;
+              vs = make_uint2(finite_or_zero_bf16x2(vs.x), finite_or_zero_bf16x2(vs.y));
+            }
             asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(vt + to), "r"(vs.x), "r"(vs.y) : "memory");
             if (cur.i == 0) {   // the first tile's warp writes the cache
               size_t row;
@@ -3566,30 +3577,15 @@ __device__ __forceinline__ bool run_attention_steps(const KernelParams &P, const
     l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
     l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
 
-    if (parity & kAfWild) {
-      // infinities and NaNs of the value rows that this segment appended
-      parity &= ~kAfWild;
-      const int end = min((first_s + seg) * kAfRows, cur.len);
-      for (int pos = max(first_s * kAfRows, new_start); pos < end; ++pos) {
-        const __nv_bfloat16 *vp = ptr(0, true) + (size_t)(cur.q0 + pos - new_start) * ldq + (size_t)(head * (G + 2) + G + 1) * 128 + 2 * q;
-#pragma unroll
-        for (int nt = 0; nt < 16; ++nt) {
-          const uint32_t v = __ldcg(reinterpret_cast<const uint32_t *>(vp + 8 * nt)), w = finite_or_zero_bf16x2(v) ^ v;
-          if (w & 0xffffu) {
-            if (pos <= lim0) o[nt][0] += bf16_lo(v);
-            if (pos <= lim1) o[nt][2] += bf16_lo(v);
-          }
-          if (w >> 16) {
-            if (pos <= lim0) o[nt][1] += bf16_hi(v);
-            if (pos <= lim1) o[nt][3] += bf16_hi(v);
-          }
-        }
-      }
-    }
-
     // ---- results of the segment ----
     __nv_bfloat16 *out = reinterpret_cast<__nv_bfloat16 *>(d.p[7]);
     const size_t row_out = (size_t)(cur.q0 + t0) * ldo + (size_t)head * G * 128;
+    const auto put_back = [&](float *acc, int pitch) {
+      parity &= ~kAfWild;
+      const int pos = max(first_s * kAfRows, new_start);
+      af_put_back(ptr(0, true) + (size_t)(cur.q0 + pos - new_start) * ldq + (size_t)(head * (G + 2) + G + 1) * 128, ldq, pos,
+                  min((first_s + seg) * kAfRows, cur.len), new_start + t0, G, rows, acc, pitch);
+    };
     if (shared) {
       // the eight warps' parts meet in shared memory: sums and maxima where the query tiles were, outputs in the rings (idle now)
       consumer_sync();                                          // (the query tile has been read by all)
@@ -3603,8 +3599,10 @@ __device__ __forceinline__ bool run_attention_steps(const KernelParams &P, const
           for (int nt = 0; nt < 16; ++nt) *reinterpret_cast<float2 *>(mine + row * 128 + nt * 8 + 2 * q) = make_float2(o[nt][2 * half], o[nt][2 * half + 1]);
         }
       }
+      if (__builtin_expect((parity & kAfWild) != 0u, 0)) put_back(mine, 128);
       consumer_sync();
-      const int pitch = (nstg + 1) * kAfStage / 4;               // floats between two warps' areas
+      const int4 at = tab.pos(cur.e);
+      const int NC = at.w, pitch = (nstg + 1) * kAfStage / 4;               // floats between two warps' areas
       const float *ml0 = reinterpret_cast<const float *>(xtile + (tile - smem_u32(xtile)));
       for (int idx = threadIdx.x; idx < rows * 128; idx += kConsumerThreads) {
         const int row = idx >> 7, dim = idx & 127;
@@ -3621,7 +3619,7 @@ __device__ __forceinline__ bool run_attention_steps(const KernelParams &P, const
         if (NC == 1) {
           out[row_out + (size_t)(row / G) * ldo + (size_t)(row % G) * 128 + dim] = __float2bfloat16_rn(L > 0.f ? O / L : 0.f);
         } else {
-          float *rec = P.attn_scratch + (size_t)(tab.rec0[cur.e] + item - tab.step0[cur.e]) * kAfRecord + row * 132;
+          float *rec = P.attn_scratch + (size_t)(at.z + item - at.x) * kAfRecord + row * 132;
           if (dim == 0) __stcg(reinterpret_cast<float2 *>(rec), make_float2(M, L));
           __stcg(rec + 4 + dim, O);
         }
@@ -3630,7 +3628,7 @@ __device__ __forceinline__ bool run_attention_steps(const KernelParams &P, const
         consumer_sync();
         const int k = head * cur.I + cur.i;
         if (threadIdx.x == 0) {
-          unsigned int old, *ticket = &P.attn_tickets[d.a[A_TICKET] + tab.tile0[cur.e] + k];
+          unsigned int old, *ticket = &P.attn_tickets[d.a[A_TICKET] + at.y + k];
           asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(old) : "l"(ticket) : "memory");
           const bool last = old + 1u == (unsigned)NC;
           if (last) *ticket = 0u;                                // for the next launch
@@ -3639,7 +3637,7 @@ __device__ __forceinline__ bool run_attention_steps(const KernelParams &P, const
         consumer_sync();
         for (int idx = threadIdx.x; sflags[4] && idx < rows * 128; idx += kConsumerThreads) {
           const int row = idx >> 7, dim = idx & 127;
-          const float *rec = P.attn_scratch + (size_t)(tab.rec0[cur.e] + k * NC) * kAfRecord + row * 132;
+          const float *rec = P.attn_scratch + (size_t)(at.z + k * NC) * kAfRecord + row * 132;
           float M = -INFINITY, L = 0.f, O = 0.f;
           for (int c0 = 0; c0 < NC; c0 += 8) {
             float2 pm[8];
@@ -3669,7 +3667,7 @@ __device__ __forceinline__ bool run_attention_steps(const KernelParams &P, const
       }
       item += P.num_workers;
       left = 0;
-      if (item < items) {
+      if (item < tab.items()) {
         fence_proxy_async_smem();                               // the rings were written and read through the generic proxy
         consumer_sync();
         take_item();
@@ -3680,9 +3678,9 @@ __device__ __forceinline__ bool run_attention_steps(const KernelParams &P, const
       }
       continue;
     }
-    if (seg == cur.S) {
+    if (seg == cur.S && __builtin_expect((parity & kAfWild) == 0u, 1)) {
       // (a row whose sum is not positive, or NaN, is zero in every form)
-      if (!(l0 > 0.f && l1 > 0.f)) {
+      if (__builtin_expect(!(l0 > 0.f && l1 > 0.f), 0)) {
 #pragma unroll
         for (int nt = 0; nt < 16; ++nt) {
           if (!(l0 > 0.f)) o[nt][0] = o[nt][1] = 0.f;
@@ -3701,7 +3699,8 @@ __device__ __forceinline__ bool run_attention_steps(const KernelParams &P, const
         }
       }
     } else {
-      // a range has at most two records: of the tile it begins in (0) and of the one it ends in (1)
+      // a range has at most two records: of the tile it begins in (0) and of the one it ends in (1; whole tiles with values to put back
+      // pass through it)
       float *rec = P.attn_scratch + (size_t)((2 * range + (unit == u0 ? 0 : 1)) * hh + hw) * kAfRecord;
 #pragma unroll
       for (int half = 0; half < 2; ++half) {
@@ -3713,11 +3712,12 @@ __device__ __forceinline__ bool run_attention_steps(const KernelParams &P, const
           for (int nt = 0; nt < 16; ++nt) __stcg(reinterpret_cast<float2 *>(dst + 4 + nt * 8 + 2 * q), make_float2(o[nt][2 * half], o[nt][2 * half + 1]));
         }
       }
+      if (__builtin_expect((parity & kAfWild) != 0u, 0)) put_back(rec + 4, 132);
       __threadfence();
       __syncwarp();
       const int begin = unit - first_s, end = begin + cur.S;     // the tile's steps
       const int r0 = begin / per, parts = (end - 1) / per - r0 + 1;
-      unsigned int *ticket = &P.attn_tickets[d.a[A_TICKET] + tab.tile0[cur.e] + head * cur.I + cur.i];
+      unsigned int *ticket = &P.attn_tickets[d.a[A_TICKET] + tab.pos(cur.e).y + head * cur.I + cur.i];
       unsigned int old = 0;
       if (lane == 0) asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(old) : "l"(ticket) : "memory");
       old = __shfl_sync(0xffffffffu, old, 0);
@@ -3754,7 +3754,7 @@ __device__ __forceinline__ bool run_attention_steps(const KernelParams &P, const
             }
             M = N;
           }
-          if (!(L > 0.f)) acc = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (__builtin_expect(!(L > 0.f), 0)) acc = make_float4(0.f, 0.f, 0.f, 0.f);
           const float inv = L > 0.f ? 1.f / L : 0.f;
           *reinterpret_cast<uint2 *>(out + row_out + (size_t)(row / G) * ldo + (size_t)(row % G) * 128 + lane * 4) =
               make_uint2(pack_bf16(acc.x * inv, acc.y * inv), pack_bf16(acc.z * inv, acc.w * inv));
@@ -3764,7 +3764,7 @@ __device__ __forceinline__ bool run_attention_steps(const KernelParams &P, const
     left -= seg;
     unit += seg;
     cur.s += seg;
-    if (cur.s == cur.S) af_next_tile(cur, tab, G, groups, n);
+    if (cur.s == cur.S) af_next_tile(cur, tab, G, groups);
   }
   if (!ok) {
     // abandoned: what is in flight always arrives; wait for it, a bounded number of polls each
@@ -3786,17 +3786,15 @@ static __device__ __forceinline__ bool run_attention_flat(const KernelParams &P,
                                                           uint64_t deadline, int task) {
   const int warp = threadIdx.x >> 5;
   const int hkv = d.a[A_HKV], G = d.a[A_HQ] / hkv, flags = d.a[A_FLAGS];
-  AfHead *th = reinterpret_cast<AfHead *>(reinterpret_cast<uint8_t *>(sflags) - kFlagsOffset + kMiscBytes);
-  const AfTable tab = af_table(reinterpret_cast<uint8_t *>(th + 1), d.a[A_CAP]);
+  const AfTable tab{reinterpret_cast<int4 *>(reinterpret_cast<uint8_t *>(sflags) - kFlagsOffset + kMiscBytes)};
   fence_proxy_async_smem();                                     // earlier generic accesses to the area come before its copies
   if (warp == 0) {
-    const int4 k = th->key;
-    if (k.x != d.a[A_SLOT] || k.y != hkv || k.z != G || k.w != ((flags & 4) ? -d.a[A_PAGE] : d.a[A_PAGE])) af_build_table(P, d, tab, th);
+    const int4 k = tab.at[0];
+    if (k.x != d.a[A_SLOT] || k.y != hkv || k.z != G || k.w != ((flags & 4) ? -d.a[A_PAGE] : d.a[A_PAGE])) af_build_table(P, d, tab);
   }
   consumer_sync();
-  const int n = th->n, total = th->total, items = th->items;
-  if (total == 0 || items > 0) return run_attention_steps<true>(P, d, xtile, sflags, tab, n, total, items, iteration, deadline, task);
-  return run_attention_steps<false>(P, d, xtile, sflags, tab, n, total, items, iteration, deadline, task);
+  if (tab.total() == 0 || tab.items() > 0) return run_attention_steps<true>(P, d, xtile, sflags, tab, iteration, deadline, task);
+  return run_attention_steps<false>(P, d, xtile, sflags, tab, iteration, deadline, task);
 }
 
 static __device__ void run_embed(const Ctx &c, const TaskDesc &d) {

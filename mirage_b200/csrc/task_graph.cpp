@@ -549,7 +549,7 @@ struct Builder {
         // the general instantiation: a query tile and a ring of copy stages per warp, and the table of the requests
         if (general_graph()) {
           attn = 1024 + 8 * (attention_stages() + 1) * 4096;   // (1024: alignment)
-          g->attn_table_bytes = std::max(g->attn_table_bytes, (32 + 28 * attention_requests(l) + 12 + 15) / 16 * 16);
+          g->attn_table_bytes = std::max(g->attn_table_bytes, 32 + 32 * attention_requests(l));
         }
         need = std::max(need, attn - kPartialBytes);
       }
