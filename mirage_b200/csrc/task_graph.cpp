@@ -503,7 +503,7 @@ struct Builder {
   // ---- shared-memory plan ---------------------------------------------------------
   int plan_smem() {
     const int ntok = std::min(std::max(cfg.max_num_batched_tokens, 1), (int)kMaxLinearTokens);
-    int64_t need = 24 * 1024;
+    int64_t need = 24 * 1024, rings = 0;   // rings: the attention tasks' (general instantiation), aligned to 1 KB
     for (const auto &l : L) {
       if (l.folded) continue;
       if (hybrid_op(l.op)) {
@@ -548,7 +548,7 @@ struct Builder {
         int64_t attn = (int64_t)G * (128 + 16 + 8 * 128) * 4 + (int64_t)cfg.max_num_batched_tokens * 512;
         // the general instantiation: a query tile and a ring of copy stages per warp, and the table of the requests
         if (general_graph()) {
-          attn = 1024 + 8 * (attention_stages() + 1) * 4096;   // (1024: alignment)
+          rings = attn = 8 * (attention_stages() + 1) * 4096;
           g->attn_table_bytes = std::max(g->attn_table_bytes, 32 + 32 * attention_requests(l));
         }
         need = std::max(need, attn - kPartialBytes);
@@ -556,27 +556,29 @@ struct Builder {
     }
     if (!no_batch_task()) need = std::max<int64_t>(need, (int64_t)(16 * cfg.max_num_batched_requests + 20 + (cfg.mode == MPK_MODE_ONLINE ? cfg.total_num_requests : 0)) * 4 - kPartialBytes);
     need = (need + 255) / 256 * 256;
-    // 64 KB stages (4 KB row segments) when at least three of them fit, else 32 KB stages
-    const int64_t room = kSmemBudget - kMiscBytes - g->attn_table_bytes - kPartialBytes - need;
-    g->x_tile_bytes = (int)need;
+    const int64_t room = kSmemBudget - kMiscBytes - g->attn_table_bytes - kPartialBytes;
+    // Weight stages of `bytes` beside the tile buffer, which starts behind them: what aligns the attention rings there is part of the
+    // buffer.  Four 32 KB stages need none, and with a whole KB set aside for it a graph of few tokens kept three of them (FP8, 6 layers of
+    // width 4096: 1 request 713 -> 700 us, 8 requests 856 -> 847; 12 layers of width 2048, 1 request 852 -> 859).
+    auto tile_behind = [&](int64_t stages, int bytes) {
+      return rings ? std::max(need, (rings - kPartialBytes + (1024 - stages * bytes % 1024) % 1024 + 255) / 256 * 256) : need;
+    };
+    auto fitting = [&](int bytes) {   // eight at most: the kernel uses the upper half of its 16-entry barrier arrays as scratch
+      int n = 0;
+      while (n < 8 && (n + 1) * (int64_t)bytes + tile_behind(n + 1, bytes) <= room) ++n;
+      return n;
+    };
     g->tc_tokens = tc_np();
-    if (g->use_tmem) {
-      // tcgen05 graphs: a ring of 16 KB slots (whole swizzle atoms), each filled by one tensor-map TMA; tasks that
-      // still stream padded rows (FP8, expert projections) take the widest chunk such a slot holds
-      const int stages = (int)(room / kTcSlotBytes);
-      if (stages < 2) return fail(MPK_ERR_UNSUPPORTED, "activation tile leaves fewer than 2 weight stages");
-      g->stage_bytes = kTcSlotBytes;
-      g->chunk_cols = 448;                 // 16 rows x (448 x 2 + 16) bytes <= 16 KB
-      g->num_stages = std::min(stages, 8);
-      return MPK_OK;
-    }
+    // tcgen05 graphs: a ring of 16 KB slots (whole swizzle atoms), each filled by one tensor-map TMA; tasks that
+    // still stream padded rows (FP8, expert projections) take the widest chunk such a slot holds.
+    // Others: 64 KB stages (4 KB row segments) when at least three of them fit, else 32 KB stages
     int cols = kChunkColsMax;
-    if (room / stage_bytes_for(cols) < (nb_max <= 8 ? 3 : 2)) cols = kChunkColsMax / 2;
-    const int stages = (int)(room / stage_bytes_for(cols));
-    if (stages < 2) return fail(MPK_ERR_UNSUPPORTED, "activation tile leaves fewer than 2 weight stages");
-    g->chunk_cols = cols;
-    g->stage_bytes = stage_bytes_for(cols);
-    g->num_stages = std::min(stages, 8);   // (the kernel uses the upper half of its 16-entry barrier arrays as scratch)
+    if (!g->use_tmem && fitting(stage_bytes_for(cols)) < (nb_max <= 8 ? 3 : 2)) cols = kChunkColsMax / 2;
+    g->chunk_cols = g->use_tmem ? 448 : cols;          // 16 rows x (448 x 2 + 16) bytes <= 16 KB
+    g->stage_bytes = g->use_tmem ? kTcSlotBytes : stage_bytes_for(cols);
+    g->num_stages = fitting(g->stage_bytes);
+    if (g->num_stages < 2) return fail(MPK_ERR_UNSUPPORTED, "activation tile leaves fewer than 2 weight stages");
+    g->x_tile_bytes = (int)tile_behind(g->num_stages, g->stage_bytes);
     return MPK_OK;
   }
 

@@ -3,6 +3,7 @@ transitive reduction, and that the host simulation of the event protocol runs ev
 import json
 
 import pytest
+import torch
 
 import mirage_b200 as mi
 from graph_shapes import KINDS, build
@@ -155,3 +156,37 @@ def test_expert_projection_refuses_misaligned_scale_tensors():
     build(0)
     with pytest.raises(N.MpkError, match="16-byte"):
         build(4)
+
+
+def _attention_and_fp8_linear(tokens, requests, heads, kv, K):
+    meta = lambda dtype, *s: torch.empty(*s, dtype=dtype, device="meta")
+    i32 = lambda n: meta(torch.int32, n)
+    params = mi.PersistentKernel.get_default_init_parameters()
+    params.update(test_mode=True, num_workers=148, max_num_batched_tokens=tokens, max_num_batched_requests=requests, dry_run=True, page_size=64,
+                  max_num_pages=requests, max_seq_length=64,
+                  meta_tensors={"qo_indptr_buffer": i32(requests + 1), "paged_kv_indptr_buffer": i32(requests + 1), "paged_kv_indices_buffer": i32(requests),
+                                "paged_kv_last_page_len_buffer": i32(requests)})
+    pk = mi.PersistentKernel(**params)
+    att = lambda name, dtype, *s: pk.attach_input(meta(dtype, *s), name)
+    bf = torch.bfloat16
+    grid = dict(grid_dim=(requests, kv, 1), block_dim=(128, 1, 1))
+    caches = [att(n, bf, requests, 64, kv, 128) for n in ("k", "v")]
+    out = att("attention", bf, tokens, heads * 128)
+    pk.paged_attention_layer(input=att("qkv", bf, tokens, (heads + 2 * kv) * 128), k_cache=caches[0], v_cache=caches[1], q_norm=att("qn", bf, 128), k_norm=att("kn", bf, 128),
+                             cos_pos_embed=att("cos", bf, 64, 128), sin_pos_embed=att("sin", bf, 64, 128), output=out, **grid)
+    if K:
+        xq, xs = att("xq", torch.float8_e4m3fn, tokens, K), pk.new_tensor((tokens, K // 512), dtype=mi.uint32, name="xs")
+        pk.quantize_fp8_layer(input=att("x", bf, tokens, K), output_fp8=xq, output_scale=xs, **grid)
+        pk.linear_fp8_layer(input_fp8=xq, input_scale=xs, weight_fp8=att("w", torch.float8_e4m3fn, 512, K), weight_scale=att("ws", torch.uint32, 512, K // 512),
+                            output=att("y", bf, tokens, 512), **grid)
+    pk.compile()
+    return json.loads(pk.dump_task_graph())
+
+
+@pytest.mark.parametrize("tokens,heads,kv", [(1, 32, 8), (8, 32, 8), (8, 8, 1), (4, 4, 4)])
+def test_few_token_graphs_with_attention_keep_four_weight_stages(tokens, heads, kv):
+    g = _attention_and_fp8_linear(tokens, tokens, heads, kv, 4096)
+    assert g["num_stages"] == 4 and g["stage_bytes"] == 33024
+    # two copy stages and a query tile for each of eight warps, from a 1 KB boundary behind the weight stages
+    pad = -g["num_stages"] * g["stage_bytes"] % 1024
+    assert g["x_tile_bytes"] + 8192 >= pad + 8 * 3 * 4096
