@@ -3165,10 +3165,11 @@ __device__ __forceinline__ void ldmatrix_x2(uint32_t (&r)[2], uint32_t smem_addr
 }
 
 // Table of the requests that have tokens, behind the other small areas of shared memory: two vectors in front, [0] what it was built for
-// (slots, kv heads, query heads of one, page | contiguous) and [1] the number of entries, the steps, the items of shared tiles (0: ranges); then two
+// (slots, kv heads, query heads of one, page | contiguous) and [1] the number of entries, the steps, the items of shared tiles (0: ranges), the first slot; then two
 // vectors an entry, {first token, tokens, kv0 (contiguous caches: slot), length} and {first step (shared tiles: item), first tile,
-// first record, parts of a tile}.  The order is that of the batch slots, the same in every worker.  Warp 0
-// builds it in the first attention task of a launch (three round trips to L2); it holds for every layer with the same geometry.
+// first record (ranges: of the pass), parts of a tile}.  The order is that of the batch slots, the same in every worker.  Warp 0
+// builds it in the first attention task of a launch (three round trips to L2); it holds for every layer with the same geometry.  More than kAttnTableCap
+// requests (graphs without linears) are gone through in passes of so many slots, each a task with a table of its own.
 // One pointer and counts that are read where they are used: held in registers they were spilled in the loop over the steps.
 struct AfTable {
   int4 *at;
@@ -3188,9 +3189,11 @@ __device__ __forceinline__ int af_heads(int hkv) { return min(hkv & -hkv, 8); }
 // 1000 positions, 53, 51 and 51 at 16000, 121, 98 and 88 at 100000 (64: 76); in a model of 4 kv heads, 16000 positions, 23, 31, 36 and 37 parts 19.2, 18.3, 17.3 and 15.0.
 __device__ __forceinline__ int af_parts(int S, int workers, int tile_steps) { return max(1, min(S * workers / tile_steps, min(16 + S / 96, 64))); }
 static __device__ __noinline__ void af_build_table(const KernelParams &P, const TaskDesc &d, const AfTable t) {
-  const int lane = threadIdx.x & 31, slots = d.a[A_SLOT], G = d.a[A_HQ] / d.a[A_HKV], hkv = d.a[A_HKV], page = d.a[A_PAGE], hh = af_heads(hkv);
-  int n = 0, steps = 0, tiles = 0;
-  for (int s0 = 0; s0 < slots; s0 += 32) {
+  const int lane = threadIdx.x & 31, slot0 = d.a[A_SLOT0], slots = min(d.a[A_SLOT], slot0 + d.a[A_PASS]), G = d.a[A_HQ] / d.a[A_HKV], hkv = d.a[A_HKV], page = d.a[A_PAGE], hh = af_heads(hkv);
+  // records and tickets of a pass are its own: the tiles of earlier slots are no more than one a slot and kv head and one for each 16 rows
+  const int record0 = slot0 / d.a[A_PASS] * P.num_workers * 16;
+  int n = 0, steps = 0, tiles = hkv * (slot0 + (slot0 && !(d.a[A_FLAGS] & 4) ? __ldcg(&P.meta.qo_indptr[slot0]) * G / 16 : 0));
+  for (int s0 = slot0; s0 < slots; s0 += 32) {
     const int slot = s0 + lane;
     int4 r = make_int4(0, 0, 0, 0);
     if (slot < slots) {
@@ -3216,7 +3219,7 @@ static __device__ __noinline__ void af_build_table(const KernelParams &P, const 
     }
     if (on && at < d.a[A_CAP]) {
       t.req(at) = r;
-      t.pos(at) = make_int4(steps + is - ns, tiles + it - nt, 0, 1);
+      t.pos(at) = make_int4(steps + is - ns, tiles + it - nt, record0, 1);
     }
     steps += __shfl_sync(0xffffffffu, is, 31);
     tiles += __shfl_sync(0xffffffffu, it, 31);
@@ -3243,7 +3246,7 @@ static __device__ __noinline__ void af_build_table(const KernelParams &P, const 
       }
       if (e < n) {
         t.pos(e).x = items + it - own;
-        t.pos(e).z = recs + ir - rec;
+        t.pos(e).z = record0 + recs + ir - rec;
         t.pos(e).w = parts;
       }
       items += __shfl_sync(0xffffffffu, it, 31);
@@ -3251,8 +3254,8 @@ static __device__ __noinline__ void af_build_table(const KernelParams &P, const 
     }
   }
   if (lane == 0) {
-    t.at[0] = make_int4(slots, hkv, G, (d.a[A_FLAGS] & 4) ? -page : page);
-    t.at[1] = make_int4(n, steps, items, 0);
+    t.at[0] = make_int4(d.a[A_SLOT], hkv, G, (d.a[A_FLAGS] & 4) ? -page : page);
+    t.at[1] = make_int4(n, steps, items, slot0);
   }
 }
 
@@ -3701,7 +3704,7 @@ __device__ __forceinline__ bool run_attention_steps(const KernelParams &P, const
     } else {
       // a range has at most two records: of the tile it begins in (0) and of the one it ends in (1; whole tiles with values to put back
       // pass through it)
-      float *rec = P.attn_scratch + (size_t)((2 * range + (unit == u0 ? 0 : 1)) * hh + hw) * kAfRecord;
+      float *rec = P.attn_scratch + (size_t)(tab.pos(cur.e).z + (2 * range + (unit == u0 ? 0 : 1)) * hh + hw) * kAfRecord;
 #pragma unroll
       for (int half = 0; half < 2; ++half) {
         const int row = g + 8 * half;
@@ -3724,6 +3727,7 @@ __device__ __forceinline__ bool run_attention_steps(const KernelParams &P, const
       if (old + 1u == (unsigned)parts) {
         __syncwarp();                                           // lane 0's acquire holds for all of them: a shuffle orders no memory
         if (lane == 0) *ticket = 0u;                            // for the next launch
+        const int record0 = tab.pos(cur.e).z;
         for (int row = 0; row < rows; ++row) {
           float M = -INFINITY, L = 0.f;
           float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -3736,7 +3740,7 @@ __device__ __forceinline__ bool run_attention_steps(const KernelParams &P, const
               ov[k] = make_float4(0.f, 0.f, 0.f, 0.f);
               if (k0 + k < parts) {
                 const int r = r0 + k0 + k;
-                const float *src = P.attn_scratch + (size_t)((2 * r + (begin <= r * per ? 0 : 1)) * hh + hw) * kAfRecord + row * 132;
+                const float *src = P.attn_scratch + (size_t)(record0 + (2 * r + (begin <= r * per ? 0 : 1)) * hh + hw) * kAfRecord + row * 132;
                 ml[k] = __ldcg(reinterpret_cast<const float2 *>(src));
                 ov[k] = __ldcg(reinterpret_cast<const float4 *>(src + 4) + lane);
               }
@@ -3790,7 +3794,8 @@ static __device__ __forceinline__ bool run_attention_flat(const KernelParams &P,
   fence_proxy_async_smem();                                     // earlier generic accesses to the area come before its copies
   if (warp == 0) {
     const int4 k = tab.at[0];
-    if (k.x != d.a[A_SLOT] || k.y != hkv || k.z != G || k.w != ((flags & 4) ? -d.a[A_PAGE] : d.a[A_PAGE])) af_build_table(P, d, tab);
+    if (k.x != d.a[A_SLOT] || k.y != hkv || k.z != G || k.w != ((flags & 4) ? -d.a[A_PAGE] : d.a[A_PAGE]) || tab.at[1].w != d.a[A_SLOT0])
+      af_build_table(P, d, tab);
   }
   consumer_sync();
   if (tab.total() == 0 || tab.items() > 0) return run_attention_steps<true>(P, d, xtile, sflags, tab, iteration, deadline, task);

@@ -549,7 +549,7 @@ struct Builder {
         // the general instantiation: a query tile and a ring of copy stages per warp, and the table of the requests
         if (general_graph()) {
           rings = attn = 8 * (attention_stages() + 1) * 4096;
-          g->attn_table_bytes = std::max(g->attn_table_bytes, 32 + 32 * attention_requests(l));
+          g->attn_table_bytes = std::max(g->attn_table_bytes, 32 + 32 * std::min(attention_requests(l), kAttnTableCap));
         }
         need = std::max(need, attn - kPartialBytes);
       }
@@ -1120,8 +1120,9 @@ struct Builder {
     NC = std::min(NC, std::max(1, max_seq / 32));
     NC = std::min(NC, 32);
     const int rope_rows = rope ? (int)T[l.t[5]].dim(0) : 1;
-    // (general instantiation: one task per worker, each of its warps takes a range of all requests' steps)
+    // (general instantiation: one task per worker and pass, each of its warps takes a range of all requests' steps)
     const bool flat = general_graph();
+    const int pass = attention_requests(l) > kAttnTableCap ? kAttnTableCap : slots;   // slots that go through the request table at once
     int map = 0;
     if (flat) {
       NC = W;
@@ -1138,17 +1139,17 @@ struct Builder {
         g->tmaps.push_back(m);
       }
     }
-    for (int s = 0; s < (flat ? 1 : slots); ++s)
+    for (int s = 0; s < (flat ? (slots + pass - 1) / pass : slots); ++s)
       for (int h = 0; h < (flat ? 1 : hkv); ++h)
         for (int c = 0; c < NC; ++c) {
           TaskDesc d = blank(TASK_ATTENTION, li);
           for (int i = 0; i < 8; ++i) d.p[i] = l.t[i] >= 0 ? (uint64_t)T[l.t[i]].ptr : 0;
           d.a[A_SLOT] = flat ? slots : s;
-          d.a[A_HEAD] = h;
+          d.a[flat ? A_SLOT0 : A_HEAD] = flat ? s * pass : h;
           d.a[A_CHUNK] = c;
-          d.a[A_NCHUNK] = NC;
+          d.a[flat ? A_PASS : A_NCHUNK] = flat ? pass : NC;
           d.a[A_NSTAGE] = attention_stages();
-          d.a[A_CAP] = attention_requests(l);
+          d.a[A_CAP] = std::min(attention_requests(l), kAttnTableCap);
           d.a[A_TMAP] = map;
           d.a[A_HQ] = hq;
           d.a[A_HKV] = hkv;
@@ -1163,12 +1164,12 @@ struct Builder {
           d.a[A_TICKET] = attn_ordinal;   // ticket bank
           d.a[A_EARLY_EV] = no_batch_task() ? -1 : 0;   // exec layer 0 is the batching task
           d.a[A_EARLY_NEED] = 1;
-          put(((s * hkv + h) * NC + c + rot) % W, d, ex);
+          put(((flat ? 0 : (s * hkv + h) * NC) + c + rot) % W, d, ex);
         }
     if (flat) {
-      // two records per warp; a ticket per (kv head, 16-row query tile) of every request
-      g->attn_scratch_floats = std::max<int64_t>(g->attn_scratch_floats, (int64_t)W * 8 * 2 * 16 * 132);
-      g->attn_tickets = std::max<int64_t>(g->attn_tickets, (int64_t)hkv * (attention_requests(l) + cfg.max_num_batched_tokens * G / 16 + 1));
+      // two records per warp and pass; a ticket per (kv head, 16-row query tile) of every request
+      g->attn_scratch_floats = std::max<int64_t>(g->attn_scratch_floats, (int64_t)W * 8 * 2 * 16 * 132 * ((slots + pass - 1) / pass));
+      g->attn_tickets = std::max<int64_t>(g->attn_tickets, (int64_t)hkv * ((pass < slots ? slots : attention_requests(l)) + (int64_t)cfg.max_num_batched_tokens * G / 16 + 1));
     } else {
       g->attn_scratch_floats = std::max<int64_t>(g->attn_scratch_floats, (int64_t)cfg.max_num_batched_tokens * hq * NC * 130);
       g->attn_tickets = std::max<int64_t>(g->attn_tickets, (int64_t)slots * hkv);

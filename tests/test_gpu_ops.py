@@ -328,10 +328,11 @@ class _Ranges:
     def check(self):
         ref, first = self.reference(), self.launch()
         assert rel_err(first.cpu(), ref) <= TOL
+        kc, vc = self.kc.cpu(), self.vc.cpu()
         for r, n in enumerate(self.lens):
             for pos in range(n):
                 at = self.row(r, pos)
-                assert rel_err(self.kc[at].cpu(), self.kc_ref[at]) <= 1e-2 and torch.equal(self.vc[at].cpu(), self.vc_ref[at])
+                assert rel_err(kc[at], self.kc_ref[at]) <= 1e-2 and torch.equal(vc[at], self.vc_ref[at])
         assert torch.equal(first, self.launch())
 
 
@@ -371,6 +372,15 @@ def test_paged_attention_unequal_requests(mi, workers, hkv, G, page, lens, new):
     a = _Ranges(mi, hkv, G, page, lens, new, num_workers=workers)
     per, parts, items = _form(hkv, G, lens, new, workers)
     assert per == 0 and max(parts) > 1 and min(parts) == 1 and items > (workers or 148)
+    a.check()
+
+
+# more requests than the request table holds at once: two workers take ranges, all of them share tiles
+@pytest.mark.parametrize("workers", [2, 0])
+def test_paged_attention_many_requests(mi, workers):
+    lens = [(i * 37) % 23 + 1 for i in range(1100)]
+    lens[700] = 400
+    a = _Ranges(mi, 2, 2, 8, lens, [0 if i % 11 == 5 else 1 for i in range(1100)], num_workers=workers)
     a.check()
 
 

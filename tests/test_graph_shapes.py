@@ -190,3 +190,8 @@ def test_few_token_graphs_with_attention_keep_four_weight_stages(tokens, heads, 
     # two copy stages and a query tile for each of eight warps, from a 1 KB boundary behind the weight stages
     pad = -g["num_stages"] * g["stage_bytes"] % 1024
     assert g["x_tile_bytes"] + 8192 >= pad + 8 * 3 * 4096
+
+
+@pytest.mark.parametrize("requests", [512, 513, 1400, 8000])
+def test_attention_of_any_number_of_requests_fits_shared_memory(requests):
+    assert _attention_and_fp8_linear(requests, requests, 8, 2, 0)["num_stages"] >= 2
