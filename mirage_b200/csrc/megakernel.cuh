@@ -3681,7 +3681,7 @@ __device__ __forceinline__ bool run_attention_steps(const KernelParams &P, const
       }
       continue;
     }
-    if (seg == cur.S && __builtin_expect((parity & kAfWild) == 0u, 1)) {
+    if (seg == cur.S && __builtin_expect((parity & kAfWild) == 0u && !(flags & 8), 1)) {
       // (a row whose sum is not positive, or NaN, is zero in every form)
       if (__builtin_expect(!(l0 > 0.f && l1 > 0.f), 0)) {
 #pragma unroll
@@ -3703,7 +3703,7 @@ __device__ __forceinline__ bool run_attention_steps(const KernelParams &P, const
       }
     } else {
       // a range has at most two records: of the tile it begins in (0) and of the one it ends in (1; whole tiles with values to put back
-      // pass through it)
+      // pass through it, and all tiles where the output allows no wide stores)
       float *rec = P.attn_scratch + (size_t)(tab.pos(cur.e).z + (2 * range + (unit == u0 ? 0 : 1)) * hh + hw) * kAfRecord;
 #pragma unroll
       for (int half = 0; half < 2; ++half) {
@@ -3760,8 +3760,15 @@ __device__ __forceinline__ bool run_attention_steps(const KernelParams &P, const
           }
           if (__builtin_expect(!(L > 0.f), 0)) acc = make_float4(0.f, 0.f, 0.f, 0.f);
           const float inv = L > 0.f ? 1.f / L : 0.f;
-          *reinterpret_cast<uint2 *>(out + row_out + (size_t)(row / G) * ldo + (size_t)(row % G) * 128 + lane * 4) =
-              make_uint2(pack_bf16(acc.x * inv, acc.y * inv), pack_bf16(acc.z * inv, acc.w * inv));
+          __nv_bfloat16 *dst = out + row_out + (size_t)(row / G) * ldo + (size_t)(row % G) * 128 + lane * 4;
+          const uint2 y = make_uint2(pack_bf16(acc.x * inv, acc.y * inv), pack_bf16(acc.z * inv, acc.w * inv));
+          if (__builtin_expect((flags & 8) != 0, 0)) {
+            const uint32_t h[2] = {y.x, y.y};
+#pragma unroll
+            for (int k = 0; k < 4; ++k) reinterpret_cast<uint16_t *>(dst)[k] = (uint16_t)(h[k >> 1] >> (16 * (k & 1)));
+          } else {
+            *reinterpret_cast<uint2 *>(dst) = y;
+          }
         }
       }
     }

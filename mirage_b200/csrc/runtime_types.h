@@ -204,7 +204,7 @@ enum { LR_POST = 13, LR_ADD = 14, LR_ROW = 16, L_CAP = 23, LR_BIAS = 24, LR_LDAD
 // ---- TASK_ATTENTION ----------------------------------------------------------
 //  p[0] qkv  p[1] k_cache  p[2] v_cache  p[3] q_norm  p[4] k_norm  p[5] cos  p[6] sin  p[7] out
 //  a[0] slot  a[1] kv head  a[2] chunk  a[3] num chunks  a[4] local q heads  a[5] local kv heads
-//  a[6] head_dim  a[7] page_size  a[8] flags(1 qk_norm, 2 rope, 4 contiguous cache)  a[9] ld_qkv
+//  a[6] head_dim  a[7] page_size  a[8] flags(1 qk_norm, 2 rope, 4 contiguous cache, 8 output rows on no 8-byte boundary (general instantiation))  a[9] ld_qkv
 //  a[10] ld_out  a[11] eps bits  a[12] rope table rows  a[13] cache seq (contiguous mode)
 //  a[14] ticket bank offset  a[15] event of the batching task (-1: none)  a[16] its arrivals per iteration
 //  general instantiation: one task per worker and pass (run_attention_flat): a[0] batch slots  a[1] first slot  a[2] the worker's number  a[3] slots of a pass  a[17] copy stages of a warp  a[18] requests the table holds

@@ -1123,6 +1123,7 @@ struct Builder {
     // (general instantiation: one task per worker and pass, each of its warps takes a range of all requests' steps)
     const bool flat = general_graph();
     const int pass = attention_requests(l) > kAttnTableCap ? kAttnTableCap : slots;   // slots that go through the request table at once
+    const bool narrow_out = flat && (((uint64_t)T[l.t[7]].ptr | (uint64_t)T[l.t[7]].ld() * 2) & 7) != 0;   // no 8-byte stores
     int map = 0;
     if (flat) {
       NC = W;
@@ -1155,7 +1156,7 @@ struct Builder {
           d.a[A_HKV] = hkv;
           d.a[A_HD] = 128;
           d.a[A_PAGE] = page;
-          d.a[A_FLAGS] = (qk_norm ? 1 : 0) | (rope ? 2 : 0) | (paged ? 0 : 4);
+          d.a[A_FLAGS] = (qk_norm ? 1 : 0) | (rope ? 2 : 0) | (paged ? 0 : 4) | (narrow_out ? 8 : 0);
           d.a[A_LDQKV] = (int)T[l.t[0]].ld();
           d.a[A_LDO] = (int)T[l.t[7]].ld();
           d.a[A_EPS] = float_bits(1e-6f);

@@ -280,7 +280,7 @@ def test_paged_attention_long_context(mi, lens, new, hkv, max_seq, token_budget)
 class _Ranges:
     """One paged attention layer over requests of `lens` positions, the last new[r] of them appended by the launch."""
 
-    def __init__(self, mi, hkv, G, page, lens, new, **kw):
+    def __init__(self, mi, hkv, G, page, lens, new, shift=0, **kw):
         self.hkv, self.G, self.page, self.lens, self.new = hkv, G, page, lens, new
         D, R, T = 128, len(lens), sum(new)
         g = torch.Generator().manual_seed(sum(lens))
@@ -305,7 +305,8 @@ class _Ranges:
         self.pk = pk = make_test_kernel(mi, max(T, 16), max_num_batched_requests=R, max_num_pages=total, page_size=page,
                                         max_seq_length=max(need) * page, meta_tensors=meta, **kw)
         self.qkv_d, self.kc, self.vc = self.qkv.cuda(), kc.cuda(), vc.cuda()
-        self.out = torch.zeros(T, hkv * G * D, dtype=torch.bfloat16, device="cuda")
+        self.buffer = torch.full((T * hkv * G * D + 8,), 7.0, dtype=torch.bfloat16, device="cuda")
+        self.out = self.buffer[shift:shift + T * hkv * G * D].view(T, -1)
         att = lambda t, name: pk.attach_input(t, name)
         pk.paged_attention_layer(
             input=att(self.qkv_d, "qkv"), k_cache=att(self.kc, "kc"), v_cache=att(self.vc, "vc"), q_norm=att(self.qn.cuda(), "qn"),
@@ -382,6 +383,18 @@ def test_paged_attention_many_requests(mi, workers):
     lens[700] = 400
     a = _Ranges(mi, 2, 2, 8, lens, [0 if i % 11 == 5 else 1 for i in range(1100)], num_workers=workers)
     a.check()
+
+
+# an output that starts on any element; one worker: whole tiles, two: merged ones as well, all of them: shared tiles
+@pytest.mark.parametrize("workers", [1, 2, 0])
+@pytest.mark.parametrize("shift", [1, 2])
+def test_paged_attention_output_without_alignment(mi, workers, shift):
+    lens, new = [300, 40, 90], [21, 1, 2]
+    aligned, a = (_Ranges(mi, 2, 2, 16, lens, new, shift=k, num_workers=workers) for k in (0, shift))
+    aligned.check()
+    assert torch.equal(a.launch(), aligned.launch())
+    edge = torch.cat([a.buffer[:shift], a.buffer[shift + a.out.numel():]])
+    assert edge.numel() == 8 and bool((edge == 7.0).all())
 
 
 # one worker: ranges of steps; all of them: the warps of a worker share a tile
