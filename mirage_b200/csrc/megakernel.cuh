@@ -3622,7 +3622,7 @@ __device__ __forceinline__ bool run_attention_steps(const KernelParams &P, const
         if (NC == 1) {
           out[row_out + (size_t)(row / G) * ldo + (size_t)(row % G) * 128 + dim] = __float2bfloat16_rn(L > 0.f ? O / L : 0.f);
         } else {
-          float *rec = P.attn_scratch + (size_t)(at.z + item - at.x) * kAfRecord + row * 132;
+          float *rec = P.attn_scratch + (size_t)(d.a[A_BANK] + at.z + item - at.x) * kAfRecord + row * 132;
           if (dim == 0) __stcg(reinterpret_cast<float2 *>(rec), make_float2(M, L));
           __stcg(rec + 4 + dim, O);
         }
@@ -3640,7 +3640,7 @@ __device__ __forceinline__ bool run_attention_steps(const KernelParams &P, const
         consumer_sync();
         for (int idx = threadIdx.x; sflags[4] && idx < rows * 128; idx += kConsumerThreads) {
           const int row = idx >> 7, dim = idx & 127;
-          const float *rec = P.attn_scratch + (size_t)(at.z + k * NC) * kAfRecord + row * 132;
+          const float *rec = P.attn_scratch + (size_t)(d.a[A_BANK] + at.z + k * NC) * kAfRecord + row * 132;
           float M = -INFINITY, L = 0.f, O = 0.f;
           for (int c0 = 0; c0 < NC; c0 += 8) {
             float2 pm[8];
@@ -3704,7 +3704,7 @@ __device__ __forceinline__ bool run_attention_steps(const KernelParams &P, const
     } else {
       // a range has at most two records: of the tile it begins in (0) and of the one it ends in (1; whole tiles with values to put back
       // pass through it, and all tiles where the output allows no wide stores)
-      float *rec = P.attn_scratch + (size_t)(tab.pos(cur.e).z + (2 * range + (unit == u0 ? 0 : 1)) * hh + hw) * kAfRecord;
+      float *rec = P.attn_scratch + (size_t)(d.a[A_BANK] + tab.pos(cur.e).z + (2 * range + (unit == u0 ? 0 : 1)) * hh + hw) * kAfRecord;
 #pragma unroll
       for (int half = 0; half < 2; ++half) {
         const int row = g + 8 * half;
@@ -3727,7 +3727,7 @@ __device__ __forceinline__ bool run_attention_steps(const KernelParams &P, const
       if (old + 1u == (unsigned)parts) {
         __syncwarp();                                           // lane 0's acquire holds for all of them: a shuffle orders no memory
         if (lane == 0) *ticket = 0u;                            // for the next launch
-        const int record0 = tab.pos(cur.e).z;
+        const int record0 = d.a[A_BANK] + tab.pos(cur.e).z;
         for (int row = 0; row < rows; ++row) {
           float M = -INFINITY, L = 0.f;
           float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);

@@ -208,9 +208,9 @@ enum { LR_POST = 13, LR_ADD = 14, LR_ROW = 16, L_CAP = 23, LR_BIAS = 24, LR_LDAD
 //  a[10] ld_out  a[11] eps bits  a[12] rope table rows  a[13] cache seq (contiguous mode)
 //  a[14] ticket bank offset  a[15] event of the batching task (-1: none)  a[16] its arrivals per iteration
 //  general instantiation: one task per worker and pass (run_attention_flat): a[0] batch slots  a[1] first slot  a[2] the worker's number  a[3] slots of a pass  a[17] copy stages of a warp  a[18] requests the table holds
-//  a[19] tensor map of the keys (the next one: the values)
+//  a[19] tensor map of the keys (the next one: the values)  a[20] first scratch record of its bank
 enum { A_SLOT = 0, A_HEAD, A_CHUNK, A_NCHUNK, A_HQ, A_HKV, A_HD, A_PAGE, A_FLAGS, A_LDQKV, A_LDO, A_EPS, A_ROPE_ROWS, A_CSEQ,
-       A_TICKET, A_EARLY_EV, A_EARLY_NEED, A_NSTAGE, A_CAP, A_TMAP, A_SLOT0 = A_HEAD, A_PASS = A_NCHUNK };
+       A_TICKET, A_EARLY_EV, A_EARLY_NEED, A_NSTAGE, A_CAP, A_TMAP, A_BANK, A_SLOT0 = A_HEAD, A_PASS = A_NCHUNK };
 // ---- TASK_EMBED / RMSNORM / SILU / ADD / INIT ---------------------------------
 //  rows [a[0],a[1]) of the token dimension, width a[2]; p[0] in  p[1] weight/second input  p[2] out
 //  a[3] ld_in  a[4] ld_out  a[5] eps bits | silu groups | vocab  a[6] ld_in2

@@ -1092,7 +1092,7 @@ struct Builder {
     return MPK_OK;
   }
 
-  int emit_attention(int li, int ex, int attn_ordinal) {
+  int emit_attention(int li, int ex, int attn_ordinal, int bank) {
     const LayerInfo &l = L[li];
     const bool paged = l.op == MPK_OP_PAGED_ATTENTION;
     if (l.params.size() < 4) return fail(MPK_ERR_INVALID, "attention needs [hq, hkv, qk_norm, rope] params");
@@ -1152,6 +1152,7 @@ struct Builder {
           d.a[A_NSTAGE] = attention_stages();
           d.a[A_CAP] = std::min(attention_requests(l), kAttnTableCap);
           d.a[A_TMAP] = map;
+          d.a[A_BANK] = bank;             // of the scratch records
           d.a[A_HQ] = hq;
           d.a[A_HKV] = hkv;
           d.a[A_HD] = 128;
@@ -1863,7 +1864,7 @@ struct Builder {
     }
   }
 
-  int emit(int li, int ex, int *attn_ordinal) {
+  int emit(int li, int ex, int *attn_ordinal, int attn_bank) {
     const LayerInfo &l = L[li];
     const int mbt = cfg.max_num_batched_tokens;
     switch (l.op) {
@@ -2028,7 +2029,7 @@ struct Builder {
         return MPK_OK;
       }
       case MPK_OP_ATTENTION: case MPK_OP_PAGED_ATTENTION:
-        return emit_attention(li, ex, (*attn_ordinal)++);
+        return emit_attention(li, ex, (*attn_ordinal)++, attn_bank);
       case MPK_OP_EMBED: {
         const TensorInfo &tab = T[l.t[1]], &y = T[l.t[2]];
         if (T[l.t[0]].dtype != MPK_I64) return fail(MPK_ERR_INVALID, "embed ids must be int64");
@@ -2316,6 +2317,18 @@ struct Builder {
         return fail(MPK_ERR_UNSUPPORTED, "a layer depends on more than 3 independent producers");
     }
 
+    // Attention layers of the general instantiation leave parts of split tiles in scratch records.  Layers that follow one another share
+    // them; a layer that does not depend on the last user of any bank gets one of its own.
+    std::vector<int> attn_bank(E, 0), bank_user;
+    for (int e = 0; e < E; ++e) {
+      if (g->exec[e].layer < 0) continue;
+      const int op = L[g->exec[e].layer].op;
+      if (op != MPK_OP_ATTENTION && op != MPK_OP_PAGED_ATTENTION) continue;
+      while (attn_bank[e] < (int)bank_user.size() && !anc[e][bank_user[attn_bank[e]]]) ++attn_bank[e];
+      if (attn_bank[e] == (int)bank_user.size()) bank_user.push_back(e);
+      bank_user[attn_bank[e]] = e;
+    }
+
     // ---- tasks ---------------------------------------------------------------------
     per_worker.assign(W, {});
     per_worker_exec.assign(W, {});
@@ -2329,7 +2342,7 @@ struct Builder {
         x.type = TASK_BATCH;
         continue;
       }
-      rc = emit(x.layer, e, &attn_ordinal);
+      rc = emit(x.layer, e, &attn_ordinal, attn_bank[e]);
       if (rc) return rc;
       if (x.num_tasks == 0) return fail(MPK_ERR_INVALID, "layer " + std::to_string(x.layer) + " produced no task");
     }
@@ -2380,6 +2393,12 @@ struct Builder {
     const int64_t bank = attn_ordinal > 0 ? g->attn_tickets / attn_ordinal : 0;
     for (auto &d : g->tasks)
       if (d.type == TASK_ATTENTION) d.a[A_TICKET] = (int)(d.a[A_TICKET] * bank);
+    if (general_graph() && bank_user.size() > 1) {   // likewise the scratch banks
+      const int64_t records = g->attn_scratch_floats / (16 * 132);
+      for (auto &d : g->tasks)
+        if (d.type == TASK_ATTENTION) d.a[A_BANK] = (int)(d.a[A_BANK] * records);
+      g->attn_scratch_floats *= (int64_t)bank_user.size();
+    }
     return simulate_task_graph(*g, err);
   }
 };
@@ -2498,7 +2517,7 @@ std::string dump_task_graph(const CompiledGraph &g, const std::vector<TensorInfo
   std::ostringstream os;
   os << "{\"num_workers\": " << g.num_workers << ", \"num_tasks\": " << g.tasks.size()
      << ", \"num_events\": " << g.num_events << ", \"num_layers\": " << layers.size()
-     << ", \"num_folded\": " << g.num_folded << ", \"num_stages\": " << g.num_stages << ", \"stage_bytes\": " << g.stage_bytes
+     << ", \"num_folded\": " << g.num_folded << ", \"attn_scratch_floats\": " << g.attn_scratch_floats << ", \"num_stages\": " << g.num_stages << ", \"stage_bytes\": " << g.stage_bytes
      << ", \"x_tile_bytes\": " << g.x_tile_bytes << ", \"weight_bytes\": " << g.weight_bytes
      << ",\n \"events\": [\n";
   for (size_t e = 0; e < g.exec.size(); ++e) {

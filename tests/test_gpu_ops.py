@@ -302,17 +302,21 @@ class _Ranges:
         i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
         meta = {"qo_indptr_buffer": i32(self.qo), "paged_kv_indptr_buffer": i32(self.indptr), "paged_kv_indices_buffer": i32(perm),
                 "paged_kv_last_page_len_buffer": i32([(n - 1) % page + 1 for n in lens])}
-        self.pk = pk = make_test_kernel(mi, max(T, 16), max_num_batched_requests=R, max_num_pages=total, page_size=page,
-                                        max_seq_length=max(need) * page, meta_tensors=meta, **kw)
+        self.params = dict(max_num_batched_requests=R, max_num_pages=total, page_size=page, max_seq_length=max(need) * page, meta_tensors=meta, **kw)
+        self.kernel = lambda **params: make_test_kernel(mi, max(T, 16), **params)
         self.qkv_d, self.kc, self.vc = self.qkv.cuda(), kc.cuda(), vc.cuda()
         self.buffer = torch.full((T * hkv * G * D + 8,), 7.0, dtype=torch.bfloat16, device="cuda")
         self.out = self.buffer[shift:shift + T * hkv * G * D].view(T, -1)
-        att = lambda t, name: pk.attach_input(t, name)
+        self.pk = self.kernel(**self.params)
+        self.layer(self.pk)
+        self.pk.compile()
+
+    def layer(self, pk, name=""):
+        att = lambda t, what: pk.attach_input(t, what + name)
         pk.paged_attention_layer(
             input=att(self.qkv_d, "qkv"), k_cache=att(self.kc, "kc"), v_cache=att(self.vc, "vc"), q_norm=att(self.qn.cuda(), "qn"),
             k_norm=att(self.kn.cuda(), "kn"), cos_pos_embed=att(self.tables[0].cuda(), "cos"), sin_pos_embed=att(self.tables[1].cuda(), "sin"),
-            output=att(self.out, "out"), grid_dim=(R, hkv, 1), block_dim=(128, 1, 1))
-        pk.compile()
+            output=att(self.out, "out"), grid_dim=(len(self.lens), self.hkv, 1), block_dim=(128, 1, 1))
 
     def row(self, r, pos):
         return self.perm[self.indptr[r] + pos // self.page], pos % self.page
@@ -395,6 +399,24 @@ def test_paged_attention_output_without_alignment(mi, workers, shift):
     assert torch.equal(a.launch(), aligned.launch())
     edge = torch.cat([a.buffer[:shift], a.buffer[shift + a.out.numel():]])
     assert edge.numel() == 8 and bool((edge == 7.0).all())
+
+
+# layers of different head counts that do not depend on one another: the request table is built again, and neither meets the other's records
+@pytest.mark.parametrize("workers", [2, 0])
+def test_paged_attention_layers_side_by_side(mi, workers):
+    lens, new = [700, 40, 90, 1100], [1, 1, 2, 9]
+    pair = [_Ranges(mi, hkv, G, 16, lens, new, num_workers=workers) for hkv, G in ((4, 2), (1, 8))]
+    want = [a.launch() for a in pair]
+    pk = pair[0].kernel(**pair[0].params)
+    for i, a in enumerate(pair):
+        a.out.zero_()
+        a.layer(pk, str(i))
+    pk.compile()
+    for _ in range(20):
+        pk.run_test_mode()
+        for a, w in zip(pair, want):
+            assert torch.equal(a.out, w)
+            a.out.zero_()
 
 
 # one worker: ranges of steps; all of them: the warps of a worker share a tile

@@ -195,3 +195,31 @@ def test_few_token_graphs_with_attention_keep_four_weight_stages(tokens, heads, 
 @pytest.mark.parametrize("requests", [512, 513, 1400, 8000])
 def test_attention_of_any_number_of_requests_fits_shared_memory(requests):
     assert _attention_and_fp8_linear(requests, requests, 8, 2, 0)["num_stages"] >= 2
+
+
+@pytest.mark.parametrize("depends", [False, True])
+def test_attention_layers_share_scratch_only_in_a_chain(depends):
+    """The second layer of a chain starts after the first one's merges; layers that are free to overlap have records of their own."""
+    meta = lambda dtype, *s: torch.empty(*s, dtype=dtype, device="meta")
+    bf, requests, heads, kv = torch.bfloat16, 16, 8, 2
+    one = _attention_and_fp8_linear(requests, requests, heads, kv, 0)
+    params = mi.PersistentKernel.get_default_init_parameters()
+    i32 = lambda n: meta(torch.int32, n)
+    params.update(test_mode=True, num_workers=148, max_num_batched_tokens=requests, max_num_batched_requests=requests, dry_run=True, page_size=64,
+                  max_num_pages=requests, max_seq_length=64,
+                  meta_tensors={"qo_indptr_buffer": i32(requests + 1), "paged_kv_indptr_buffer": i32(requests + 1), "paged_kv_indices_buffer": i32(requests),
+                                "paged_kv_last_page_len_buffer": i32(requests)})
+    pk = mi.PersistentKernel(**params)
+    att = lambda name, *s: pk.attach_input(meta(bf, *s), name)
+    norms = dict(q_norm=att("qn", 128), k_norm=att("kn", 128), cos_pos_embed=att("cos", 64, 128), sin_pos_embed=att("sin", 64, 128),
+                 grid_dim=(requests, kv, 1), block_dim=(128, 1, 1))
+    qkv = att("qkv", requests, (heads + 2 * kv) * 128)
+    for i in range(2):
+        out = att(f"out{i}", requests, heads * 128)
+        pk.paged_attention_layer(input=qkv, k_cache=att(f"k{i}", requests, 64, kv, 128), v_cache=att(f"v{i}", requests, 64, kv, 128), output=out, **norms)
+        if depends:
+            qkv = att("next", requests, (heads + 2 * kv) * 128)
+            pk.linear_layer(input=out, weight=att(f"w{i}", (heads + 2 * kv) * 128, heads * 128), output=qkv, grid_dim=(64, 1, 1), block_dim=(128, 1, 1))
+    pk.compile()
+    both = json.loads(pk.dump_task_graph())
+    assert one["attn_scratch_floats"] > 0 and both["attn_scratch_floats"] == (1 if depends else 2) * one["attn_scratch_floats"]
