@@ -1130,6 +1130,8 @@ struct Builder {
       // boxes of 8 positions x 128 columns over the rows of a cache, in the 128-byte-swizzled layout
       map = (int)g->tmaps.size();
       for (int t : {l.t[1], l.t[2]}) {
+        if (((uint64_t)T[t].ptr & 15u) != 0)
+          return fail(MPK_ERR_UNSUPPORTED, "with more than 8 batched tokens (or FP8 / expert layers) a kv cache starts on a 16-byte boundary: " + T[t].name);
         TmapSpec m;
         m.base = (uint64_t)T[t].ptr;
         m.rows = T[t].dim(0) * T[t].dim(1);

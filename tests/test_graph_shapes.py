@@ -223,3 +223,33 @@ def test_attention_layers_share_scratch_only_in_a_chain(depends):
     pk.compile()
     both = json.loads(pk.dump_task_graph())
     assert one["attn_scratch_floats"] > 0 and both["attn_scratch_floats"] == (1 if depends else 2) * one["attn_scratch_floats"]
+
+
+def test_attention_names_a_misaligned_cache():
+    """The general kernel copies cached rows by tensor maps: a cache that starts on no 16-byte boundary is refused by its name."""
+    import ctypes as C
+    from mirage_b200 import _native as N
+    tokens, hkv, G, seq = 16, 2, 2, 64
+
+    def build(offset):
+        cfg = N.MpkConfig()
+        cfg.test_mode, cfg.dry_run, cfg.world_size, cfg.num_workers = 1, 1, 1, 4
+        cfg.max_num_batched_tokens = cfg.max_num_batched_requests = tokens
+        h = C.c_void_p()
+        N.check(h, N.lib.mpk_create(C.byref(cfg), C.byref(h)))
+
+        def attach(name, ptr, *shape):
+            return N.check(h, N.lib.mpk_attach_tensor(h, name.encode(), C.c_void_p(ptr), N.BF16, len(shape), (C.c_int64 * len(shape))(*shape), None))
+
+        base = 0x20000000
+        t = [attach("qkv", base, tokens, hkv * (G + 2) * 128), attach("keys", base + 0x1000000, tokens, seq, hkv, 128),
+             attach("values", base + 0x2000000 + offset, tokens, seq, hkv, 128), -1, -1, -1, -1, attach("out", base + 0x3000000, tokens, hkv * G * 128)]
+        N.check(h, N.lib.mpk_add_layer(h, N.OP_ATTENTION, (C.c_int * 8)(*t), 8, (C.c_int * 3)(tokens, hkv, 1), (C.c_int64 * 4)(hkv * G, hkv, 0, 0), 4))
+        try:
+            N.check(h, N.lib.mpk_compile(h))
+        finally:
+            N.lib.mpk_destroy(h)
+
+    build(0)
+    with pytest.raises(N.MpkError, match="kv cache starts on a 16-byte boundary: values"):
+        build(8)
