@@ -2285,7 +2285,7 @@ static __device__ void run_moe_mul_sum_add(const Ctx &c, const TaskDesc &d) {
   const float *w = reinterpret_cast<const float *>(d.p[1]);
   const __nv_bfloat16 *res = reinterpret_cast<const __nv_bfloat16 *>(d.p[3]);
   __nv_bfloat16 *out = reinterpret_cast<__nv_bfloat16 *>(d.p[2]);
-  if (((c0 | c1 | H | ldo | ldres) & 7) == 0 && ((d.p[0] | d.p[2] | d.p[3]) & 15) == 0 && topk <= 16) {
+  if (((c0 | c1 | H | ldo | ldres) & 7) == 0 && ((d.p[0] | d.p[2] | d.p[3]) & 15) == 0) {
     // Eight columns of a token a thread, the slots' rows in flight together: a task holds 64 columns of every token, and walked
     // token by token, slot by slot it took 50 us for 32 tokens x 8 slots.  The sum runs in slot order as below.
     const int nv = (c1 - c0) >> 3;

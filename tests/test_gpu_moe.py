@@ -223,6 +223,33 @@ def test_moe_silu_mul_and_weighted_sum(mi):
     assert rel_err(y.cpu(), M.moe_mul_sum_add(down, wts, res)) <= 1e-2
 
 
+# slots taken four at a time: fewer, remainders, many; with and without a residual, a slot of weight 0 whose row is never read.  The last two
+# widths and the shifted output are summed column by column.  The output is the bf16 rounding of a float32 sum in slot order: one
+# step of bf16 apart (2^-7 of the value) where the products are contracted differently.
+@pytest.mark.parametrize("shift", [0, 1])
+@pytest.mark.parametrize("residual", [True, False])
+@pytest.mark.parametrize("b,topk,h", [(1, 1, 64), (3, 3, 2056), (33, 6, 1024), (2, 17, 512), (5, 40, 256), (4, 5, 1001), (7, 8, 516)])
+def test_moe_weighted_sum_shapes(mi, b, topk, h, residual, shift):
+    from mirage_b200 import _native as N
+    g = torch.Generator().manual_seed(b * topk + h)
+    x = torch.randn(b, topk, h, generator=g).to(torch.bfloat16)
+    wts = torch.rand(b, topk, generator=g)
+    wts[0, topk - 1] = 0
+    res = torch.randn(b, h, generator=g).to(torch.bfloat16) if residual else torch.zeros(b, h, dtype=torch.bfloat16)
+    ref = M.moe_mul_sum_add(x, wts, res)
+    x[0, topk - 1] = float("nan")
+    pk = make_test_kernel(mi, b)
+    buffer = torch.full((b * h + 8,), 7.0, dtype=torch.bfloat16, device="cuda")
+    y = buffer[shift:shift + b * h].view(b, h)
+    # (through the C ABI's layer, where the residual may be absent)
+    pk._layer(N.OP_MOE_MUL_SUM_ADD, [pk.attach_input(x.cuda(), "x"), pk.attach_input(wts.cuda(), "wts"),
+                                     pk.attach_input(res.cuda(), "res") if residual else None, pk.attach_input(y, "y")], (b, 1, 1))
+    pk.compile()
+    pk.run_test_mode()
+    assert rel_err(y.cpu(), ref) <= 2.0 ** -7
+    assert bool((buffer[:shift] == 7.0).all()) and bool((buffer[shift + b * h:] == 7.0).all())
+
+
 def test_moe_block_in_one_graph(mi):
     """router logits -> routing -> quantize -> W13 (fp8) -> silu-mul -> quantize -> W2 (fp8) -> weighted sum +
     residual: the routed-expert half of a DeepSeek-V3 layer (python/mirage/mpk/models/deepseek_v3/builder.py:
