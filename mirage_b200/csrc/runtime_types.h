@@ -354,7 +354,7 @@ struct KernelParams {
   DeviceStatus *status;
   BatchMeta meta;
   float *attn_scratch;                  // split-KV partials
-  unsigned int *attn_tickets;           // [max_requests * kv_heads] per attention layer slot
+  unsigned int *attn_tickets;           // per attention layer: [requests * kv heads], general instantiation [16-row query tiles of all kv heads]
   uint64_t *profiler;
   uint64_t profiler_entries;
   long long eos_token_id;
@@ -378,7 +378,7 @@ struct KernelParams {
   int32_t general_kernel;               // host side: launch the instantiation with FP8 and > 8-token linear tasks
   int32_t x_tile_bytes;                 // bytes reserved for the activation tile
   uint32_t spin_limit;                  // polls before a wait gives up
-  const void *tmaps;                    // array of 128-byte tensor maps (one per tcgen05 linear task), 64-byte aligned
+  const void *tmaps;                    // array of 128-byte tensor maps (one per tcgen05 linear task, two per attention layer of the general instantiation), 64-byte aligned
   int32_t use_tmem;                     // the graph has tcgen05 tasks: every worker CTA allocates tensor memory
   int32_t tc_tokens;                    // token rows of the activation operand tile (batched tokens rounded up to 16)
   int32_t attn_table_bytes;             // area of the attention tasks' request table, behind the small things (general instantiation)

@@ -81,7 +81,9 @@ struct Builder {
   // The e4m3 activation tile with its scale words may run on into the partial-sum area that follows the tile buffer
   // (these tasks keep no partial sums there), and the buffer may grow until five 16 KB ring slots remain (what the
   // 129 KB bf16 tile leaves as well): at 64 tokens that admits k tiles of 2048 instead of 1024, i.e. half as many
-  // stage / drain pauses per task.
+  // stage / drain pauses per task.  The attention tasks' request table (2 KB for 64 requests) is left out: tiles of whole 512 columns leave it
+  // 7 KB of the fifth slot at least.
+  static int64_t fp8_tc_tile_cap() { return (kSmemBudget - kMiscBytes - kPartialBytes - 5 * kTcSlotBytes) / 256 * 256; }
   // Copy stages of a warp's attention ring (general instantiation): 64 KB in flight per worker with three; graphs of few tokens keep the
   // room for their weight ring.
   int attention_stages() const { return nb_max > 8 ? kAttnStages : 2; }
@@ -89,7 +91,6 @@ struct Builder {
   int attention_requests(const LayerInfo &l) const {
     return std::min(l.op == MPK_OP_PAGED_ATTENTION ? cfg.max_num_batched_requests : std::max(l.grid[0], 1), std::max(cfg.max_num_batched_tokens, 1));
   }
-  static int64_t fp8_tc_tile_cap() { return (kSmemBudget - kMiscBytes - kPartialBytes - 5 * kTcSlotBytes) / 256 * 256; }
   int64_t linear_tile_bytes(int64_t K) const {
     return tc_linear(K) ? (int64_t)tc_np() * K * 2 : (int64_t)nb_max * (K * 2 + kRowPadBytes);
   }

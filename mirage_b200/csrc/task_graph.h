@@ -100,7 +100,7 @@ struct CompiledGraph {
   int hybrid = 0;                         // HYB_* family: recurrent / extended-attention layers present
   bool use_tmem = false;                  // some linear runs on tcgen05: workers allocate tensor memory
   int tc_tokens = 0;                      // token rows of the tcgen05 activation operand tile
-  std::vector<TmapSpec> tmaps;            // indexed by TaskDesc::a[L_TMAP]
+  std::vector<TmapSpec> tmaps;            // indexed by TaskDesc::a[L_TMAP], a[A_TMAP]
   int64_t weight_bytes = 0;
   int64_t inbox_floats_per_buffer = 0;    // world * mbt * Nmax
   int64_t attn_scratch_floats = 0;
