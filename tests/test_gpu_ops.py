@@ -341,8 +341,8 @@ class _Ranges:
         assert torch.equal(first, self.launch())
 
 
-# kv heads that go together are powers of two; pages smaller and larger than a step of 8 positions; query tiles of 16 rows with one, some
-# and all of them in use; requests shorter than a step, idle slots, and many more tiles than workers share
+# query tiles of 16 rows with one, some and all of them in use; requests shorter than a step, idle slots (on 148 workers all but the
+# fifth share tiles)
 @pytest.mark.parametrize("hkv,G,page,lens,new", [
     (1, 8, 8, [8, 1, 129, 17], [1, 1, 9, 3]),
     (3, 2, 24, [65, 200, 7], [16, 30, 7]),
@@ -364,6 +364,47 @@ def _form(hkv, G, lens, new, workers):
         return -(-steps // ranges), [], 0
     parts = [max(1, min(S * workers // (steps * hh), 16 + S // 96, 64)) for _, S in live]
     return 0, parts, sum(nt * p for (nt, _), p in zip(live, parts))
+
+
+# ranges of steps: one, two, four and eight kv heads side by side (with fewer than eight a worker has several ranges), one and several
+# groups of them; pages of one, three and eight steps; decoding batches, prompts, idle slots, requests shorter than a step
+@pytest.mark.parametrize("workers,hkv,G,page,lens,new", [
+    (2, 1, 8, 8, [600, 1, 700, 999, 64], [1, 1, 4, 0, 1]),
+    (1, 3, 4, 24, [200, 65, 7, 300], [16, 30, 7, 1]),
+    (3, 2, 1, 64, [(i * 97) % 211 + 1 for i in range(40)], [0 if i % 7 == 3 else 1 for i in range(40)]),
+    (2, 6, 2, 8, [400, 33, 90], [9, 1, 24]),
+    (4, 4, 4, 16, [1500, 3, 250, 31], [1, 1, 1, 1]),
+    (3, 16, 1, 64, [300, 40, 64, 9], [17, 1, 1, 0]),
+    (5, 24, 2, 24, [240, 100], [1, 40]),
+])
+def test_paged_attention_equal_ranges(mi, workers, hkv, G, page, lens, new):
+    assert _form(hkv, G, lens, new, workers)[0] >= 16
+    _Ranges(mi, hkv, G, page, lens, new, num_workers=workers).check()
+
+
+# contiguous caches, one token a slot: steps that end behind a slot read its neighbour's first rows, the last slot's end behind the cache
+@pytest.mark.parametrize("workers,seq", [(1, 100), (0, 100), (1, 96), (0, 13)])
+def test_contiguous_attention_of_many_slots(mi, workers, seq):
+    hkv, G, D, R = 2, 2, 128, 12
+    lens = [(i * 41) % seq + 1 for i in range(R - 2)] + [seq - 1, seq]
+    assert (_form(hkv, G, lens, [1] * R, workers)[0] > 0) == (workers == 1)
+    qkv, kc, vc = _bf16(R, hkv * (G + 2) * D, seed=3), _bf16(R, seq, hkv, D, seed=4), _bf16(R, seq, hkv, D, seed=5)
+    qn, kn, tables = _bf16(D, seed=14, scale=0.1, shift=1.0), _bf16(D, seed=15, scale=0.1, shift=1.0), ops.rope_tables(D, seq, 1e6)
+    kc_ref, vc_ref = kc.clone(), vc.clone()
+    ref = torch.cat([ops.paged_attention_request(qkv[r:r + 1], kc_ref, vc_ref, [r], n, hkv * G, hkv, qn, kn, *tables, 1e-6) for r, n in enumerate(lens)])
+    for r, n in enumerate(lens):
+        kc[r, n - 1:] = vc[r, n - 1:] = float("nan")
+    pk = make_test_kernel(mi, R, num_workers=workers, meta_tensors={"step": torch.tensor([n - 1 for n in lens], dtype=torch.int32, device="cuda")})
+    kc_d, vc_d, out = kc.cuda(), vc.cuda(), torch.zeros(R, hkv * G * D, dtype=torch.bfloat16, device="cuda")
+    att = lambda t, name: pk.attach_input(t, name)
+    pk.attention_layer(input=att(qkv.cuda(), "qkv"), k_cache=att(kc_d, "kc"), v_cache=att(vc_d, "vc"), q_norm=att(qn.cuda(), "qn"), k_norm=att(kn.cuda(), "kn"),
+                       cos_pos_embed=att(tables[0].cuda(), "cos"), sin_pos_embed=att(tables[1].cuda(), "sin"), output=att(out, "out"),
+                       grid_dim=(R, hkv, 1), block_dim=(128, 1, 1))
+    pk.compile()
+    pk.run_test_mode()
+    assert rel_err(out.cpu(), ref) <= TOL
+    for r, n in enumerate(lens):
+        assert rel_err(kc_d[r, :n].cpu(), kc_ref[r, :n]) <= 1e-2 and torch.equal(vc_d[r, :n].cpu(), vc_ref[r, :n])
 
 
 # one long request among short ones: tiles of several parts beside whole ones, and more of them than workers
