@@ -3188,6 +3188,22 @@ __device__ __forceinline__ int af_heads(int hkv) { return min(hkv & -hkv, 8); }
 // one request, 1 kv head, 1000 positions 80 -> 35 us, 16000 84 -> 50, 100000 94 -> 76.  Caps tried there: 16, 24 and 32 parts 35, 39 and 41 us at
 // 1000 positions, 53, 51 and 51 at 16000, 121, 98 and 88 at 100000 (64: 76); in a model of 4 kv heads, 16000 positions, 23, 31, 36 and 37 parts 19.2, 18.3, 17.3 and 15.0.
 __device__ __forceinline__ int af_parts(int S, int workers, int tile_steps) { return max(1, min(S * workers / tile_steps, min(16 + S / 96, 64))); }
+// Whole shares leave a tile of just under two of them in one part.  Where all tiles get a worker at once (tiles <= workers), the smallest
+// limit of steps that keeps the parts no more than the workers is taken if its longest part is shorter (returns the limit, 0: whole shares).
+// Limits are the average share times 1, 9/8, 10/8 .. 39/8, one per lane.  FP8, 12 layers of width 2048, 8 requests of 700 to 1400 positions
+// 1201 -> 1180 us (every tile in workers / tiles parts: 1166), 6 layers of width 4096 1067 -> 1061 us; one long request among short ones keeps whole shares.
+__device__ __forceinline__ int af_limit(const AfTable &t, int n, int hkv, int G, int workers, int tile_steps) {
+  const int lane = threadIdx.x & 31, limit = ((tile_steps + workers - 1) / workers * (8 + lane) + 7) / 8;
+  int parts = 0, longest = 0, shares = 0;
+  for (int e = 0; e < n; ++e) {
+    const int S = (t.req(e).w + kAfRows - 1) / kAfRows, k = min((S + limit - 1) / limit, min(16 + S / 96, 64)), f = af_parts(S, workers, tile_steps);
+    parts += hkv * ((t.req(e).y * G + 15) / 16) * k;
+    longest = max(longest, (S + k - 1) / k);
+    shares = max(shares, (S + f - 1) / f);
+  }
+  const unsigned fits = __ballot_sync(0xffffffffu, parts <= workers && longest < shares);
+  return fits ? __shfl_sync(0xffffffffu, limit, __ffs(fits) - 1) : 0;
+}
 static __device__ __noinline__ void af_build_table(const KernelParams &P, const TaskDesc &d, const AfTable t) {
   const int lane = threadIdx.x & 31, slot0 = d.a[A_SLOT0], slots = min(d.a[A_SLOT], slot0 + d.a[A_PASS]), G = d.a[A_HQ] / d.a[A_HKV], hkv = d.a[A_HKV], page = d.a[A_PAGE], hh = af_heads(hkv);
   // records and tickets of a pass are its own: the tiles of earlier slots are no more than one a slot and kv head and one for each 16 rows
@@ -3230,12 +3246,14 @@ static __device__ __noinline__ void af_build_table(const KernelParams &P, const 
   if (steps < P.num_workers * (8 / hh) * kAfMinSteps) {   // few steps to a range: the warps share tiles
     int recs = 0;
     __syncwarp();
+    const int limit = n > 0 && n * hkv <= P.num_workers ? af_limit(t, n, hkv, G, P.num_workers, steps * hh) : 0;
     for (int e0 = 0; e0 < n; e0 += 32) {
       const int e = e0 + lane;
       int parts = 0, nt = 0;
       if (e < n) {
         nt = hkv * ((t.req(e).y * G + 15) / 16);
-        parts = af_parts((t.req(e).w + kAfRows - 1) / kAfRows, P.num_workers, steps * hh);
+        const int S = (t.req(e).w + kAfRows - 1) / kAfRows;
+        parts = limit ? min((S + limit - 1) / limit, min(16 + S / 96, 64)) : af_parts(S, P.num_workers, steps * hh);
       }
       int it = nt * parts, ir = parts > 1 ? it : 0;
       const int own = it, rec = ir;

@@ -363,6 +363,14 @@ def _form(hkv, G, lens, new, workers):
     if steps >= ranges * 16:
         return -(-steps // ranges), [], 0
     parts = [max(1, min(S * workers // (steps * hh), 16 + S // 96, 64)) for _, S in live]
+    if hkv * len(live) <= workers:      # a limit of steps instead of whole shares
+        longest = max(-(-S // p) for (_, S), p in zip(live, parts))
+        for k in range(8, 40):
+            limit = -(-(-(-steps * hh // workers)) * k // 8)
+            cut = [min(-(-S // limit), 16 + S // 96, 64) for _, S in live]
+            if sum(nt * p for (nt, _), p in zip(live, cut)) <= workers and max(-(-S // p) for (_, S), p in zip(live, cut)) < longest:
+                parts = cut
+                break
     return 0, parts, sum(nt * p for (nt, _), p in zip(live, parts))
 
 
@@ -419,6 +427,17 @@ def test_paged_attention_unequal_requests(mi, workers, hkv, G, page, lens, new):
     per, parts, items = _form(hkv, G, lens, new, workers)
     assert per == 0 and max(parts) > 1 and min(parts) == 1 and items > (workers or 148)
     a.check()
+
+
+# few tiles of unlike lengths: cut by a limit of steps, every part at once
+@pytest.mark.parametrize("workers,hkv,G,page,lens,new,parts", [
+    (148, 8, 2, 64, [700, 1400, 870, 950, 1100, 1010, 1290, 780], [1] * 8, [2, 3, 2, 2, 2, 2, 3, 2]),   # (whole shares: 1 3 1 2 2 2 2 1)
+    (148, 2, 4, 8, [90, 170, 120, 9] * 6, [1, 2, 1, 1] * 6, [3, 5, 3, 1] * 6),                          # (2 5 3 1 ..)
+    (32, 4, 1, 16, [300, 170, 450], [1, 16, 3], [2, 2, 3]),                                             # (2 1 3)
+])
+def test_paged_attention_limited_parts(mi, workers, hkv, G, page, lens, new, parts):
+    assert _form(hkv, G, lens, new, workers)[1] == parts
+    _Ranges(mi, hkv, G, page, lens, new, num_workers=workers).check()
 
 
 # more requests than the request table holds at once: two workers take ranges, all of them share tiles
