@@ -33,6 +33,9 @@
 namespace mpk {
 
 constexpr int kFlagsOffset = 960;   // of the flags in the area of small things
+constexpr int kXIssuers = 5;        // warps that issue the MMAs of a tcgen05 linear, at most
+constexpr int kXBarsOffset = 1248;  // of the barriers of the tcgen05 linears' activations and borrowed slots
+static_assert(kFlagsOffset + 64 + 8 * kAttnStages * 8 + 32 <= kXBarsOffset && kXBarsOffset + 33 * 8 <= kMiscBytes, "small things overlap");
 
 struct Smem {
   uint8_t *stages;      // num_stages * stage_bytes
@@ -65,7 +68,7 @@ __device__ __forceinline__ Smem carve(uint8_t *base, const KernelParams &P) {
 
 struct LinearState {   // position of the compute warps in the weight stage ring
   int stage;
-  uint32_t phase;
+  uint32_t phase;       // parity of the next completion of its slots behind `stage`; with borrowed slots (XRing) a bit for each slot
   uint32_t acc_phase;   // parity of the next completion of the tcgen05 accumulator barrier
 };
 
@@ -77,6 +80,35 @@ struct Ctx {
   int worker;
   uint32_t tmem_base;     // tensor-memory address of column 0 (general instantiation, graphs with tcgen05 tasks)
 };
+
+// Barriers of the activations of tcgen05 linears, behind those of the attention rings: [0, 8) ring slot full, [8, 16) ring slot free (one arrival
+// per issuing warp, at most); of the borrowed weight slots: [16, 24) full, [24, 32) free, [32] the tile area is the task's.
+__device__ __forceinline__ uint64_t *x_bars(const Ctx &c) { return c.s.full + kXBarsOffset / 8; }
+
+// Weight slots of a tcgen05 linear in graphs without other streaming tasks (KernelParams::borrow).  The tile area, which attention and other bodies need
+// between linears, is mostly empty during one: the task borrows what its activations leave of it for further slots.  Boxes 0, 1, ... of a task go
+// to positions 0, 1, ... of a ring of `base` slots, which are filled ahead of the task, and `extra` borrowed ones, which are filled once the task
+// has begun.  What bounds the stream is the bytes in flight: a box takes some 2.3 us from its copy to the commit that frees its slot, so 148
+// workers need about 100 KB each to draw 6.5 TB/s (64 tokens, gate and up rows of width 4096: 70 KB 45 us, 90 KB 34 us).
+struct XRing {
+  int base, size;              // slots of the ring proper, with the borrowed ones
+  uint32_t stages, extra;      // shared-memory addresses
+  uint64_t *full, *empty, *xbars;
+  int bytes;                   // of a slot
+  __device__ __forceinline__ uint32_t slot(int i) const { return i < base ? stages + (uint32_t)(i * bytes) : extra + (uint32_t)((i - base) * bytes); }
+  __device__ __forceinline__ uint64_t *full_bar(int i) const { return i < base ? full + i : xbars + 16 + i - base; }
+  __device__ __forceinline__ uint64_t *empty_bar(int i) const { return i < base ? empty + i : xbars + 24 + i - base; }
+};
+__device__ __forceinline__ XRing x_ring(const Ctx &c, const TaskDesc &d) {
+  XRing r;
+  r.base = c.P.num_stages;
+  r.size = r.base + d.a[LX_EXTRA];
+  r.bytes = c.P.stage_bytes;
+  r.stages = smem_u32(c.s.stages);
+  r.extra = smem_u32(c.s.xtile) + (uint32_t)d.a[LX_XBYTES];
+  r.full = c.s.full; r.empty = c.s.empty; r.xbars = x_bars(c);
+  return r;
+}
 
 // ---------------------------------------------------------------------------
 // bounded waits
@@ -149,6 +181,58 @@ static __device__ void prefetch_attention_kv_l2(const Ctx &c, const TaskDesc *d,
 // A linear task streams its weight panel [n0, n1) x K as chunks of 16 rows x KC columns (KC <= 1024):
 // one cp.async.bulk per row segment, rows padded by 16 bytes in shared memory so that ldmatrix reads
 // are bank-conflict free.  Order: k tile (activation tile) -> 16-row group -> k chunk.
+// The same for graphs whose streaming tasks are all tcgen05 linears, with slots borrowed from the tile area (XRing).  A wait, the barrier's byte
+// count and a tensor-map copy take a thread 290 cycles whatever the box (16 KB boxes: 57 bytes a cycle), so all four warps of the streaming
+// warpgroup issue, one thread each; a slot belongs to one of them.
+// (Inlined: a function of its own could use more registers than the streaming warp keeps.)
+__device__ __forceinline__ void stream_borrowing(const Ctx &c, int t_begin, int t_end) {
+  const KernelParams &P = c.P;
+  const uint64_t policy = l2_policy_evict_first();
+  const int mine = (threadIdx.x >> 5) & 3;
+  uint32_t par = 0, used = 0, gate = 0;   // per slot of this warp: parity of its uses, used at all
+  bool ok = true;
+  for (int t = t_begin; t < t_end && ok; ++t) {
+    const TaskDesc *d = &P.tasks[t];
+    if (d->type != TASK_LINEAR) continue;
+    if (d->flags & TF_STREAM_AFTER_DEP) {
+      for (int i = 0; i < kMaxDeps && ok; ++i)
+        if (d->dep_event[i] >= 0) ok = wait_counter(c, &P.counters[d->dep_event[i]], (unsigned long long)d->dep_need[i] * c.iteration, false, 1, t);
+      fence_proxy_async_all();   // the weights were written through the generic proxy; the copies read through the async proxy
+    }
+    const XRing r = x_ring(c, *d);
+    const uint8_t *tmap = reinterpret_cast<const uint8_t *>(P.tmaps) + (size_t)d->a[L_TMAP] * 128;
+    const int RB = d->a[L_ROWS], nkb = d->a[L_KC] / kTcKBlock, kball = d->a[L_K] / kTcKBlock, tiles = (d->a[L_N1] - d->a[L_N0] + RB - 1) / RB;
+    const uint32_t tx = (uint32_t)(nkb * RB * 128);
+    int s = 0;
+    bool open = false;
+    for (int kb = 0; kb < kball && ok; kb += nkb)
+      for (int tile = 0; tile < tiles && ok; ++tile) {
+        if (s >= r.base && !open) {   // (every warp, so that none falls behind the gate's phases)
+          ok = wait_mbar(c, r.xbars + 32, gate, t);
+          gate ^= 1u;
+          open = true;
+        }
+        if ((s & 3) == mine) {
+          ok = ok && wait_mbar(c, r.empty_bar(s), ((par >> s) & 1u) ^ 1u, t);
+          if (!ok) break;
+          mbar_arrive_expect_tx(r.full_bar(s), tx);
+          tma_load_3d_hint(r.slot(s), tmap, 0, tile * RB, kb, smem_u32(r.full_bar(s)), policy);
+          mbar_arrive_n(r.empty_bar(s), 7);   // (of the eight arrivals its barrier counts; the last is the commit of the warp that reads the slot)
+          used |= 1u << s;
+          par ^= 1u << s;
+        }
+        if (++s == r.size) s = 0;
+      }
+  }
+  // Every copy must have landed before the CTA may exit.
+  for (int i = 0; i < 16; ++i) {
+    if (!((used >> i) & 1u)) continue;
+    uint64_t *bar = i < P.num_stages ? c.s.full + i : x_bars(c) + 16 + i - P.num_stages;
+    uint32_t polls = 0;
+    while (!mbar_try_wait(bar, ((par >> i) & 1u) ^ 1u) && ++polls < (1u << 24)) {}   // copies in flight always complete; the bound only guards the loop
+  }
+}
+
 template <bool GENERAL, int HYB>
 __device__ void streamer_loop(const Ctx &c, int t_begin, int t_end) {
   constexpr bool kMoe = HYB ? HYB == HYB_BF16 : GENERAL;   // expert projections stream one panel per active expert
@@ -338,7 +422,7 @@ __device__ __forceinline__ float gelu_tanh_f(float x) {
 // Stage the activation tile [B, KT] (bf16, rows padded by 16 bytes) for k range [k0, k0 + KT).
 // `gpre` holds this thread's first two gamma vectors, loaded before the dependency wait.
 // Address of 16-byte vector v (k elements 8v .. 8v + 7 of the tile) of token row b.  MODE 0 / 1: row-major rows
-// padded by 16 bytes (mma.sync fragments); MODE 2: the tcgen05 operand layout -- blocks of 64 columns, each block
+// padded by 16 bytes (mma.sync fragments); MODE 2 (FP8 linears): the tcgen05 operand layout -- blocks of 64 columns, each block
 // [token rows][128 bytes] with the 16-byte chunks of a row XOR-swizzled by (row & 7) (128-byte swizzle, K-major).
 template <int MODE>
 __device__ __forceinline__ uint8_t *x_vec(uint8_t *xs, int b, int v, int xstride, int np) {
@@ -567,17 +651,14 @@ static __device__ __noinline__ void stage_poly(const Ctx c, const TaskDesc &d, i
 
 // Copies B rows of `vecs` 16-byte vectors into the activation tile, one warp per row, every copy in flight.  A function of its own:
 // at the register cap of the linear bodies its loop would reload spilled variables for each copy.
-template <int MODE>
-__device__ __noinline__ void stage_rows(uint32_t xs, const uint4 *src, int ld, int B, int vecs, int xstride, int np) {
+static __device__ __noinline__ void stage_rows(uint32_t xs, const uint4 *src, int ld, int B, int vecs, int xstride) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (int b = warp; b < B; b += 8) {
     const uint4 *row = src + (size_t)b * ld;
-    const uint32_t dst = MODE == 2 ? xs + b * 128 + (((lane & 7) ^ (b & 7)) << 4) : xs + b * xstride + lane * 16;
+    const uint32_t dst = xs + b * xstride + lane * 16;
 #pragma unroll 4
     for (int v = lane; v < vecs; v += 32)
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + (MODE == 2 ? (uint32_t)((v >> 3) * np * 128) : (uint32_t)(v - lane) * 16u)),
-                   "l"(row + v)
-                   : "memory");
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + (uint32_t)(v - lane) * 16u), "l"(row + v) : "memory");
   }
   asm volatile("cp.async.commit_group;" ::: "memory");
   asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -726,7 +807,7 @@ __device__ void stage_x(const Ctx &c, const TaskDesc &d, int B, int k0, int KT, 
   }
   if (WIDE && (pro == PRO_PLAIN || pro == PRO_RMSNORM)) {
     // many tokens: asynchronous 16-byte copies straight into shared memory (all in flight, no registers held)
-    stage_rows<MODE>(smem_u32(xs), reinterpret_cast<const uint4 *>(src + k0), ldx >> 3, B, vec_per_row, xstride, np);
+    stage_rows(smem_u32(xs), reinterpret_cast<const uint4 *>(src + k0), ldx >> 3, B, vec_per_row, xstride);
     consumer_sync();
     if (pro == PRO_PLAIN) return;
     // RMSNorm in place.  Pass 1: one warp per token sums the squares and leaves 1 / rms in shared memory.  Pass 2:
@@ -1038,14 +1119,6 @@ __device__ __forceinline__ void run_linear(const Ctx &c, const TaskDesc &d, Line
 }
 
 // ---------------------------------------------------------------------------
-// TASK_LINEAR on the tensor path (general instantiation, graphs with more than 8 batched tokens): the weights are
-// the M operand (swap-AB, as in include/mirage/persistent_kernel/tasks/blackwell/linear_sm100_mpk.cuh:31-735),
-// 128 rows per tcgen05.mma, the batched tokens the N operand (16 .. 64), fp32 accumulators in tensor memory.
-// The task's rows are cut into tiles of RB <= 128 rows; tile t accumulates into columns [t * NP, t * NP + N) over
-// ALL k tiles of the activation, so the weights stream exactly once and the activation tile is staged once per k
-// tile.  Thread 0 issues the MMAs as ring slots fill and hands each slot back with tcgen05.commit; after the last
-// k block all eight warps read their lane quadrant of the accumulators (tcgen05.ld) and run the epilogue.
-// ---------------------------------------------------------------------------
 // Everything the epilogue of a tcgen05 linear task needs from its descriptor, read once into registers: the
 // descriptor lives in shared memory behind a generic reference, and a load from it may not move across the global
 // stores of the epilogue (they could alias), so reading it per element costs a chain of dependent loads every time.
@@ -1111,131 +1184,386 @@ __device__ __forceinline__ void linear_emit(const Ctx &c, const EmitArgs &e, int
   }
 }
 
+// Four rows of two tokens through the epilogue (fewer rows at the end of the panel: `cnt`); `wide`: output and operands lie on vector boundaries.
+struct XsOut {
+  EmitArgs e;
+  const uint8_t *operand;   // residual (bf16), gate (float32) or bias (bf16, a row of it: ldr = 0)
+  int ldr;
+  bool wide;
+};
 template <int HYB>
-__device__ void run_linear_tc(const Ctx &c, const TaskDesc &d, LinearState &ls, int task, const uint4 (&gpre)[2], bool ok) {
+__device__ __forceinline__ void xs_emit(const Ctx &c, const XsOut &x, int b0, int b1, int col, int cnt, const float (&v)[2][4]) {   // tokens b0 and b1 (-1: none)
+  const int epi = x.e.epi;
+  if (epi == EPI_SILU_PAIR || (HYB && (epi == EPI_GATED_SILU || epi == EPI_GATED_GELU))) {   // rows come as [gate, gate, up, up]
+    float o[2][2];
+#pragma unroll
+    for (int t = 0; t < 2; ++t)
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        if (!HYB || epi == EPI_SILU_PAIR) o[t][j] = round_bf16(silu_f(round_bf16(v[t][j]))) * round_bf16(v[t][j + 2]);
+        else o[t][j] = (epi == EPI_GATED_SILU ? silu_exact_f(v[t][j]) : gelu_tanh_f(v[t][j])) * v[t][j + 2];
+      }
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+      const int b = t == 0 ? b0 : b1;
+      if (b < 0) return;
+      __nv_bfloat16 *out = x.e.out + (size_t)b * x.e.ldo + (col >> 1);
+      if (x.wide) *reinterpret_cast<uint32_t *>(out) = pack_bf16(o[t][0], o[t][1]);
+      else { out[0] = __float2bfloat16_rn(o[t][0]); out[1] = __float2bfloat16_rn(o[t][1]); }
+    }
+    return;
+  }
+  if (epi == EPI_PUSH_LL || epi == EPI_PUSH_F32) {
+#pragma unroll
+    for (int t = 0; t < 2; ++t)
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (j < cnt && (t == 0 ? b0 : b1) >= 0) linear_emit<HYB>(c, x.e, t == 0 ? b0 : b1, col + j, v[t][j], 0.f, 0.f);
+    return;
+  }
+  float o[2][4];
+#pragma unroll
+  for (int t = 0; t < 2; ++t) {
+    const int b = t == 0 || b1 < 0 ? b0 : b1;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) o[t][j] = v[t][j];
+    if (epi == EPI_RESIDUAL || (HYB && epi == EPI_BIAS_F32)) {
+      const __nv_bfloat16 *r = reinterpret_cast<const __nv_bfloat16 *>(x.operand) + (size_t)b * x.ldr + col;
+      if (x.wide && cnt == 4) {
+        const uint2 w = __ldcg(reinterpret_cast<const uint2 *>(r));
+        o[t][0] += bf16_lo(w.x); o[t][1] += bf16_hi(w.x); o[t][2] += bf16_lo(w.y); o[t][3] += bf16_hi(w.y);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) if (j < cnt) o[t][j] += bf16_to_f(__ldcg(r + j));
+      }
+    }
+    if (HYB && epi == EPI_GATE_SIGMOID) {
+      const float *g = reinterpret_cast<const float *>(x.operand) + (size_t)b * x.ldr + col;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) if (j < cnt) o[t][j] /= 1.0f + expf(-__ldcg(g + j));
+    }
+    if (HYB && epi == EPI_RELU2) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) o[t][j] = fmaxf(o[t][j], 0.f) * fmaxf(o[t][j], 0.f);
+    }
+    if (HYB && (epi == EPI_SOFTCAP || epi == EPI_SCALE_F32)) {
+      const float f = __uint_as_float(x.e.seq_hi);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) o[t][j] = epi == EPI_SCALE_F32 ? f * o[t][j] : f * tanhf(o[t][j] / f);
+    }
+  }
+#pragma unroll
+  for (int t = 0; t < 2; ++t) {
+    const int b = t == 0 ? b0 : b1;
+    if (b < 0) return;
+    const size_t at = (size_t)b * x.e.ldo + col;
+    if (HYB && (epi == EPI_STORE_F32 || epi == EPI_BIAS_F32 || epi == EPI_SOFTCAP || epi == EPI_SCALE_F32)) {
+      float *out = reinterpret_cast<float *>(x.e.out) + at;
+      if (x.wide && cnt == 4) {
+        *reinterpret_cast<float4 *>(out) = make_float4(o[t][0], o[t][1], o[t][2], o[t][3]);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) if (j < cnt) out[j] = o[t][j];
+      }
+    } else {
+      __nv_bfloat16 *out = x.e.out + at;
+      if (x.wide && cnt == 4) {
+        *reinterpret_cast<uint2 *>(out) = make_uint2(pack_bf16(o[t][0], o[t][1]), pack_bf16(o[t][2], o[t][3]));
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) if (j < cnt) out[j] = __float2bfloat16_rn(o[t][j]);
+      }
+    }
+  }
+}
+
+// Prologue PRO_RMSNORM: the whole rows as the operand tile, bf16(x / rms * gamma).  Rows and gamma are copied with everything in flight, then a
+// warp sums and scales its own rows (16 tokens of 4096 columns: 6.5 us beside the weight stream).
+static __device__ __noinline__ void xs_stage_norm(const uint4 *src, const uint4 *gam, uint32_t xs, uint32_t gsm, int ldv, int B, int NP, int vecs, float eps) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const bool gamma_here = vecs * 16 <= kPartialBytes;
+  for (int b = warp; b < B; b += 8) {
+    const uint32_t row = xs + b * 128 + (((lane & 7) ^ (b & 7)) << 4);
+#pragma unroll 4
+    for (int v = lane; v < vecs; v += 32)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(row + (uint32_t)((v >> 3) * NP * 128)), "l"(src + (size_t)b * ldv + v) : "memory");
+  }
+  if (gamma_here)
+    for (int v = threadIdx.x; v < vecs; v += kConsumerThreads) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(gsm + v * 16), "l"(gam + v) : "memory");
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  consumer_sync();
+  for (int b = warp; b < B; b += 8) {
+    const uint32_t row = xs + b * 128 + (((lane & 7) ^ (b & 7)) << 4);
+    float ss = 0.f;
+#pragma unroll 4
+    for (int v = lane; v < vecs; v += 32) {
+      const uint4 x = lds_u4(row + (uint32_t)((v >> 3) * NP * 128));
+      const uint32_t w[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+      for (int q = 0; q < 4; ++q) ss += bf16_lo(w[q]) * bf16_lo(w[q]) + bf16_hi(w[q]) * bf16_hi(w[q]);
+    }
+    const float inv = rsqrtf(warp_sum(ss) / (float)(vecs * 8) + eps);
+#pragma unroll 4
+    for (int v = lane; v < vecs; v += 32) {
+      const uint32_t at = row + (uint32_t)((v >> 3) * NP * 128);
+      const uint4 x = lds_u4(at), g = gamma_here ? lds_u4(gsm + v * 16) : __ldg(gam + v);
+      const uint32_t xw[4] = {x.x, x.y, x.z, x.w}, gw[4] = {g.x, g.y, g.z, g.w};
+      uint32_t ow[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) ow[q] = pack_bf16(bf16_lo(xw[q]) * inv * bf16_lo(gw[q]), bf16_hi(xw[q]) * inv * bf16_hi(gw[q]));
+      asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(at), "r"(ow[0]), "r"(ow[1]), "r"(ow[2]), "r"(ow[3]) : "memory");
+    }
+  }
+  fence_proxy_async_smem();   // written with generic stores, read by the MMAs
+  consumer_sync();
+}
+
+// ---------------------------------------------------------------------------
+// TASK_LINEAR on the tensor path (general instantiation, graphs with more than 8 batched tokens): the weights are the M operand (swap-AB, as in
+// include/mirage/persistent_kernel/tasks/blackwell/linear_sm100_mpk.cuh:31-735), 128 rows per tcgen05.mma, the batched tokens the N operand
+// (16 .. 64), fp32 accumulators in tensor memory.
+//
+// The task is one pipeline along k.  A ring slot brings nkb k blocks of 64 columns of one row tile (RB <= 128 rows), all tiles of a k
+// position in turn; the activations of that position come once, for all tiles, through a ring of their own: one box {64 columns, token rows,
+// nkb blocks} of the tensor map of the layer's input, issued by warp 7 as soon as the dependency is met (PRO_RMSNORM: the whole rows are there
+// from the start).  Measured: an MMA takes a thread 64 cycles to issue and a commit 200, while the tensor pipe needs 39 (16 tokens) to 49 (64
+// tokens) for any M up to 128, so up to four warps issue, each its row tiles and chunks of k, those of different chunks into accumulators of their
+// own (`sets`, added in order by the epilogue): results do not depend on timing.  Commits hand the slots of both rings back.
+// Where a row panel per worker would be thin (a linear of few rows and long k), `splits` workers share a panel and each takes a part of k
+// (LX_*): full MMAs, and each reads its part of the activations only.  Parts meet in scratch memory in fp32; the last worker to arrive adds
+// them up in order.
+// ---------------------------------------------------------------------------
+template <int N> struct Columns { static constexpr int value = N; };
+
+template <int HYB>
+__device__ __noinline__ LinearState run_linear_tc(const Ctx c, const TaskDesc &d, LinearState ls, int task, bool ok) {
   const KernelParams &P = c.P;
+  if (!ok) return ls;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int B = ok ? min(active_tokens(P), kMaxLinearTokens) : 0;
+  const uint32_t x_par = (uint32_t)c.s.flags[3];            // parities of the next completions of the activation ring's slots
+  const int B = min(active_tokens(P), kMaxLinearTokens);
   const int NP = P.tc_tokens;                               // token rows of the operand tile / columns per accumulator
   const int Nmma = min(NP, max(16, (B + 15) & ~15));        // N of the instruction
-  const int n0 = d.a[L_N0], rows = d.a[L_N1] - n0, K = d.a[L_K], KT = d.a[L_KT], RB = d.a[L_ROWS];
-  const int nkb = d.a[L_KC] / kTcKBlock, kbt = KT / kTcKBlock;
+  const int n0 = d.a[L_N0], rows = d.a[L_N1] - n0, RB = d.a[L_ROWS];
+  const int nkb = d.a[L_KC] / kTcKBlock, kball = d.a[L_K] / kTcKBlock;
   const int tiles = (rows + RB - 1) / RB;
-  const int NST = P.num_stages;
-  const uint32_t idesc = umma_idesc(1u, 128, Nmma);
+  const XRing ring = x_ring(c, d);
+  const bool staged = d.a[L_PRO] == PRO_RMSNORM;
   const bool prof = P.profiler != nullptr && (uint64_t)(task + 1) * 8 <= P.profiler_entries;
-  // Several warps issue MMAs concurrently, and MMAs of different threads execute in no fixed order: were they to
-  // share an accumulator, the order of the fp32 additions -- and with it the last bit of the result -- would change
-  // from launch to launch.  So every issuing warp owns a SET of accumulators (set i, tile t at columns
-  // (i * tiles + t) * NP), filled only by its own MMAs, which execute in issue order; the epilogue adds the sets in
-  // set order.  As many issuers as the accumulator columns allow, eight at most.  Every MMA accumulates, so the
-  // columns start at zero: warps 0-3 clear their lane quadrants.
-  const int sets = max(1, min(8, kTcAccCols / (tiles * NP)));
-  tc_fence_after_sync();
-  if (ok && warp < 4) {
-    const uint32_t t0 = c.tmem_base + ((uint32_t)(warp * 32) << 16);
-    for (int col = 0; col < sets * tiles * NP; col += 16) tmem_st_zero_x16(t0 + (uint32_t)col);
-    tmem_st_wait();
-  }
-  tc_fence_before_sync();
-  // descriptor templates: shared-memory addresses enter as (address >> 4) in the low 14 bits
-  const uint64_t desc_hi = umma_desc_k_sw128(0);
-  const uint32_t x_base = smem_u32(c.s.xtile) >> 4;
-  for (int kt = 0; kt < K; kt += KT) {
-    if (ok && !((d.flags & TF_SAME_X_AS_PREV) && KT == K)) {
-      stage_x<2>(c, d, B, kt, KT, gpre);   // (a barrier of the compute warps precedes every return)
-      fence_proxy_async_smem();            // the tile was written with generic stores; the MMA reads it through the async proxy
-    }
-    consumer_sync();
-    tc_fence_after_sync();
-    if (tid == 0 && prof && kt == 0) P.profiler[(size_t)task * 8 + 4] = globaltimer_ns();
-    // Ring slots in stream order (row tile, then k blocks).  A slot holds nkb k blocks = 4 nkb MMAs of K = 16; warp w
-    // issues MMAs w, w + 8, ... of the slot from its lane 0 and then commits to the slot's empty barrier, which
-    // counts eight arrivals: the slot returns to the streaming warp when the MMAs of all warps have read it.
-    for (int tile = 0; tile < tiles; ++tile) {
-      const uint32_t d_tmem = c.tmem_base + (uint32_t)((warp * tiles + tile) * NP);   // (used by warps < sets only)
-      for (int kb = 0; kb < kbt; kb += nkb) {
-        const int s = ls.stage;
-        const uint32_t ph = ls.phase;
-        if (++ls.stage == NST) { ls.stage = 0; ls.phase ^= 1u; }
-        if (ok) ok = wait_mbar(c, &c.s.full[s], ph, task);
-        if (ok && lane == 0) {
-          tc_fence_after_sync();
-          const uint32_t a_base = smem_u32(c.s.stages + (size_t)s * P.stage_bytes) >> 4;
-          for (int m = warp; warp < sets && m < nkb * 4; m += sets) {
-            const int j = m >> 2, ks = m & 3;
-            const uint32_t a_lo = a_base + (uint32_t)(j * RB * 8 + ks * 2);
-            const uint32_t b_lo = x_base + (uint32_t)((kb + j) * NP * 8 + ks * 2);
-            umma_bf16_acc(d_tmem, desc_hi | a_lo, desc_hi | b_lo, idesc);
-          }
-          umma_commit(&c.s.empty[s]);
+  uint64_t *xfull = x_bars(c), *xempty = xfull + 8;
+  const uint32_t x_chunk = (uint32_t)(NP * nkb * 128);                // bytes of a ring chunk
+  const int nx = d.a[LX_NX], nch = (kball + nkb - 1) / nkb;
+  // where the ring stands: borrowing tasks start at its first slot (ls.phase: a bit per slot), others follow on
+  const int s0 = P.borrow ? 0 : ls.stage;
+  const uint32_t par0 = P.borrow ? ls.phase : (ls.phase ? 0xffffu : 0u) ^ ((1u << ls.stage) - 1u);
+  if (tid == 0 && ring.size > ring.base && nch * tiles > ring.base) mbar_arrive(ring.xbars + 32);   // (the tile area is free: all threads are past their last task)
+  const uint32_t xs_smem = smem_u32(c.s.xtile);
+  // Issuing warps.  A warp must neither fall a lap of a ring behind nor run one ahead (a barrier's parity says no more than that), and following slots
+  // that are another's costs 300 cycles each; so a slot belongs to one warp, by row tile and by chunk.  Measured (64 tokens, two row tiles, chunks of one
+  // k block): a chunk takes a warp 1550 cycles, 670 of them for four MMAs and their commit, so that two warps drew 3.7 TB/s.
+  const XIssuers wi = x_issuers(tiles, ring.size, staged ? 0 : nx);
+  const int issuers = wi.tiles * wi.chunks, sets = min(wi.chunks, nch);
+  if (staged)
+    xs_stage_norm(reinterpret_cast<const uint4 *>(d.p[1]), reinterpret_cast<const uint4 *>(d.p[4]), xs_smem, smem_u32(c.s.partial), d.a[L_LDX] >> 3, B, NP,
+                  d.a[L_K] / 8, __int_as_float(d.a[L_EPS]));
+  if (warp < issuers) {
+    const uint32_t idesc = umma_idesc(1u, 128, Nmma);
+    const uint64_t desc_hi = umma_desc_k_sw128(0);   // shared-memory addresses enter as (address >> 4) in the low 14 bits
+    const int first = warp / wi.tiles, tile0 = warp - first * wi.tiles;   // chunk and row tile of this warp
+    int xslot = 0;
+    uint32_t par = par0, xpar = x_par;
+    int s = s0;
+    for (int i = 0; i < nch && ok; ++i) {
+      const bool mine = (i & (wi.chunks - 1)) == first;   // (a power of two)
+      if (mine) {
+        const int kb = i * nkb, nb = min(nkb, kball - kb);
+        uint32_t xa = xs_smem >> 4;
+        if (staged) {
+          xa += (uint32_t)(kb * NP * 8);
+        } else {
+          ok = wait_mbar(c, &xfull[xslot], (xpar >> xslot) & 1u, task);
+          xa += (uint32_t)xslot * (x_chunk >> 4);
         }
+        if (prof && tid == 0 && i == 0) P.profiler[(size_t)task * 8 + 4] = globaltimer_ns();
+        for (int tile = tile0; tile < tiles && ok; tile += wi.tiles) {
+          const int sl = s + tile < ring.size ? s + tile : s + tile - ring.size;
+          ok = wait_mbar(c, ring.full_bar(sl), (par >> sl) & 1u, task);
+          if (!ok) break;
+          if (lane == 0) {
+            tc_fence_after_sync();
+            const uint32_t wa = ring.slot(sl) >> 4, dt = c.tmem_base + (uint32_t)((first * tiles + tile) * NP);
+            for (int j = 0; j < nb; ++j) {
+              const uint64_t a0 = desc_hi | (wa + (uint32_t)(j * RB * 8)), b0 = desc_hi | (xa + (uint32_t)(j * NP * 8));
+#pragma unroll
+              for (int ks = 0; ks < 4; ++ks) umma_bf16(dt, a0 + ks * 2, b0 + ks * 2, idesc, i - first + j + ks > 0 ? 1u : 0u);
+            }
+            if (!P.borrow) mbar_arrive_n(ring.empty_bar(sl), 7);   // (the slot's barrier counts the eight warps of the other bodies)
+            umma_commit(ring.empty_bar(sl));
+          }
+          __syncwarp();
+        }
+        if (!staged && lane == 0 && ok) umma_commit(&xempty[xslot]);
         __syncwarp();
       }
+      // on by the chunk's boxes: a pass over the ring's end flips the parities of its slots
+      par ^= ((1u << tiles) - 1u) << s;
+      s += tiles;
+      if (s >= ring.size) { s -= ring.size; par = (par & ((1u << ring.size) - 1u)) ^ ((1u << s) - 1u); }
+      xpar ^= 1u << xslot;
+      if (++xslot == nx) xslot = 0;
     }
-    // accumulators complete for this k tile / activation tile free again: one arrival per warp
-    if (lane == 0) umma_commit(c.s.acc_bar);
-    if (!wait_mbar(c, c.s.acc_bar, ls.acc_phase, task)) ok = false;
-    ls.acc_phase ^= 1u;
-    if (!ok) c.s.flags[0] = 1;
-    consumer_sync();
-    ok = ok && (c.s.flags[0] == 0);
-    if (!ok) break;
-  }
-  if (tid == 0 && prof) P.profiler[(size_t)task * 8 + 5] = globaltimer_ns();
-  if (!ok) { c.s.flags[0] = 1; return; }
-  tc_fence_after_sync();
-  if (B > 0) {
-    const int quad = warp & 3, half = warp >> 2;
-    const int nh = Nmma >> 1;   // a multiple of 8
-    const EmitArgs ea = emit_args(c, d);
-    const int epi = ea.epi;
-    const __nv_bfloat16 *resp = reinterpret_cast<const __nv_bfloat16 *>(d.p[3]);
-    const int ldr = d.a[L_LDR];
-    for (int tile = 0; tile < tiles; ++tile) {
-      if (quad * 32 >= RB) break;                           // this warp's lanes hold no row of a tile (warp-uniform)
-      const int r_in_tile = quad * 32 + lane;
-      const int row = tile * RB + r_in_tile;
-      const bool row_ok = r_in_tile < RB && row < rows;
-      const uint32_t taddr = c.tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(tile * NP + half * nh);
-      float bias = 0.f;
-      if (HYB && epi == EPI_BIAS_F32 && row_ok) bias = bf16_to_f(__ldg(*reinterpret_cast<const __nv_bfloat16 *const *>(&d.a[LR_BIAS]) + n0 + row));
-      for (int c0 = 0; c0 < nh; c0 += 8) {
-        uint32_t r[8];
-        tmem_ld_x8(taddr + (uint32_t)c0, r);
-        for (int st = 1; st < sets; ++st) {   // the other issuers' accumulators of this tile, in set order
-          uint32_t r2[8];
-          tmem_ld_wait();
-          tmem_ld_x8(taddr + (uint32_t)(st * tiles * NP + c0), r2);
-          tmem_ld_wait();
-#pragma unroll
-          for (int j = 0; j < 8; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(r2[j]));
-        }
-        // residual values of the group's eight tokens: all loads in flight together, ahead of the stores (which the
-        // compiler may not move them across: the output may alias the residual)
-        float resv[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const int b = half * nh + c0 + j;
-          resv[j] = HYB ? bias : 0.f;
-          if (epi == EPI_RESIDUAL && row_ok && b < B)
-            resv[j] = bf16_to_f(__ldcg(resp + (size_t)b * ldr + n0 + row));
-          if (HYB && epi == EPI_GATE_SIGMOID && row_ok && b < B) resv[j] = __ldcg(reinterpret_cast<const float *>(resp) + (size_t)b * ldr + n0 + row);
-        }
-        tmem_ld_wait();
-        if (tid == 0 && prof && tile == 0 && c0 == 0) P.profiler[(size_t)task * 8 + 6] = globaltimer_ns();
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const float v = __uint_as_float(r[j]);
-          const float u = (epi == EPI_SILU_PAIR || (HYB && (epi == EPI_GATED_SILU || epi == EPI_GATED_GELU))) ? __shfl_down_sync(0xffffffffu, v, 2) : 0.f;
-          const int b = half * nh + c0 + j;
-          if (row_ok && b < B) linear_emit<HYB>(c, ea, b, n0 + row, v, u, resv[j]);
-        }
-        if (tid == 0 && prof && tile == 0 && c0 == 0) P.profiler[(size_t)task * 8 + 7] = globaltimer_ns();
+    if (lane == 0 && ok) {
+      if (warp == 0) mbar_arrive_n(c.s.acc_bar, 8 - issuers);
+      umma_commit(c.s.acc_bar);
+    }
+    __syncwarp();
+  } else if (warp == 7 && !staged) {
+    if (lane == 0) {
+      const uint8_t *xmap = reinterpret_cast<const uint8_t *>(P.tmaps) + (size_t)d.a[LX_TMAP] * 128;
+      uint32_t xpar = x_par;
+      int xslot = 0, issued = 0;
+      bool good = true;
+      fence_proxy_async_all();   // the activations were written through the generic proxy
+      for (int i = 0; i < nch && good; ++i) {
+        if (i >= nx) good = wait_mbar(c, &xempty[xslot], ((xpar >> xslot) & 1u) ^ 1u, task);
+        if (!good) break;
+        mbar_arrive_expect_tx(&xfull[xslot], x_chunk);
+        if (wi.tiles < kXIssuers) mbar_arrive_n(&xempty[xslot], kXIssuers - wi.tiles);   // (of the arrivals its barrier counts; a warp of each row tile commits)
+        tma_load_3d_shared(xs_smem + (uint32_t)xslot * x_chunk, xmap, 0, 0, i * nkb, smem_u32(&xfull[xslot]));
+        xpar ^= 1u << xslot;
+        if (++xslot == nx) xslot = 0;
+        ++issued;
+      }
+      // the launch is being abandoned: what this thread issued lands before the CTA may exit
+      for (int i = 0; !good && i < min(issued, nx); ++i) {
+        uint32_t polls = 0;
+        while (!mbar_try_wait(&xfull[i], ((xpar >> i) & 1u) ^ 1u) && ++polls < (1u << 24)) {}
       }
     }
+    __syncwarp();
+  }
+  // what all threads know about the rings after this task
+  {
+    const int used = s0 + nch * tiles;
+    if (P.borrow) {
+      const int laps = used / ring.size, rest = used - laps * ring.size;
+      ls.phase ^= ((laps & 1 ? 0xffffu : 0u) ^ ((1u << rest) - 1u)) & ((1u << ring.size) - 1u);
+    } else {
+      ls.phase ^= (uint32_t)(used / ring.size) & 1u;
+      ls.stage = used % ring.size;
+    }
+  }
+  if (!wait_mbar(c, c.s.acc_bar, ls.acc_phase, task)) ok = false;
+  ls.acc_phase ^= 1u;
+  if (!ok) c.s.flags[0] = 1;
+  consumer_sync();
+  if (c.s.flags[0] != 0) return ls;
+  tc_fence_after_sync();
+  if (tid == 0 && !staged) {
+    uint32_t flips = 0;
+    for (int i = 0; i < nx; ++i) flips |= (uint32_t)((nch + nx - 1 - i) / nx & 1) << i;
+    c.s.flags[3] = (int)(x_par ^ flips);
+  }
+  if (tid == 0 && prof) P.profiler[(size_t)task * 8 + 5] = globaltimer_ns();
+  if (B == 0) { tc_fence_before_sync(); return ls; }
+  // Epilogue.  A warp reads its lane quadrant of half the tokens, adds the sets and leaves the sums as [token][row] in shared memory (the tile
+  // area is free now), or in scratch memory where the panel is shared; then a warp takes a token at a time, four rows a lane.  Straight from
+  // the accumulators to the output, a row per lane, it took 1 to 1.5 us for eight tokens of a tile: long unrolled code that leaves the
+  // instruction caches at each pass, and stores of single elements (64 tokens, gate and up rows of width 4096: 25 us before, 6 now).
+  const int quad = warp & 3, half = warp >> 2;
+  const int nh = Nmma >> 1;   // tokens of a warp's half: a multiple of 8
+  const int S = d.a[LX_SPLITS];
+  float *sums = reinterpret_cast<float *>(c.s.xtile);
+  const size_t part_floats = (size_t)tiles * NP * RB;
+  if (S > 1) sums = P.split_scratch + d.p[6] + (size_t)d.a[LX_PART] * part_floats;
+  const int fit = S > 1 ? tiles : P.x_tile_bytes / (NP * RB * 4);   // row tiles at a time
+  XsOut xo{emit_args(c, d), reinterpret_cast<const uint8_t *>(d.p[3]), d.a[L_LDR], false};
+  {
+    const int epi = xo.e.epi;
+    const bool f32 = HYB && (epi == EPI_STORE_F32 || epi == EPI_BIAS_F32 || epi == EPI_SOFTCAP || epi == EPI_SCALE_F32);
+    if (HYB && epi == EPI_BIAS_F32) { xo.operand = *reinterpret_cast<const uint8_t *const *>(&d.a[LR_BIAS]); xo.ldr = 0; }
+    const bool reads = epi == EPI_RESIDUAL || (HYB && epi == EPI_BIAS_F32);
+    xo.wide = (n0 & 3) == 0 && (reinterpret_cast<uintptr_t>(xo.e.out) & (f32 ? 15 : 7)) == 0 && (xo.e.ldo & 3) == 0 &&
+              (!reads || ((reinterpret_cast<uintptr_t>(xo.operand) & 7) == 0 && (xo.ldr & 3) == 0));
+  }
+  for (int tile0 = 0; tile0 < tiles; tile0 += fit) {
+    const int tile1 = min(tiles, tile0 + fit);
+    if (tile0 > 0) consumer_sync();
+    for (int tile = tile0; quad * 32 < RB && tile < tile1; ++tile) {
+      const uint32_t at = c.tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(tile * NP + half * nh);
+      float *dst = sums + (size_t)((tile - tile0) * NP + half * nh) * RB + quad * 32 + lane;
+      const bool keep = quad * 32 + lane < RB;
+      const auto add_sets = [&](auto n, int c0) {
+        constexpr int kCols = decltype(n)::value;
+        float v[kCols];
+#pragma unroll
+        for (int j = 0; j < kCols; ++j) v[j] = 0.f;
+#pragma unroll 1
+        for (int q = 0; q < sets; ++q) {   // (two loads at a time cost the kernel that calls this 260 bytes of spills)
+          uint32_t r[kCols];
+          tmem_ld(at + (uint32_t)(q * tiles * NP + c0), r);
+          tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < kCols; ++j) v[j] += __uint_as_float(r[j]);
+        }
+        if (keep)
+#pragma unroll
+          for (int j = 0; j < kCols; ++j) dst[(c0 + j) * RB] = v[j];
+      };
+      int c0 = 0;
+#pragma unroll 1
+      for (; c0 + 16 <= nh; c0 += 16) add_sets(Columns<16>(), c0);
+      if (c0 < nh) add_sets(Columns<8>(), c0);
+    }
+    if (S > 1) {
+      __threadfence();
+      consumer_sync();
+      if (tid == 0) {
+        unsigned int *ticket = P.attn_tickets + d.a[LX_TICKET];
+        const unsigned int old = atomicAdd(ticket, 1u);
+        __threadfence();
+        if (old == (unsigned)S - 1u) *ticket = 0u;   // (its next use waits for this task)
+        c.s.flags[1] = old == (unsigned)S - 1u ? 1 : 0;
+      }
+      consumer_sync();
+      if (c.s.flags[1] == 0) break;
+      sums = P.split_scratch + d.p[6];
+    } else {
+      consumer_sync();
+    }
+    if (tid == 0 && prof && tile0 == 0) P.profiler[(size_t)task * 8 + 6] = globaltimer_ns();
+    const int lanes = RB > 64 ? 32 : RB > 32 ? 16 : 8, sub = lane & (lanes - 1), step = 8 * (32 / lanes);
+    const int r0 = sub * 4;
+    for (int tile = tile0; r0 < RB && tile < tile1; ++tile) {
+      const int row = tile * RB + r0, cnt = min(4, rows - row);
+      if (cnt <= 0) break;
+      const size_t src = (size_t)(tile - tile0) * NP * RB + r0;
+#pragma unroll 1
+      for (int b = warp * (32 / lanes) + lane / lanes; b < B; b += 2 * step) {   // two tokens at a time, so that their chains overlap
+        float v[2][4];
+        const int b1 = min(b + step, B - 1);
+        if (S > 1) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) v[0][j] = v[1][j] = 0.f;
+#pragma unroll 2
+          for (int p = 0; p < S; ++p) {
+            const float *at = sums + (size_t)p * part_floats + src;
+            const float4 t = __ldcg(reinterpret_cast<const float4 *>(at + (size_t)b * RB)), u = __ldcg(reinterpret_cast<const float4 *>(at + (size_t)b1 * RB));
+            v[0][0] += t.x; v[0][1] += t.y; v[0][2] += t.z; v[0][3] += t.w;
+            v[1][0] += u.x; v[1][1] += u.y; v[1][2] += u.z; v[1][3] += u.w;
+          }
+        } else {
+          lds_f4(xs_smem + (uint32_t)(src + (size_t)b * RB) * 4, v[0]);
+          lds_f4(xs_smem + (uint32_t)(src + (size_t)b1 * RB) * 4, v[1]);
+        }
+        xs_emit<HYB>(c, xo, b, b + step < B ? b1 : -1, n0 + row, cnt, v);
+      }
+    }
+    if (tid == 0 && prof && tile0 == 0) P.profiler[(size_t)task * 8 + 7] = globaltimer_ns();
   }
   tc_fence_before_sync();   // the accumulators have been read: the next task's MMAs may overwrite them after the task barrier
+  return ls;
 }
 
 // ---------------------------------------------------------------------------
@@ -4520,6 +4848,12 @@ __device__ __forceinline__ bool task_linear(const Ctx &c, const TaskDesc &d, int
   const int tid = threadIdx.x;
   // constants the prologue needs are fetched before the dependency wait
   uint4 gpre[2] = {make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0)};
+  if (GENERAL && (d.flags & TF_TC) && !(d.flags & TF_FP8)) {
+    fence_proxy_async_smem();   // the tile area was used by generic accesses; what comes next writes it by tensor-map copies
+    ok = wait_dependencies(c, d, t, ok, tt);
+    ls = run_linear_tc<HYB>(c, d, ls, t, ok);
+    return ok;
+  }
   if (d.a[L_PRO] == PRO_RMSNORM) {
     const uint4 *gam = reinterpret_cast<const uint4 *>(d.p[4]);
     const int vecs = d.a[L_KT] / 8;
@@ -4529,7 +4863,6 @@ __device__ __forceinline__ bool task_linear(const Ctx &c, const TaskDesc &d, int
   ok = wait_dependencies(c, d, t, ok, tt);
   // the weight chunks must be consumed even when the launch is being abandoned or no token is active
   if (GENERAL && !HYB && (d.flags & TF_TC) && (d.flags & TF_FP8)) run_linear_fp8_tc(c, d, ls, t, ok);
-  else if (GENERAL && (d.flags & TF_TC)) run_linear_tc<HYB>(c, d, ls, t, gpre, ok);
   else if (GENERAL && !HYB && (d.flags & TF_FP8)) run_linear_fp8(c, d, ls, t, ok);
   else run_linear<GENERAL, TPX, HYB>(c, d, ls, t, gpre, ok);
   return ok;
@@ -4684,13 +5017,19 @@ __global__ void __launch_bounds__(block_threads(GENERAL), 1) mpk_megakernel(cons
     s.flags[0] = 0;
     s.flags[1] = 0;
     s.flags[2] = 0;
+    s.flags[3] = 0;   // (run_linear_tc)
     if (!GENERAL) *reinterpret_cast<volatile int *>(&s.full[8]) = -1;   // attention stash: empty
     if (GENERAL) {
       mbar_init(s.acc_bar, 8);   // one tcgen05.commit per compute warp
-      for (int i = 0; i < 8 * kAttnStages; ++i) mbar_init(reinterpret_cast<uint64_t *>(s.flags + 16) + i, 1);
       for (int i = 0; i < 8; ++i) s.flags[16 + 16 * kAttnStages + i] = 0;
       if (P.attn_table_bytes) *reinterpret_cast<int *>(reinterpret_cast<uint8_t *>(s.flags) - kFlagsOffset + kMiscBytes) = -1;   // the request table: not built
     }
+    mbar_fence_init();
+  }
+  if (GENERAL && tid >= 64 && tid < 128) {   // (one thread for all of them: 1 us of every launch)
+    const int i = tid - 64;
+    if (i < 8 * kAttnStages) mbar_init(reinterpret_cast<uint64_t *>(s.flags + 16) + i, 1);
+    if (i < 33) mbar_init(s.full + kXBarsOffset / 8 + i, i < 8 ? 1 : i < 16 ? kXIssuers : i >= 24 && i < 32 ? 8 : 1);
     mbar_fence_init();
   }
   // graphs with tcgen05 tasks: warp 0 takes all 512 tensor-memory columns (one CTA per SM, so nothing else asks)
@@ -4704,7 +5043,12 @@ __global__ void __launch_bounds__(block_threads(GENERAL), 1) mpk_megakernel(cons
   const int t_begin = P.worker_begin[blockIdx.x], t_end = P.worker_begin[blockIdx.x + 1];
   if (tid >= kConsumerThreads) {
     if (GENERAL) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kStreamerRegs));
-    if (tid < kConsumerThreads + 32) streamer_loop<GENERAL, HYB>(c, t_begin, t_end);
+    if (GENERAL && P.borrow) {
+      if ((tid & 31) == 0) stream_borrowing(c, t_begin, t_end);
+      __syncwarp();
+    } else if (tid < kConsumerThreads + 32) {
+      streamer_loop<GENERAL, HYB>(c, t_begin, t_end);
+    }
   } else {
     if (GENERAL) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kConsumerRegs));
     consumer_loop<GENERAL, TPX, HYB>(c, t_begin, t_end);

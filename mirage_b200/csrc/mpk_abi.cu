@@ -86,6 +86,7 @@ struct mpk_handle {
   int32_t *d_request_ids = nullptr, *d_state_slots = nullptr, *d_page_queue = nullptr, *d_sched = nullptr;
   float *d_attn_scratch = nullptr;
   unsigned int *d_attn_tickets = nullptr;
+  float *d_split_scratch = nullptr;   // parts of linears that are split along k
   void *d_tmaps = nullptr;            // tensor maps of the tcgen05 linear tasks
   KernelParams params;
   KernelFamily kernels;
@@ -409,6 +410,7 @@ int mpk_compile(mpk_handle *h) {
   rc = dev_alloc(h, (void **)&h->d_page_queue, (uint64_t)std::max(cfg.max_num_pages, 1) * 4); if (rc) return rc;
   rc = dev_alloc(h, (void **)&h->d_sched, 64); if (rc) return rc;
   rc = dev_alloc(h, (void **)&h->d_attn_scratch, (uint64_t)g.attn_scratch_floats * 4); if (rc) return rc;
+  if (g.split_floats > 0) { rc = dev_alloc(h, (void **)&h->d_split_scratch, (uint64_t)g.split_floats * 4, false); if (rc) return rc; }
   rc = dev_alloc(h, (void **)&h->d_attn_tickets, (uint64_t)std::max<int64_t>(g.attn_tickets, 1) * 4); if (rc) return rc;
   rc = dev_alloc(h, (void **)&h->d_tasks, (uint64_t)g.tasks.size() * sizeof(TaskDesc), false); if (rc) return rc;
   rc = dev_alloc(h, (void **)&h->d_worker_begin, (uint64_t)(W + 1) * 4, false); if (rc) return rc;
@@ -441,6 +443,8 @@ int mpk_compile(mpk_handle *h) {
   P.meta.request_ctl = (cfg.mode == MPK_MODE_ONLINE && !cfg.test_mode) ? cfg.request_ctl : nullptr;
   P.attn_scratch = h->d_attn_scratch;
   P.attn_tickets = h->d_attn_tickets;
+  P.split_scratch = h->d_split_scratch;
+  P.borrow = g.borrow ? 1 : 0;
   P.profiler = cfg.profiler_buffer;
   P.profiler_entries = cfg.profiler_entries;
   P.eos_token_id = cfg.eos_token_id;

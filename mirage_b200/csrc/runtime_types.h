@@ -14,7 +14,7 @@ constexpr int kMaxDeps = 3;
 constexpr int kConsumerThreads = 256;          // 8 compute warps
 // + 1 weight-streaming warp.  That ninth warp costs the compute warps a third of the register file (three warps on a scheduler instead
 // of two: 168 registers a thread), and what is spilled comes back from L2: beside 220 KB of shared memory there is next to no L1.  So in
-// the general instantiations the streaming warp is the first of a warpgroup (the other three idle) that hands its registers over.
+// the general instantiations the streaming warp is the first of a warpgroup (the other three help it where all streaming is by tensor-map copies) that hands its registers over.
 // 36 layers of width 4096: 16 requests 7842 -> 7539 us, 64 requests 12.58 -> 12.05 ms, 64 prompt tokens 16.90 -> 14.58 ms (88 or 104 registers
 // for the streaming warp: 1 % slower).  Not in the narrow instantiations: their streaming warp copies row by row and loses more to
 // spills than their bodies gain (one request 3.34 -> 3.53 ms).
@@ -92,6 +92,18 @@ enum TaskType : uint32_t {
 MPK_HD constexpr int mlstm_quads(int dim) { return dim <= 128 ? 16 : (dim <= 256 ? 8 : (dim <= 512 ? 4 : 2)); }
 MPK_HD constexpr int mlstm_rows_per_thread(int dim) { return dim > 64 ? 8 : 4; }
 MPK_HD constexpr int mlstm_rows(int dim) { return kConsumerThreads / mlstm_quads(dim) * mlstm_rows_per_thread(dim); }
+
+// Warps that issue the MMAs of a tcgen05 linear task: `tiles` of them share out its row tiles, `chunks` (a power of two) the chunks of k.  Each ring slot
+// is one warp's, so the sizes of the rings (`slots` of the weights, `nx` of the activations or 0) are multiples.
+struct XIssuers { int tiles, chunks; };
+MPK_HD constexpr XIssuers x_issuers(int tiles, int slots, int nx) {
+  if (tiles <= 2)
+    for (int n = 4 / tiles; n > 1; n >>= 1)
+      if (slots % (n * tiles) == 0 && nx % n == 0) return {tiles, n};
+  for (int n = 5; n > 1; --n)
+    if (tiles % n == 0 && slots % n == 0) return {n, 1};
+  return {1, 1};
+}
 
 // Query rows a bf16 extended-attention task keeps in shared memory: whole 16-row tiles, a power of two of them (the
 // warps are split over the tiles), at most as many as the graph can batch.
@@ -197,9 +209,15 @@ static_assert(sizeof(TaskDesc) == 16 * kDescVecs, "TaskDesc must stay 224 bytes 
 //  tcgen05 path (TF_TC): a[18] rows of one weight tile (the TMA box height, a multiple of 8, at most 128; the task's rows are
 //        cut into ceil(rows / a[18]) tiles, each one 128-lane accumulator), a[12] = 64 x (k blocks of 64 columns per ring slot),
 //        a[27] index of the task's tensor map (dims {64, rows of the task, K / 64}, box {64, a[18], a[12] / 64}, 128-byte swizzle)
+//        a[11] = a[12]; tasks that share a row panel: a[2] columns of the task's part of k, a[LX_SPLITS] parts, a[LX_PART] this one, p[6] their place in the
+//        scratch memory of split linears (floats), a[LX_TICKET] their ticket;  a[LX_TMAP] tensor map of the activations (dims {64, token rows, K / 64},
+//        box {64, token rows of the operand tile, a[12] / 64}; PRO_RMSNORM: none), a[LX_NX] chunks of their ring, a[LX_XBYTES] bytes they take of the tile
+//        area, a[LX_EXTRA] weight slots behind them
 enum { L_N0 = 0, L_N1, L_K, L_LDW, L_LDX, L_LDO, L_LDR, L_PRO, L_EPI, L_EPS, L_GROUPS, L_KT, L_KC, L_SLOT, L_N, L_ARIDX, L_NAR, L_PARSTRIDE, L_ROWS,
        L_GATHER, L_G_LDRES, L_G_LDOUT, L_G_SLOT, L_WS_S0, L_WS_S1, L_XS_S0, L_XS_S1, L_TMAP };
 static_assert(L_TMAP == 27, "TaskDesc::a has 28 entries");
+enum { LX_NX = 10, LX_EXTRA = 19, LX_TMAP, LX_SPLITS, LX_PART, LX_TICKET = 26 };
+constexpr int LX_XBYTES = L_LDW;   // tcgen05 path (the fields of allreduce prologues and folded norms are free there)
 enum { LR_POST = 13, LR_ADD = 14, LR_ROW = 16, L_CAP = 23, LR_BIAS = 24, LR_LDADD = 26 };   // hybrid graphs (the fields of allreduces and FP8 tasks are free there)
 // ---- TASK_ATTENTION ----------------------------------------------------------
 //  p[0] qkv  p[1] k_cache  p[2] v_cache  p[3] q_norm  p[4] k_norm  p[5] cos  p[6] sin  p[7] out
@@ -384,6 +402,8 @@ struct KernelParams {
   int32_t attn_table_bytes;             // area of the attention tasks' request table, behind the small things (general instantiation)
   int32_t meta_static;                  // the batch description is the caller's and final at launch (test mode, online_notoken):
                                         // the graph has no batching task
+  float *split_scratch;                 // parts of linears that are split along k
+  int32_t borrow;                       // all streaming tasks are tcgen05 linears: they borrow weight slots from the tile area
 };
 
 }  // namespace mpk

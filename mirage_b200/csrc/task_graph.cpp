@@ -45,6 +45,9 @@ struct Builder {
   int rot = 0;
   static constexpr int kMaxFoldedTerms = 16;   // results a linear's prologue averages at most: every task of the linear reads them all
   TaskDesc xattn_task;      // the last extended-attention task (its merge layer shares the fields)
+  int split_tickets = 0;    // tickets handed to the panels of split linears
+  std::vector<int64_t> split_banks;   // floats of the scratch banks of split linears
+  std::map<int, int> split_bank_of;   // exec layer -> its bank
   int hybrid_tickets = 0;   // arrival tickets handed to the tasks of hybrid graphs
   std::map<int, std::map<int, int>> slices;   // storage -> (first column -> id) of outputs that layers write by column range
 
@@ -93,6 +96,93 @@ struct Builder {
   }
   int64_t linear_tile_bytes(int64_t K) const {
     return tc_linear(K) ? (int64_t)tc_np() * K * 2 : (int64_t)nb_max * (K * 2 + kRowPadBytes);
+  }
+
+  // Ring of the activations of tcgen05 linears: 8 k blocks (512 columns) of all token rows, at least 32 KB.
+  int64_t x_ring_bytes() const { return std::max<int64_t>(32 * 1024, (int64_t)tc_np() * 128 * 8); }
+  static bool bf16_linear(const LayerInfo &l) { return l.op == MPK_OP_LINEAR || l.op == MPK_OP_LINEAR_RESIDUAL || l.op == MPK_OP_SPLITK_LINEAR; }
+  // Rows of a tcgen05 linear that stay in one task: pairs of gate and up rows; otherwise what the epilogue stores at once, where the rows allow it.
+  int row_unit(const LayerInfo &l) const { return T[l.t[1]].dim(0) % 4 == 0 ? 4 : 1; }
+  // row tiles of a task: one for each issuing warp (five where the ring, which follows on from task to task, has five slots)
+  int tc_task_tiles(int slots) const { return std::max(1, std::min(!g->borrow && slots == 5 ? 5 : 4, kTcAccCols / tc_np())); }
+  // Cut of a tcgen05 linear: `splits` workers share a row panel and take a part of k each.  Per worker the weights, the activations (once for
+  // all row tiles of a task) and the MMAs run side by side, so the slowest of them counts; a split pays for writing, counting and adding the
+  // parts.  The ring proper is full when the task starts.  Rates measured on these parts: a worker draws its 148th of 6.5 TB/s of weights with 100 KB in
+  // flight, fills shared memory at 75 KB/us over all, a chunk of activations takes 2 us from its copy to its release, an M = 128 MMA takes the tensor pipe 25 ns, a box costs
+  // its streaming thread 290 cycles, an MMA its issuing thread 64 and a commit 200 (two a chunk, and the waits), a row tile's epilogue 20 ns a token.
+  struct SplitPlan { int splits = 0, groups = 0, tiles = 0, rb = 0, nkb = 0; double us = 0; };
+  // Activations and borrowed weight slots of a task in the tile area: a ring of `nx` chunks that covers as much of k as the weight slots do (at
+  // least three, at most eight), slots behind it.  An MMA reads 128 rows whatever the box holds: what it reads behind the last slot has to be shared memory.
+  struct TilePlan { int nx = 0, bytes = 0, extra = 0; XIssuers issuers{1, 1}; };
+  TilePlan plan_tile(int64_t K, bool staged, int tiles, int rb, int nkb, int slot_bytes, int slots, int64_t tile_bytes) const {
+    TilePlan p;
+    const int chunk = tc_np() * 128 * nkb, nmax = (int)std::min<int64_t>(8, tile_bytes / chunk);
+    auto slots_behind = [&](int64_t bytes) {
+      if (!g->borrow) return 0;
+      int n = 0;
+      while (n < 8 && bytes + (int64_t)(n + 1) * slot_bytes <= tile_bytes &&
+             bytes + (int64_t)n * slot_bytes + (int64_t)(nkb - 1) * rb * 128 + 128 * 128 <= tile_bytes + kPartialBytes + kMiscBytes) ++n;
+      return n;
+    };
+    // the warps that issue share the rings' slots out among themselves (x_issuers in megakernel.cuh)
+    // as many warps to a row tile as keep up with the stream, the chunks shared out among them
+    int parts = 1;
+    while (2 * parts * tiles <= 4 && (staged || 2 * parts <= nmax) && (nkb * 256 + 900) / (1.9e3 * parts) > 0.8 * tiles * rb * nkb * 128 / 44e3) parts *= 2;
+    // a multiple of the warps, two slots for each where there are as many
+    auto fitted = [&]() {
+      int n = slots + slots_behind(p.bytes);
+      if (g->borrow) {
+        int warps = std::min(tiles, 4) * parts;
+        while (n < 2 * warps && warps > std::min(tiles, 4)) warps /= 2;
+        if (n >= warps) n = n / warps * warps;
+      }
+      p.extra = n - slots;
+      p.issuers = x_issuers(tiles, n, p.nx);
+    };
+    if (staged) {
+      p.bytes = (int)((tc_np() * K * 2 + 1023) / 1024 * 1024);
+      fitted();
+      return p;
+    }
+    const int step = std::max(1, parts);
+    for (p.nx = std::min(step < 3 ? 4 : step, nmax) / step * step; ; p.nx += step) {
+      p.bytes = (p.nx * chunk + 1023) / 1024 * 1024;
+      fitted();
+      if (p.nx + step > nmax || p.nx * tiles > slots + p.extra) return p;
+    }
+  }
+  std::map<std::vector<int64_t>, SplitPlan> plans;   // layers of one shape share a plan
+  const SplitPlan &plan_split(int64_t N, int64_t K, int unit, bool staged, int slot_bytes, int slots, int64_t tile_bytes) {
+    SplitPlan &best = plans[{N, K, unit, staged, slot_bytes, slots, tile_bytes}];
+    if (best.splits > 0) return best;
+    const int kb = (int)(K / kTcKBlock), max_tiles = tc_task_tiles(slots);
+    const int64_t units = (N + unit - 1) / unit;
+    for (int S = 1; S <= 8 && S <= W; ++S) {
+      if (S > 1 && (staged || kb / S < 8)) break;
+      const int groups = (int)std::min<int64_t>(W / S, units), kbs = (kb + S - 1) / S;
+      const int64_t cnt = (units + groups - 1) / groups * unit;
+      const int tmin = (int)((cnt + 127) / 128);
+      if (S > 1 && tmin > max_tiles) break;
+      for (int tiles = tmin; tiles <= tmin + 3; ++tiles) {
+        const int rb = (int)(((cnt + tiles - 1) / tiles + 7) / 8 * 8);
+        if (rb > 128 || (S > 1 && tiles > max_tiles)) continue;
+        for (int nkb = std::min({kbs, slot_bytes / (rb * 128), 8}); nkb >= 1; --nkb) {
+          if (!staged && nkb > 1 && (int64_t)tc_np() * 128 * nkb * 3 > tile_bytes) continue;
+          const int passes = (tiles + max_tiles - 1) / max_tiles, boxes = (kbs + nkb - 1) / nkb;
+          const double w = (double)cnt * kbs * 128, x = staged ? 0 : (double)tc_np() * kbs * 128 * passes;
+          const double box = (double)cnt / tiles * nkb * 128, ahead = slots * box;
+          // (a last task of fewer tiles may not share out its slots: its warps decide)
+          const int group = tiles % max_tiles && passes > 1 ? tiles % max_tiles : std::min(tiles, max_tiles);
+          const TilePlan tp = plan_tile(K, staged, group, rb, nkb, slot_bytes, slots, tile_bytes);
+          const double in_flight = ahead + tp.extra * box, x_rate = std::min(75e3, tp.nx * tc_np() * 128.0 * nkb / 2.0);
+          const double issue = std::max(tiles * (g->borrow ? 0.04 : 0.15), (double)((group + tp.issuers.tiles - 1) / tp.issuers.tiles) * passes * (nkb * 256 + 900) / (1.9e3 * tp.issuers.chunks));
+          double us = std::max({std::max(0.0, w - ahead) / (44e3 * std::min(1.0, in_flight / 100e3)), (w + x) / 75e3, x > 0 ? x / x_rate : 0.0, kbs * 4 * tiles * 0.025, boxes * issue}) + tiles * tc_np() * 0.02;
+          if (S > 1) us += 4.0 + (double)(S + 1) * tiles * tc_np() * rb * 4 / 50e3;
+          if (best.splits == 0 || us < best.us * 0.98) best = SplitPlan{S, groups, tiles, rb, nkb, us};
+        }
+      }
+    }
+    return best;
   }
 
   // activation tile of an FP8 linear: [tokens, KT] e4m3 rows padded by 16 bytes, then one scale exponent per
@@ -282,6 +372,11 @@ struct Builder {
           else consumers.push_back(j);
           // the norm prologue needs the whole row in the activation tile
           if (ok && p.op == MPK_OP_RMSNORM && linear_tile_bytes(T[c.t[1]].dim(1)) > x_tile_cap()) ok = false;
+          // A row panel of some size gains more from a ring of activations (the tile area serves as weight slots, the weights stream on) than a
+          // task group of its own costs: 16 tokens, gate and up rows of width 4096 47 us with the norm as the prologue, 3.5 + 1.2 + 38.7 us apart.
+          if (ok && p.op == MPK_OP_RMSNORM && tc_linear(T[c.t[1]].dim(1)) && T[c.t[1]].dim(0) >= 16 * (int64_t)W) ok = false;
+          // the activations of a tcgen05 linear come as they are, by tensor-map copies
+          if (ok && p.op == MPK_OP_SILU_MUL && tc_linear(T[c.t[1]].dim(1))) ok = false;
         }
         if (raw_writes(c, T[y].storage)) break;           // y redefined: later readers see the new value
       }
@@ -509,14 +604,18 @@ struct Builder {
       if (l.folded) continue;
       if (hybrid_op(l.op)) {
         need = std::max<int64_t>(need, hybrid_smem(l) - kPartialBytes);
-        if (l.op == MPK_OP_GROUPED_LINEAR && g->hybrid == HYB_BF16 && tc_linear(T[l.t[1]].dim(2))) g->use_tmem = true;
+        if (l.op == MPK_OP_GROUPED_LINEAR && g->hybrid == HYB_BF16 && tc_linear(T[l.t[1]].dim(2))) {
+          g->use_tmem = true;
+          need = std::max(need, x_ring_bytes());
+        }
       } else if (g->hybrid == HYB_F32 && l.op == MPK_OP_LINEAR) {
         const int64_t K = T[l.t[1]].dim(1);
         need = std::max<int64_t>(need, (int64_t)linear_f32_tokens(K) * K * 4 - kPartialBytes);
       } else if (l.op == MPK_OP_LINEAR || l.op == MPK_OP_LINEAR_RESIDUAL || l.op == MPK_OP_SPLITK_LINEAR) {
         const int64_t K = T[l.t[1]].dim(1);
-        need = std::max(need, std::min<int64_t>(linear_tile_bytes(K), x_tile_cap()));
-        if (tc_linear(K) && T[l.t[1]].dtype == MPK_BF16) g->use_tmem = true;
+        const bool tc = tc_linear(K) && T[l.t[1]].dtype == MPK_BF16;
+        need = std::max(need, tc && l.prologue == PRO_PLAIN ? x_ring_bytes() : std::min<int64_t>(linear_tile_bytes(K), x_tile_cap()));
+        if (tc) g->use_tmem = true;
       } else if (l.op == MPK_OP_LINEAR_FP8 || l.op == MPK_OP_LINEAR_FP8_RESIDUAL) {
         const int64_t K = T[l.t[2]].dim(1);
         if (tc_linear_fp8(K)) {
@@ -578,6 +677,33 @@ struct Builder {
     g->chunk_cols = g->use_tmem ? 448 : cols;          // 16 rows x (448 x 2 + 16) bytes <= 16 KB
     g->stage_bytes = g->use_tmem ? kTcSlotBytes : stage_bytes_for(cols);
     g->num_stages = fitting(g->stage_bytes);
+    // Slots as large as serves the graph's linears best: whole boxes of their row tiles, several of them in flight.  (FP8 and expert
+    // projections are planned for 16 KB.)
+    bool only_linears = g->use_tmem;
+    g->borrow = g->use_tmem;
+    for (const auto &l : L) {
+      if (l.folded) continue;
+      if (bf16_linear(l) && !tc_linear(T[l.t[1]].dim(1))) g->borrow = false;
+      if (l.op == MPK_OP_GROUPED_LINEAR && !tc_linear(T[l.t[1]].dim(2))) g->borrow = false;
+      switch (l.op) {
+        case MPK_OP_LINEAR_FP8: case MPK_OP_LINEAR_FP8_RESIDUAL: case MPK_OP_MOE_W13_FP8: case MPK_OP_MOE_W2_FP8: case MPK_OP_MOE_W13_LINEAR: case MPK_OP_MOE_W2_LINEAR:
+          only_linears = false;
+          break;
+        default: break;
+      }
+    }
+    g->borrow = g->borrow && only_linears;
+    double best = 0;
+    for (int kb = 32; only_linears && kb >= 16; --kb) {   // (large ones first: fewer boxes for the same bytes)
+      const int n = fitting(kb * 1024);
+      if (n < 2) continue;
+      double us = 0;
+      for (const auto &l : L) {
+        if (l.folded || !bf16_linear(l) || !tc_linear(T[l.t[1]].dim(1))) continue;
+        us += plan_split(T[l.t[1]].dim(0), T[l.t[1]].dim(1), row_unit(l), l.prologue != PRO_PLAIN, kb * 1024, n, tile_behind(n, kb * 1024)).us;
+      }
+      if (best == 0 || us < best * 0.995) { best = us; g->stage_bytes = kb * 1024; g->num_stages = n; }
+    }
     if (g->num_stages < 2) return fail(MPK_ERR_UNSUPPORTED, "activation tile leaves fewer than 2 weight stages");
     g->x_tile_bytes = (int)tile_behind(g->num_stages, g->stage_bytes);
     return MPK_OK;
@@ -599,7 +725,7 @@ struct Builder {
     g->exec[exec].num_tasks++;
   }
 
-  int emit_linear(int li, int ex) {
+  int emit_linear(int li, int ex, int split_bank) {
     const LayerInfo &l = L[li];
     const TensorInfo &w = T[l.t[1]];
     const int yid = l.op == MPK_OP_LINEAR_RESIDUAL ? l.t[3] : l.t[2];
@@ -614,12 +740,10 @@ struct Builder {
     // k tiling of the activation tile: the fewest tiles whose [tokens, KT] slab fits the tile buffer
     const int ntok = std::min(std::max(cfg.max_num_batched_tokens, 1), (int)kMaxLinearTokens);
     const bool tc = g->use_tmem && tc_linear(K);
-    const int kq = tc ? kTcKBlock : 16;   // granularity of a k tile
     int nkt = 1;
-    while (nkt <= K / kq &&
-           !(K % nkt == 0 && (K / nkt) % kq == 0 && linear_tile_bytes(K / nkt) <= g->x_tile_bytes))
-      ++nkt;
-    if (nkt > K / kq) return fail(MPK_ERR_UNSUPPORTED, "cannot tile K for " + w.name);
+    if (!tc || l.prologue != PRO_PLAIN)
+      while (nkt <= K / 16 && !(K % nkt == 0 && (K / nkt) % 16 == 0 && linear_tile_bytes(K / nkt) <= g->x_tile_bytes)) ++nkt;
+    if (nkt > K / 16) return fail(MPK_ERR_UNSUPPORTED, "cannot tile K for " + w.name);
     const int KT = K / nkt;
     const bool f32_source = l.prologue == PRO_RESNORM || l.prologue == PRO_POLY;   // formed from float32 values by the prologue
     if ((l.prologue == PRO_RMSNORM || f32_source) && nkt != 1)
@@ -677,7 +801,7 @@ struct Builder {
     const int out_cols = gated ? N / 2 : N;
     if (g->hybrid ? y.dim(y.dims.size() - 1) < out_cols : y.dim(y.dims.size() - 1) != N)
       return fail(MPK_ERR_INVALID, "linear output width != N for " + w.name);
-    const int unit = l.silu_out >= 0 || gated ? 4 : 1;      // paired rows stay in one task
+    const int unit = l.silu_out >= 0 || gated ? 4 : tc ? row_unit(l) : 1;      // paired rows stay in one task
     if (l.silu_out >= 0) {
       if (epi != EPI_STORE || N % 4 != 0) return fail(MPK_ERR_INVALID, "activation epilogue on an unsupported linear: " + w.name);
       epi = EPI_SILU_PAIR;
@@ -686,45 +810,27 @@ struct Builder {
     }
     bool w_dynamic = false;
     for (const auto &o : L) if (!o.folded && raw_writes(o, w.storage)) w_dynamic = true;
-    const int base = (N / unit) / W, rem = (N / unit) % W;
-    // tcgen05 path: cut the widest worker panel into row tiles of RB <= 128 rows (one accumulator each) and give a
-    // ring slot as many 64-column k blocks of such a tile as it holds; among the tilings near the minimum, take
-    // the one that fills the slots best (the bytes in flight per worker are what hides the HBM latency)
-    int tc_rb = 0, tc_nkb = 1, tc_task_rows = 0;
+    // tcgen05 path: row panels of `groups` x `splits` workers, cut into row tiles of RB <= 128 rows (one accumulator each)
+    SplitPlan sp;
     if (tc) {
-      const int cnt_max = (base + (rem ? 1 : 0)) * unit;
-      const int kbt = KT / kTcKBlock;
-      const int t_min = (cnt_max + 127) / 128;
-      // Measured: an M = 128 bf16 tcgen05.mma with N <= 64 occupies the tensor pipe for about 43 cycles whatever N is
-      // and however few of its 128 rows are real, and a worker must consume ~23 weight bytes per cycle to keep up
-      // with its share of HBM.  A K = 16 step of a tile with r real rows consumes 32 r bytes: r must exceed ~31
-      // for the MMAs to stay ahead of the stream, so tiles keep at least 40 real rows where the panel allows.
-      const int need_rows = 40;
-      double best = -1.0;
-      for (int tiles = t_min; tiles <= t_min + 6; ++tiles) {
-        const int rb = ((cnt_max + tiles - 1) / tiles + 7) / 8 * 8;
-        if (rb > 128 || rb <= 0) continue;
-        if (tiles > t_min && cnt_max / tiles < need_rows) break;
-        int nkb = std::min(kbt, g->stage_bytes / (rb * 128));
-        while (nkb > 1 && kbt % nkb != 0) --nkb;
-        if (nkb < 1) continue;
-        const double fill = (double)cnt_max / tiles * 128.0 * nkb / g->stage_bytes;
-        if (fill > best * 1.05) { best = fill; tc_rb = rb; tc_nkb = nkb; }
-      }
-      if (tc_rb == 0) return fail(MPK_ERR_UNSUPPORTED, "cannot tile the rows of " + w.name);
-      tc_task_rows = std::max(1, kTcAccCols / tc_np()) * tc_rb;   // accumulators of one task: tiles x tc_np() columns
-      g->exec[ex].tc_rows = tc_rb;
-      g->exec[ex].tc_kblocks = tc_nkb;
+      sp = plan_split(N, K, unit, l.prologue != PRO_PLAIN, g->stage_bytes, g->num_stages, g->x_tile_bytes);
+      if (sp.splits == 0) return fail(MPK_ERR_UNSUPPORTED, "cannot tile the rows of " + w.name);
+      g->exec[ex].tc_rows = sp.rb;
+      g->exec[ex].tc_kblocks = sp.nkb;
     }
-    const int task_cap = tc ? tc_task_rows : cap;
+    const int panels = tc ? sp.groups : W, splits = tc ? sp.splits : 1;
+    const int base = (N / unit) / panels, rem = (N / unit) % panels;
+    const int task_cap = tc ? tc_task_tiles(g->num_stages) * sp.rb : cap;   // accumulators of one task: tiles x tc_np() columns
+    std::vector<int> x_maps(splits, -1);
+    int64_t split_floats = 0;   // of this layer
     int row = 0;
-    for (int i = 0; i < W; ++i) {
-      const int worker = (i + rot) % W;
+    for (int i = 0; i < panels; ++i) {
       const int cnt = (base + (i < rem ? 1 : 0)) * unit;
       bool first = true;
-      for (int r = row; r < row + cnt; r += task_cap) {
+      for (int r = row, part = 0; r < row + cnt; part = (part + 1) % splits, r += part == 0 ? task_cap : 0) {
+        const int worker = (part * panels + i + rot) % W;
         TaskDesc d = blank(TASK_LINEAR, li);
-        if (!first && nkt == 1) d.flags |= TF_SAME_X_AS_PREV;
+        if (!tc && !first && nkt == 1) d.flags |= TF_SAME_X_AS_PREV;
         if (w_dynamic) d.flags |= TF_STREAM_AFTER_DEP;
         d.p[0] = (uint64_t)w.ptr;
         d.p[1] = (uint64_t)x.ptr;
@@ -778,27 +884,70 @@ struct Builder {
           put_wide(&d, LR_ROW, l.pro_row);
         }
         if (tc) {
+          const int kb = K / kTcKBlock, kb0 = (int)((int64_t)kb * part / splits), kb1 = (int)((int64_t)kb * (part + 1) / splits);
           d.flags |= TF_TC;
-          d.a[L_KC] = tc_nkb * kTcKBlock;
-          d.a[L_ROWS] = tc_rb;
+          d.a[L_K] = (kb1 - kb0) * kTcKBlock;
+          d.a[L_KT] = d.a[L_KC] = sp.nkb * kTcKBlock;
+          d.a[L_ROWS] = sp.rb;
           d.a[L_TMAP] = (int)g->tmaps.size();
           TmapSpec m;
-          m.base = (uint64_t)w.ptr + (uint64_t)r * (uint64_t)ldw * 2;
+          m.base = (uint64_t)w.ptr + (uint64_t)r * (uint64_t)ldw * 2 + (uint64_t)kb0 * 128;
           m.rows = d.a[L_N1] - d.a[L_N0];
           m.ld_bytes = (int64_t)ldw * 2;
-          m.kblocks = K / kTcKBlock;
-          m.box_rows = tc_rb;
-          m.box_kblocks = tc_nkb;
+          m.kblocks = kb1 - kb0;
+          m.box_rows = sp.rb;
+          m.box_kblocks = sp.nkb;
           m.elt_bytes = 2;
           g->tmaps.push_back(m);
+          if (l.prologue == PRO_PLAIN) {
+            if (x_maps[part] < 0) x_maps[part] = add_x_map((uint64_t)x.ptr + (uint64_t)kb0 * 128, token_rows(x), x.ld(), kb1 - kb0, sp.nkb);
+            d.a[LX_TMAP] = x_maps[part];
+          }
+          d.a[LX_SPLITS] = splits;
+          d.a[LX_PART] = part;
+          place_tile(&d, l.prologue != PRO_PLAIN, sp.nkb);
+          if (splits > 1) {   // (bank and layer offsets are patched when all sizes are known)
+            const int tiles = (d.a[L_N1] - d.a[L_N0] + sp.rb - 1) / sp.rb;
+            d.p[6] = (uint64_t)split_floats;
+            if (part == splits - 1) split_floats += (int64_t)splits * tiles * tc_np() * sp.rb;
+            d.a[LX_TICKET] = split_tickets + i;
+          }
         }
         put(worker, d, ex);
-        g->weight_bytes += (int64_t)(d.a[L_N1] - d.a[L_N0]) * K * 2;
+        g->weight_bytes += (int64_t)(d.a[L_N1] - d.a[L_N0]) * d.a[L_K] * 2;
         first = false;
       }
       row += cnt;
     }
+    if (splits > 1) {
+      split_tickets += panels;
+      split_banks.resize(std::max<size_t>(split_banks.size(), split_bank + 1), 0);
+      split_banks[split_bank] = std::max(split_banks[split_bank], split_floats);
+      split_bank_of[ex] = split_bank;
+    }
     return MPK_OK;
+  }
+
+  // Where a tcgen05 linear task keeps its activations and borrowed slots.
+  void place_tile(TaskDesc *d, bool staged, int nkb) const {
+    const int rb = d->a[L_ROWS], tiles = (d->a[L_N1] - d->a[L_N0] + rb - 1) / rb;
+    const TilePlan p = plan_tile(d->a[L_K], staged, tiles, rb, nkb, g->stage_bytes, g->num_stages, g->x_tile_bytes);
+    d->a[LX_NX] = p.nx;
+    d->a[LX_XBYTES] = p.bytes;
+    d->a[LX_EXTRA] = p.extra;
+  }
+  // Tensor map of a linear's activations from `base` on.
+  int add_x_map(uint64_t base, int64_t rows, int64_t ld, int64_t kblocks, int nkb) {
+    TmapSpec m;
+    m.base = base; m.rows = rows; m.ld_bytes = ld * 2; m.kblocks = kblocks; m.box_rows = tc_np(); m.box_kblocks = nkb; m.elt_bytes = 2;
+    g->tmaps.push_back(m);
+    return (int)g->tmaps.size() - 1;
+  }
+  // rows of an activation tensor
+  static int64_t token_rows(const TensorInfo &x) {
+    int64_t n = 1;
+    for (size_t i = 0; i + 1 < x.dims.size(); ++i) n *= x.dims[i];
+    return n;
   }
 
   // Strides (in uint32 words) of a packed UE8M0 scale tensor over (outer index, packed k).  Accepted layouts:
@@ -1386,26 +1535,27 @@ struct Builder {
       return fail(MPK_ERR_UNSUPPORTED, "grouped linear: K a multiple of 16, input columns on 16-byte boundaries: " + w.name);
     const int64_t rows = (int64_t)G * N;
     const bool tc = !f32 && g->use_tmem && tc_linear(K);
-    if (!f32 && linear_tile_bytes(K) > g->x_tile_bytes) return fail(MPK_ERR_UNSUPPORTED, "grouped linear: K too large: " + w.name);
+    if (!f32 && !tc && linear_tile_bytes(K) > g->x_tile_bytes) return fail(MPK_ERR_UNSUPPORTED, "grouped linear: K too large: " + w.name);
     const int esz_x = f32 ? 4 : 2, esz_y = y.dtype == MPK_F32 ? 4 : 2;
     int KC = std::min(K, g->chunk_cols) / 16 * 16;
     while (!f32 && KC > 16 && K % KC != 0) KC -= 16;
     // tcgen05: row tiles of at most 128 rows; a task holds as many accumulators as fit
-    const int64_t widest = std::min<int64_t>((rows + W - 1) / W, N);
+    const int64_t widest = std::min<int64_t>((rows + W - 1) / W + 3, N);
     int rb = 0, nkb = 1;
     if (tc) {
       const int tiles = (int)((widest + 127) / 128);
       rb = (int)std::min<int64_t>(128, ((widest + tiles - 1) / tiles + 7) / 8 * 8);
-      nkb = std::max(1, std::min(K / kTcKBlock, g->stage_bytes / (rb * 128)));
+      nkb = std::max(1, std::min({K / kTcKBlock, g->stage_bytes / (rb * 128), g->x_tile_bytes / (tc_np() * 128 * 3), 8}));
       while (K / kTcKBlock % nkb) --nkb;
       g->exec[ex].tc_rows = rb;
       g->exec[ex].tc_kblocks = nkb;
     }
-    const int cap = tc ? std::max(1, kTcAccCols / tc_np()) * rb : 1 << 20;
+    const int cap = tc ? tc_task_tiles(g->num_stages) * rb : 1 << 20;
+    std::vector<int> x_maps(G, -1);
     for (int i = 0; i < W; ++i) {
-      const int64_t end = rows * (i + 1) / W;
+      const int64_t unit = tc && N % 4 == 0 ? 4 : 1, end = rows / unit * (i + 1) / W * unit;
       int last = -1;
-      for (int64_t r = rows * i / W; r < end;) {
+      for (int64_t r = rows / unit * i / W * unit; r < end;) {
         const int grp = (int)(r / N), n0 = (int)(r - (int64_t)grp * N);
         const int n1 = (int)std::min<int64_t>(std::min<int64_t>(N, end - (int64_t)grp * N), n0 + cap);
         TaskDesc d = blank(f32 ? TASK_LINEAR_F32 : TASK_LINEAR, li);
@@ -1417,18 +1567,22 @@ struct Builder {
           d.p[4] = gp; d.a[9] = gate >= 0 ? (int)T[gate].ld() : 0;
           d.a[0] = n0; d.a[1] = n1; d.a[2] = K; d.a[3] = K; d.a[4] = (int)x.ld(); d.a[5] = (int)y.ld(); d.a[7] = linear_f32_tokens(K);
         } else {
-          if (grp == last) d.flags |= TF_SAME_X_AS_PREV;
+          if (!tc && grp == last) d.flags |= TF_SAME_X_AS_PREV;
           d.a[L_N0] = n0; d.a[L_N1] = n1; d.a[L_K] = K; d.a[L_LDW] = K; d.a[L_LDX] = (int)x.ld(); d.a[L_LDO] = (int)y.ld();
           d.a[L_PRO] = PRO_PLAIN; d.a[L_EPI] = gate >= 0 ? EPI_GATE_SIGMOID : y.dtype == MPK_F32 ? EPI_STORE_F32 : EPI_STORE; d.a[L_GROUPS] = 1;
           d.p[3] = gp; d.a[L_LDR] = gate >= 0 ? (int)T[gate].ld() : 0;
           d.a[L_KT] = K; d.a[L_KC] = KC; d.a[L_ROWS] = kChunkRows; d.a[L_N] = N;
           if (tc) {
             d.flags |= TF_TC;
-            d.a[L_KC] = nkb * kTcKBlock; d.a[L_ROWS] = rb; d.a[L_TMAP] = (int)g->tmaps.size();
+            if (x_maps[grp] < 0) x_maps[grp] = add_x_map(d.p[1], token_rows(x), x.ld(), K / kTcKBlock, nkb);
+            d.a[LX_TMAP] = x_maps[grp];
+            d.a[LX_SPLITS] = 1;
+            d.a[L_KT] = d.a[L_KC] = nkb * kTcKBlock; d.a[L_ROWS] = rb; d.a[L_TMAP] = (int)g->tmaps.size();
             TmapSpec m;
             m.base = d.p[0] + (uint64_t)n0 * K * 2;
             m.rows = n1 - n0; m.ld_bytes = (int64_t)K * 2; m.kblocks = K / kTcKBlock; m.box_rows = rb; m.box_kblocks = nkb; m.elt_bytes = 2;
             g->tmaps.push_back(m);
+            place_tile(&d, false, nkb);
           }
         }
         put((i + rot) % W, d, ex);
@@ -1867,12 +2021,12 @@ struct Builder {
     }
   }
 
-  int emit(int li, int ex, int *attn_ordinal, int attn_bank) {
+  int emit(int li, int ex, int *attn_ordinal, int attn_bank, int split_bank) {
     const LayerInfo &l = L[li];
     const int mbt = cfg.max_num_batched_tokens;
     switch (l.op) {
       case MPK_OP_LINEAR: case MPK_OP_LINEAR_RESIDUAL: case MPK_OP_SPLITK_LINEAR:
-        return g->hybrid == HYB_F32 ? emit_linear_f32(li, ex) : emit_linear(li, ex);
+        return g->hybrid == HYB_F32 ? emit_linear_f32(li, ex) : emit_linear(li, ex, split_bank);
       case MPK_OP_RESIDUAL_NORM: return emit_residual_norm(li, ex);
       case MPK_OP_QKV_APPEND: return emit_qkv_append(li, ex);
       case MPK_OP_EXT_ATTENTION: return emit_ext_attention(li, ex);
@@ -2332,6 +2486,18 @@ struct Builder {
       bank_user[attn_bank[e]] = e;
     }
 
+    // The parts of linears that are split along k lie in scratch memory until the last worker of a panel adds them up: banks likewise.
+    std::vector<int> split_bank(E, 0), split_user;
+    for (int e = 0; e < E; ++e) {
+      const int li = g->exec[e].layer;
+      if (li < 0 || !bf16_linear(L[li]) || !g->use_tmem || T[L[li].t[1]].dims.size() != 2 || !tc_linear(T[L[li].t[1]].dim(1)) ||
+          plan_split(T[L[li].t[1]].dim(0), T[L[li].t[1]].dim(1), row_unit(L[li]), L[li].prologue != PRO_PLAIN, g->stage_bytes, g->num_stages, g->x_tile_bytes).splits <= 1)
+        continue;
+      while (split_bank[e] < (int)split_user.size() && !anc[e][split_user[split_bank[e]]]) ++split_bank[e];
+      if (split_bank[e] == (int)split_user.size()) split_user.push_back(e);
+      split_user[split_bank[e]] = e;
+    }
+
     // ---- tasks ---------------------------------------------------------------------
     per_worker.assign(W, {});
     per_worker_exec.assign(W, {});
@@ -2345,7 +2511,7 @@ struct Builder {
         x.type = TASK_BATCH;
         continue;
       }
-      rc = emit(x.layer, e, &attn_ordinal, attn_bank[e]);
+      rc = emit(x.layer, e, &attn_ordinal, attn_bank[e], split_bank[e]);
       if (rc) return rc;
       if (x.num_tasks == 0) return fail(MPK_ERR_INVALID, "layer " + std::to_string(x.layer) + " produced no task");
     }
@@ -2401,6 +2567,17 @@ struct Builder {
       for (auto &d : g->tasks)
         if (d.type == TASK_ATTENTION) d.a[A_BANK] = (int)(d.a[A_BANK] * records);
       g->attn_scratch_floats *= (int64_t)bank_user.size();
+    }
+    if (split_tickets > 0) {   // and the places of split linears: their tickets follow all others
+      std::vector<int64_t> first(split_banks.size(), 0);
+      for (size_t i = 0; i < split_banks.size(); ++i) { first[i] = g->split_floats; g->split_floats += split_banks[i]; }
+      for (size_t t = 0; t < g->tasks.size(); ++t) {
+        TaskDesc &d = g->tasks[t];
+        if (d.type != TASK_LINEAR || !(d.flags & TF_TC) || (d.flags & TF_FP8) || d.a[LX_SPLITS] <= 1) continue;
+        d.p[6] += (uint64_t)first[split_bank_of[g->task_exec[t]]];
+        d.a[LX_TICKET] += (int)g->attn_tickets;
+      }
+      g->attn_tickets += split_tickets;
     }
     return simulate_task_graph(*g, err);
   }

@@ -99,12 +99,14 @@ struct CompiledGraph {
   bool general_kernel = false;            // FP8 tasks or more than 8 batched tokens: needs the general instantiation
   int hybrid = 0;                         // HYB_* family: recurrent / extended-attention layers present
   bool use_tmem = false;                  // some linear runs on tcgen05: workers allocate tensor memory
+  bool borrow = false;                    // tcgen05 linears borrow weight slots from the tile area (no other streaming tasks)
   int tc_tokens = 0;                      // token rows of the tcgen05 activation operand tile
   std::vector<TmapSpec> tmaps;            // indexed by TaskDesc::a[L_TMAP], a[A_TMAP]
   int64_t weight_bytes = 0;
   int64_t inbox_floats_per_buffer = 0;    // world * mbt * Nmax
   int64_t attn_scratch_floats = 0;
-  int64_t attn_tickets = 0;
+  int64_t attn_tickets = 0;               // of the attention tasks, the hybrid tasks, the panels of split linears
+  int64_t split_floats = 0;               // scratch memory of linears that are split along k
 };
 
 struct GraphInputs {
