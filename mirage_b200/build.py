@@ -26,7 +26,7 @@ KERNEL_HEADERS = ["runtime_types.h", "device_utils.cuh", "megakernel.cuh", "hybr
 TARGETS = {
     "core": ("libmpk_b200.so", ["mpk_abi.cu", "task_graph.cpp", "shuffle_rows.cu", "noalloc_attention.cu"],
              HOST_HEADERS + ["device_utils.cuh"]),
-    "decoder": ("libmpk_b200_decoder.so", ["decoder_kernels.cu"], KERNEL_HEADERS),
+    "decoder": ("libmpk_b200_decoder.so", ["decoder_kernels.cu", "decoder_kernel_few.cu"], KERNEL_HEADERS + ["decoder_kernels.h"]),
     "hybrid": ("libmpk_b200_hybrid.so", ["hybrid_kernels.cu", "hybrid_kernel_bf16.cu", "hybrid_kernel_bf16_wide.cu", "hybrid_kernel_f32.cu"],
                KERNEL_HEADERS + ["hybrid_kernels.h"]),
 }

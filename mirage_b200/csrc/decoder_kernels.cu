@@ -4,6 +4,7 @@
 // The shared-memory limit is a property of the function on the current device, shared by every handle of the process:
 // it is raised to the device's opt-in maximum (not to this handle's need), so that preparing a graph with a small
 // footprint cannot lower it under a graph prepared earlier.
+#include "decoder_kernels.h"
 #include "megakernel.cuh"
 
 extern "C" int mpk_family_prepare(int smem_bytes, int) {
@@ -19,6 +20,8 @@ extern "C" int mpk_family_prepare(int smem_bytes, int) {
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(mpk::mpk_megakernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
   if (e == cudaSuccess)
+    e = mpk_prepare_few(smem_bytes);
+  if (e == cudaSuccess)
     e = cudaFuncSetAttribute(mpk::mpk_megakernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
   return e == cudaSuccess ? 0 : (int)e;
 }
@@ -26,6 +29,8 @@ extern "C" int mpk_family_prepare(int smem_bytes, int) {
 extern "C" int mpk_family_launch(const mpk::KernelParams *params, int smem_bytes, void *stream) {
   if (params->general_kernel && params->world_size > 1)
     mpk::mpk_megakernel<true, true><<<params->num_workers, mpk::block_threads(true), smem_bytes, (cudaStream_t)stream>>>(*params);
+  else if (params->general_kernel && params->exact_weights)
+    mpk_launch_few(*params, smem_bytes, (cudaStream_t)stream);
   else if (params->general_kernel)
     mpk::mpk_megakernel<true><<<params->num_workers, mpk::block_threads(true), smem_bytes, (cudaStream_t)stream>>>(*params);
   else if (params->world_size > 1 && params->tp_extensions)

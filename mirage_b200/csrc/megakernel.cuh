@@ -3464,7 +3464,7 @@ __device__ __forceinline__ void run_attention(const Ctx &c, const TaskDesc &d, c
 // the warp that meets them (the first tile's warp writes them to the cache), so no warp waits for another's append.
 // A tile that lies in one range is written out at once; otherwise every range leaves its part in a scratch record and the last of them
 // to arrive (a ticket per tile) merges.  Per step: S = Q K^T on mma.sync m16n8k16, online softmax (fp32, base 2), P rounded to bf16 as the
-// reference does (tasks/blackwell/attention_sm100.cuh:558), O += P V on m16n8k8 with V through ldmatrix.trans.
+// reference does (tasks/blackwell/attention_sm100.cuh:558; in graphs of few tokens the sum of two), O += P V on m16n8k8 with V through ldmatrix.trans.
 // Where that leaves a range fewer than kAfMinSteps steps, the latency of a few steps in a row and of merging many parts through L2 is what
 // counts.  Then a worker takes a tile of one kv head, or one of the parts of a tile whose steps exceed a worker's average (af_parts), its eight
 // warps share the positions and combine in shared memory.
@@ -3669,7 +3669,7 @@ static __device__ __noinline__ void af_put_back(const __nv_bfloat16 *v, int ldq,
   __syncwarp();
 }
 
-template <bool shared>
+template <bool shared, bool EXACT>
 __device__ __forceinline__ bool run_attention_steps(const KernelParams &P, const TaskDesc &d, uint8_t *xtile, int *sflags, const AfTable &tab,
                                                     unsigned long long iteration, uint64_t deadline, int task) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
@@ -3910,13 +3910,22 @@ __device__ __forceinline__ bool run_attention_steps(const KernelParams &P, const
 #pragma unroll
         for (int nt = 0; nt < 16; ++nt) { o[nt][0] *= c0; o[nt][1] *= c0; o[nt][2] *= c1; o[nt][3] *= c1; }
       }
-      const uint32_t pa = pack_bf16(p0, p1), pb = pack_bf16(p2, p3);
+      uint32_t pw[4] = {pack_bf16(p0, p1), pack_bf16(p2, p3), 0u, 0u};
+      if (EXACT) {
+        // P as the sum of two bf16, side by side along k, and V twice: less than 2^-17 of a weight is lost.  Graphs of few tokens, whose batch-1 form
+        // holds the weights in fp32 (for all graphs: 16 requests 6.51 -> 6.62 ms, 64 requests 7.79 -> 7.97)
+        pw[2] = pack_bf16(p0 - bf16_lo(pw[0]), p1 - bf16_hi(pw[0]));
+        pw[3] = pack_bf16(p2 - bf16_lo(pw[1]), p3 - bf16_hi(pw[1]));
+      }
 #pragma unroll
       for (int vq = 0; vq < 4; ++vq) {
         uint32_t b[4];
         ldmatrix_x4_trans(b, vt + af_piece(lane & 7, 4 * vq + (lane >> 3)));
 #pragma unroll
-        for (int k = 0; k < 4; ++k) mma_bf16_1688(o[4 * vq + k], pa, pb, b[k]);
+        for (int k = 0; k < 4; ++k) {
+          if (EXACT) mma_bf16_16816(o[4 * vq + k], pw, b[k], b[k]);
+          else mma_bf16_1688(o[4 * vq + k], pw[0], pw[1], b[k]);
+        }
       }
       __syncwarp();                                             // every lane is done with the stage before it is refilled
     }
@@ -4139,7 +4148,8 @@ __device__ __forceinline__ bool run_attention_steps(const KernelParams &P, const
   return true;
 }
 
-static __device__ __forceinline__ bool run_attention_flat(const KernelParams &P, const TaskDesc &d, uint8_t *xtile, int *sflags, unsigned long long iteration,
+template <bool EXACT>
+__device__ __forceinline__ bool run_attention_flat(const KernelParams &P, const TaskDesc &d, uint8_t *xtile, int *sflags, unsigned long long iteration,
                                                           uint64_t deadline, int task) {
   const int warp = threadIdx.x >> 5;
   const int hkv = d.a[A_HKV], G = d.a[A_HQ] / hkv, flags = d.a[A_FLAGS];
@@ -4151,8 +4161,8 @@ static __device__ __forceinline__ bool run_attention_flat(const KernelParams &P,
       af_build_table(P, d, tab);
   }
   consumer_sync();
-  if (tab.total() == 0 || tab.items() > 0) return run_attention_steps<true>(P, d, xtile, sflags, tab, iteration, deadline, task);
-  return run_attention_steps<false>(P, d, xtile, sflags, tab, iteration, deadline, task);
+  if (tab.total() == 0 || tab.items() > 0) return run_attention_steps<true, EXACT>(P, d, xtile, sflags, tab, iteration, deadline, task);
+  return run_attention_steps<false, EXACT>(P, d, xtile, sflags, tab, iteration, deadline, task);
 }
 
 static __device__ void run_embed(const Ctx &c, const TaskDesc &d) {
@@ -4868,7 +4878,7 @@ __device__ __forceinline__ bool task_linear(const Ctx &c, const TaskDesc &d, int
   return ok;
 }
 
-template <bool GENERAL>
+template <bool GENERAL, bool EXACT>
 __device__ __forceinline__ bool task_attention(const Ctx &c, const TaskDesc &d, int t, bool ok, TaskTimes &tt) {
   const KernelParams &P = c.P;
   // the batch description must be final before the page table is read; that event fired long ago
@@ -4883,7 +4893,7 @@ __device__ __forceinline__ bool task_attention(const Ctx &c, const TaskDesc &d, 
   if (GENERAL) {
     if (tt.on && threadIdx.x == 0) tt.begin_ns = globaltimer_ns();
     if (!ok) return false;
-    ok = run_attention_flat(P, d, c.s.xtile, c.s.flags, c.iteration, c.deadline_ns, t);
+    ok = run_attention_flat<EXACT>(P, d, c.s.xtile, c.s.flags, c.iteration, c.deadline_ns, t);
     if (tt.on && threadIdx.x == 0) tt.ready_ns = *reinterpret_cast<volatile uint64_t *>(c.s.flags + 6);
     return ok;
   }
@@ -4939,7 +4949,7 @@ __device__ __forceinline__ bool task_other(const Ctx &c, const TaskDesc &d, int 
   return true;
 }
 
-template <bool GENERAL, bool TPX, int HYB>
+template <bool GENERAL, bool TPX, int HYB, bool EXACT>
 __device__ void consumer_loop(const Ctx &c, int t_begin, int t_end) {
   const KernelParams &P = c.P;
   const int tid = threadIdx.x;
@@ -4962,7 +4972,7 @@ __device__ void consumer_loop(const Ctx &c, int t_begin, int t_end) {
     } else if (GENERAL && !HYB && type == TASK_MOE_GEMM) {
       ok = wait_dependencies(c, d, t, ok, tt);
       ls = run_moe_gemm_decoder(c, d, ls, t, ok);
-    } else if (!HYB && type == TASK_ATTENTION) ok = task_attention<GENERAL>(c, d, t, ok, tt);
+    } else if (!HYB && type == TASK_ATTENTION) ok = task_attention<GENERAL, EXACT>(c, d, t, ok, tt);
     else ok = task_other<GENERAL, TPX, HYB>(c, d, t, ok, tt);
     if (fetch) reinterpret_cast<uint4 *>(&c.s.desc[(t + 1 - t_begin) & 1])[tid - 224] = nxt;
     const int trig = d.trig_event;
@@ -5002,7 +5012,9 @@ __device__ void consumer_loop(const Ctx &c, int t_begin, int t_end) {
 // HYB marks the instantiations of graphs with recurrent or extended-attention layers (hybrid_tasks.cuh): they hold the
 // linear bodies and the hybrid tasks only.  HYB_BF16 serves in bf16; HYB_F32 computes everything in 32-bit floats and has
 // no tensor-core code at all.
-template <bool GENERAL, bool TPX = false, int HYB = 0>
+// EXACT marks the general instantiation of graphs of up to 8 tokens that the batch-1 one would run too: its attention keeps the softmax weights as two bf16.
+// (A flag in the loop instead cost the graphs without it 290 bytes of spills: 64 requests 7.79 -> 8.42 ms.)
+template <bool GENERAL, bool TPX = false, int HYB = 0, bool EXACT = false>
 __global__ void __launch_bounds__(block_threads(GENERAL), 1) mpk_megakernel(const __grid_constant__ KernelParams P) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   Smem s = carve(smem_raw, P);
@@ -5051,7 +5063,7 @@ __global__ void __launch_bounds__(block_threads(GENERAL), 1) mpk_megakernel(cons
     }
   } else {
     if (GENERAL) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kConsumerRegs));
-    consumer_loop<GENERAL, TPX, HYB>(c, t_begin, t_end);
+    consumer_loop<GENERAL, TPX, HYB, EXACT>(c, t_begin, t_end);
   }
   if (use_tmem) tc_fence_before_sync();
   __syncthreads();

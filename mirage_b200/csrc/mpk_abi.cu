@@ -445,6 +445,7 @@ int mpk_compile(mpk_handle *h) {
   P.attn_tickets = h->d_attn_tickets;
   P.split_scratch = h->d_split_scratch;
   P.borrow = g.borrow ? 1 : 0;
+  P.exact_weights = g.exact_weights ? 1 : 0;
   P.profiler = cfg.profiler_buffer;
   P.profiler_entries = cfg.profiler_entries;
   P.eos_token_id = cfg.eos_token_id;

@@ -403,6 +403,7 @@ struct KernelParams {
   int32_t meta_static;                  // the batch description is the caller's and final at launch (test mode, online_notoken):
                                         // the graph has no batching task
   float *split_scratch;                 // parts of linears that are split along k
+  int32_t exact_weights;                // general instantiation of a graph of few tokens: softmax weights as two bf16
   int32_t borrow;                       // all streaming tasks are tcgen05 linears: they borrow weight slots from the tile area
 };
 

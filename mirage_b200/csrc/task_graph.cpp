@@ -64,9 +64,35 @@ struct Builder {
   bool general_graph() const {
     if (nb_max > 8 || cfg.max_num_batched_tokens > 8) return true;
     if (g->hybrid) return false;
-    for (const auto &l : L)
+    bool many = false, fits = cfg.world_size <= 1;
+    for (const auto &l : L) {
       if (l.op >= MPK_OP_QUANTIZE_FP8) return true;
-    return false;
+      if (l.op != MPK_OP_ATTENTION && l.op != MPK_OP_PAGED_ATTENTION) continue;
+      const TensorInfo &kc = T[l.t[1]], &vc = T[l.t[2]];
+      if (kc.dims.size() != 4 || l.params.size() < 2 || l.params[1] <= 0) return false;   // (refused when its tasks are made)
+      many = many || many_requests(l);
+      fits = fits && (l.op == MPK_OP_ATTENTION || kc.dim(1) % 8 == 0) && (((uint64_t)kc.ptr | (uint64_t)vc.ptr) & 15u) == 0;
+    }
+    return many && fits;
+  }
+  // Attention of the batch-1 instantiation: a task per (request, kv head, chunk).  Chunks: enough to give every worker a task, and with many
+  // requests enough that a task stays near 128 rows at full length (the rows a task prefetches before its dependency wait are its cheapest
+  // ones; long serial chunks are latency-bound).
+  int attention_slots(const LayerInfo &l) const { return l.op == MPK_OP_PAGED_ATTENTION ? cfg.max_num_batched_requests : std::max(l.grid[0], 1); }
+  int attention_chunks(const LayerInfo &l) const {
+    const int max_seq = l.op == MPK_OP_PAGED_ATTENTION ? cfg.max_seq_length : (int)T[l.t[1]].dim(1);
+    int n = std::max(1, W / std::max(attention_slots(l) * (int)l.params[1], 1));
+    n = std::max(n, std::min((max_seq + 127) / 128, 16));
+    n = std::min(n, std::max(1, max_seq / 32));
+    return std::min(n, 32);
+  }
+  // Up to 8 tokens: several requests whose tasks are more than the workers, or seven and more, run on the general instantiation, whose attention takes
+  // equal ranges of all requests.  8 layers of width 4096, us, batch-1 and general instantiation: 2 requests of 100 to 300 positions 883 and 927, of 1000 to
+  // 2000 1036 and 963; 4 of 64 to 200 960 and 940, of 500 to 1500 1230 and 985; 5 of 37 to 2000 1438 and 1019; 7 of 100 to 400 1185 and 992; 8 of 64 to 200 1103 and
+  // 996, of 500 to 3000 1959 and 1125; 12 layers of width 2048, 3 of 37 to 500 593 and 637, 4 of 64 to 200 604 and 648; 5 layers, 5 of 200 331 and 345.
+  bool many_requests(const LayerInfo &l) const {
+    const int n = attention_requests(l);
+    return n >= 7 || (n >= 2 && (int64_t)attention_slots(l) * l.params[1] * attention_chunks(l) > W);
   }
 
   // More than 8 batched tokens: bf16 linears whose K is a multiple of 64 run on tcgen05 (swap-AB, weights = M = 128,
@@ -1256,19 +1282,12 @@ struct Builder {
     if (G != 1 && G != 2 && G != 4 && G != 8) return fail(MPK_ERR_UNSUPPORTED, "GQA group size must be 1, 2, 4 or 8");
     if (kc.dim(2) != hkv) return fail(MPK_ERR_INVALID, "kv cache head count != num_kv_heads");
     if (!cfg.qo_indptr && paged && !cfg.dry_run) return fail(MPK_ERR_INVALID, "paged attention needs the batch meta tensors");
-    const int slots = paged ? cfg.max_num_batched_requests : std::max(l.grid[0], 1);
+    const int slots = attention_slots(l);
     const int page = paged ? (int)kc.dim(1) : (int)kc.dim(1);
     if (paged && page != cfg.page_size) return fail(MPK_ERR_INVALID, "kv cache page size != page_size");
     if (paged && general_graph() && page % 8 != 0)
       return fail(MPK_ERR_UNSUPPORTED, "with more than 8 batched tokens (or FP8 / expert layers) the page size must be a multiple of 8");
-    const int max_seq = paged ? cfg.max_seq_length : (int)kc.dim(1);
-    // chunks per (request, kv head): enough to give every worker a task, and with many requests enough that a
-    // task stays near 128 rows at full length (the rows a task prefetches before its dependency wait are its
-    // cheapest ones; long serial chunks are latency-bound)
-    int NC = std::max(1, W / std::max(slots * hkv, 1));
-    NC = std::max(NC, std::min((max_seq + 127) / 128, 16));
-    NC = std::min(NC, std::max(1, max_seq / 32));
-    NC = std::min(NC, 32);
+    int NC = attention_chunks(l);
     const int rope_rows = rope ? (int)T[l.t[5]].dim(0) : 1;
     // (general instantiation: one task per worker and pass, each of its warps takes a range of all requests' steps)
     const bool flat = general_graph();
@@ -2553,9 +2572,9 @@ struct Builder {
       }
     }
     g->worker_begin[W] = (int32_t)g->tasks.size();
-    g->general_kernel = cfg.max_num_batched_tokens > 8;
-    for (const auto &d : g->tasks)
-      if (!g->hybrid && ((d.type == TASK_LINEAR && (d.flags & TF_FP8)) || d.type >= TASK_QUANTIZE_FP8)) g->general_kernel = true;
+    g->general_kernel = general_graph();
+    g->exact_weights = g->general_kernel && nb_max <= 8 && cfg.max_num_batched_tokens <= 8;
+    for (const auto &l : L) if (l.op >= MPK_OP_QUANTIZE_FP8) g->exact_weights = false;
     g->num_workers = W;
     g->world_size = std::max(cfg.world_size, 1);
     // attention ticket banks: patch the ticket offset now that the bank size is known

@@ -99,6 +99,7 @@ struct CompiledGraph {
   bool general_kernel = false;            // FP8 tasks or more than 8 batched tokens: needs the general instantiation
   int hybrid = 0;                         // HYB_* family: recurrent / extended-attention layers present
   bool use_tmem = false;                  // some linear runs on tcgen05: workers allocate tensor memory
+  bool exact_weights = false;             // general kernel of a graph of few tokens without FP8, expert or latent layers
   bool borrow = false;                    // tcgen05 linears borrow weight slots from the tile area (no other streaming tasks)
   int tc_tokens = 0;                      // token rows of the tcgen05 activation operand tile
   std::vector<TmapSpec> tmaps;            // indexed by TaskDesc::a[L_TMAP], a[A_TMAP]
