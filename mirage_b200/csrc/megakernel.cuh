@@ -2022,24 +2022,32 @@ static __device__ void run_moe_routing(const Ctx &c, const TaskDesc &d) {
   const bool softmax = d.a[11] != 0;   // moe_topk_softmax_routing_layer: scores = softmax over the experts, no bias, logits kept
   for (int row = warp; row < B; row += 8) {
     float row_max = -INFINITY;
-    for (int e = lane; e < E; e += 32) {
-      float logit;
-      if (f32_in) {
-        float *lp = reinterpret_cast<float *>(d.p[0]) + (size_t)row * ldl + e;
-        logit = __ldcg(lp);
-        if (!softmax && !keep_logits) *lp = 0.f;
-      } else {
-        __nv_bfloat16 *lp = reinterpret_cast<__nv_bfloat16 *>(d.p[0]) + (size_t)row * ldl + e;
-        logit = bf16_to_f(__ldcg(lp));
-        if (!softmax && !keep_logits) *lp = __float2bfloat16_rn(0.f);
+    // eight logits of a lane at a time, loaded before the first is cleared: cleared one by one, the loads waited for one another
+    for (int e0 = lane; e0 < E; e0 += 256) {
+      float logit[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int e = e0 + 32 * j;
+        logit[j] = 0.f;
+        if (e < E) logit[j] = f32_in ? __ldcg(reinterpret_cast<const float *>(d.p[0]) + (size_t)row * ldl + e)
+                                     : bf16_to_f(__ldcg(reinterpret_cast<const __nv_bfloat16 *>(d.p[0]) + (size_t)row * ldl + e));
       }
-      if (softmax) {
-        sc[e] = logit;
-        row_max = fmaxf(row_max, logit);
-      } else {
-        const float sig = __fdiv_rn(1.0f, 1.0f + expf(-logit));
-        sc[e] = sig;
-        bi[e] = sig + __ldg(&bias[e]);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int e = e0 + 32 * j;
+        if (e >= E) continue;
+        if (!softmax && !keep_logits) {
+          if (f32_in) reinterpret_cast<float *>(d.p[0])[(size_t)row * ldl + e] = 0.f;
+          else reinterpret_cast<__nv_bfloat16 *>(d.p[0])[(size_t)row * ldl + e] = __float2bfloat16_rn(0.f);
+        }
+        if (softmax) {
+          sc[e] = logit[j];
+          row_max = fmaxf(row_max, logit[j]);
+        } else {
+          const float sig = __fdiv_rn(1.0f, 1.0f + expf(-logit[j]));
+          sc[e] = sig;
+          bi[e] = sig + __ldg(&bias[e]);
+        }
       }
     }
     if (softmax) {
@@ -2062,7 +2070,25 @@ static __device__ void run_moe_routing(const Ctx &c, const TaskDesc &d) {
     }
     __syncwarp();
     if (groups > 1) {   // (one group: nothing to choose between)
-      for (int g = lane; g < groups; g += 32) {
+      // the two largest of a group: its lanes take every `share`-th expert (groups, a power of two up to 32, share the warp out), then meet
+      const int share = groups <= 32 && (groups & (groups - 1)) == 0 && per >= 32 / groups && per > 1 ? 32 / groups : 0;
+      if (share > 0) {
+        const int g = lane / share, i0 = lane - g * share;
+        float t1 = -INFINITY, t2 = -INFINITY;
+        for (int i = i0; i < per; i += share) {
+          const float v = bi[g * per + i];
+          if (v > t1) { t2 = t1; t1 = v; }
+          else if (v > t2) t2 = v;
+        }
+        for (int o = 1; o < share; o <<= 1) {
+          const float u1 = __shfl_xor_sync(0xffffffffu, t1, o), u2 = __shfl_xor_sync(0xffffffffu, t2, o);
+          t2 = fmaxf(fminf(t1, u1), fmaxf(t2, u2));
+          t1 = fmaxf(t1, u1);
+        }
+        const float head = bi[g * per];   // (a group that begins with NaN is never chosen)
+        if (i0 == 0) gs[g] = head == head ? t1 + fmaxf(t2, -1e30f) : head;
+      }
+      for (int g = lane; share == 0 && g < groups; g += 32) {
         float t1 = bi[g * per], t2 = -1e30f;
         for (int i = 1; i < per; ++i) {
           const float v = bi[g * per + i];
